@@ -45,13 +45,9 @@
 // row, the group stores that row (the range's first row plus the rows closed
 // before it).  Every row of up to kExactMax entries is summed by one group in
 // the reference's order (bit-identical results).  No atomics: every output
-// row is written exactly once.  Three row kernels share that scheme:
-//   spmm_wide_kernel  FP32 panels of 32, 64 or 128 bytes, and unweighted BF16
-//                     into BF16: a lane owns 32 bytes of each gathered row;
-//                     8 column ids per 32-byte load
-//   spmm_kernel       16-byte lanes (BF16 into FP32, weighted BF16, FP64,
-//                     integer and odd widths), with L2 evict_last hints on
-//                     hot-pack gathers and evict_first on cold rows
+// row is written exactly once.  Two row kernels share that scheme:
+//   spmm_lane_kernel  every panel: a lane owns 2 to 32 bytes of each gathered
+//                     row, 8 or 16 gathers in flight per lane
 //   spmv_kernel       k = 1: a warp per range, gathers staged in shared memory
 // Each call first packs the hot rows: pack_hot_vec_kernel in 16-byte units,
 // pack_hot_kernel one element per thread (k = 1 and rows of odd widths).
@@ -127,23 +123,6 @@ struct xvec {
 };
 
 template <class T, int VEC>
-__device__ __forceinline__ xvec<T, VEC> ld_x(const T *p)
-{
-	xvec<T, VEC> r;
-	if constexpr (VEC * sizeof(T) == 16) {
-		uint4 u = __ldg(reinterpret_cast<const uint4 *>(p));
-		memcpy(&r, &u, 16);
-	} else if constexpr (sizeof(T) == 2) {
-		unsigned short u = __ldg(reinterpret_cast<const unsigned short *>(p));
-		memcpy(&r, &u, 2);
-	} else {
-		static_assert(VEC == 1, "scalar path");
-		r.v[0] = __ldg(p);
-	}
-	return r;
-}
-
-template <class T, int VEC>
 __device__ __forceinline__ void st_y(T *p, const T (&v)[VEC])
 {
 	if constexpr (VEC * sizeof(T) == 16) {
@@ -210,22 +189,6 @@ __device__ __forceinline__ xvec<T, VEC> ld_x_hint(const T *p, uint64_t pol)
 	return r;
 }
 
-// Store one 16-byte vector when `pred` holds, without a branch (a predicated
-// streaming store); other widths fall back to a guarded plain store.
-template <class T, int VEC>
-__device__ __forceinline__ void st_y_if(T *p, const T (&v)[VEC], bool pred)
-{
-	if constexpr (VEC * sizeof(T) == 16) {
-		uint32_t u[4];
-		memcpy(u, v, 16);
-		asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
-				"@q st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};\n\t}"
-				:: "l"(p), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(uint32_t(pred)) : "memory");
-	} else {
-		if (pred) st_y<T, VEC>(p, v);
-	}
-}
-
 struct spmm_args {
 	const uint32_t *col;
 	const void *val;
@@ -241,7 +204,6 @@ struct spmm_args {
 	int k;           // columns in this panel
 	int G;           // lanes per row group
 	int R;           // row groups per warp
-	int nv;          // vectors per lane (scalar path)
 	uint32_t n_ranges;
 };
 
@@ -313,71 +275,6 @@ struct accum {
 	}
 };
 
-template <class YT, class A, int VEC, int NV, bool SCALE_OUT>
-__device__ __forceinline__ void store_row(const spmm_args &a, int32_t row, int colbase,
-		const accum<A, VEC, NV> &acc)
-{
-	YT *Y = static_cast<YT *>(a.Y);
-	A so = A(1);
-	if constexpr (SCALE_OUT) so = static_cast<const A *>(a.s_out)[row];
-	const int stride = a.G * VEC;
-#pragma unroll
-	for (int v = 0; v < NV; v++)
-		if (v < a.nv && colbase + v * stride < a.k) {
-			YT out[VEC];
-#pragma unroll
-			for (int i = 0; i < VEC; i++) {
-				A t = acc.get(v, i);
-				if constexpr (SCALE_OUT) t = acc_mul(t, so);
-				out[i] = from_acc<YT, A>(t);
-			}
-			st_y<YT, VEC>(Y + int64_t(row) * a.ldy + colbase + v * stride, out);
-		}
-}
-
-template <int U>
-__device__ __forceinline__ void ld_idx(const uint32_t *col, uint32_t step, uint32_t (&r)[U])
-{
-	const uint4 *p = reinterpret_cast<const uint4 *>(col) + (U / 4) * step;
-#pragma unroll
-	for (int q = 0; q < U / 4; q++) {
-		// cached: a group reads each 128-byte line of its stream over several steps
-		uint4 a = __ldg(p + q);
-		r[4 * q] = a.x; r[4 * q + 1] = a.y; r[4 * q + 2] = a.z; r[4 * q + 3] = a.w;
-	}
-}
-
-template <class WT, class A, int U>
-__device__ __forceinline__ void ld_w(const void *val, uint32_t step, A (&w)[U])
-{
-	if constexpr (std::is_void<WT>::value) {
-#pragma unroll
-		for (int u = 0; u < U; u++) w[u] = A(1);
-	} else {
-		{
-			// cached like the column ids: the streaming form, which skips
-			// L1, fetched each weight line from L2 again at every step (in
-			// the 32-byte-lane kernel, cached 32-byte weight loads took a
-			// weighted call at R-MAT scale 24, k = 16 from 3.43 to 2.58 ms)
-			const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const WT *>(val) + size_t(step) * U);
-			constexpr int per = int(16 / sizeof(WT));
-			static_assert(U % per == 0, "whole 16-byte weight loads");
-#pragma unroll
-			for (int q = 0; q < U / per; q++) {
-				uint4 a = __ldg(p + q);
-				WT t[per];
-				memcpy(t, &a, 16);
-#pragma unroll
-				for (int i = 0; i < per; i++) w[q * per + i] = A(t[i]);
-			}
-		}
-	}
-}
-
-// One range in steps of U entries.  Row runs (slot == kNoSlot) store each
-// row when its end flag passes; chunks of longer rows leave their sum in
-// partial[slot].  Hot entries read the packed rows (which already carry
-// s_in); the others read X and, with SCALE_IN, s_in.
 // The PageRank update at a row close (EPI): rows of the fixup's heavy list
 // are left to the fixup.
 __device__ __forceinline__ void pr_update(const pr_epi &e, int64_t row, float out, unsigned &cnt)
@@ -392,289 +289,258 @@ __device__ __forceinline__ void pr_update(const pr_epi &e, int64_t row, float ou
 	e.pr1[row] = __fmul_rn(x, d);
 }
 
-template <class XT, class YT, class A, class WT, int VEC, int NV, int U, bool SCALE_IN, bool SCALE_OUT,
-		bool EPI = false>
-__device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, int colbase,
-		uint64_t pol_hot, uint64_t pol_cold, const pr_epi &e, unsigned &cnt)
-{
-	const XT *X = static_cast<const XT *>(a.X);
-	const XT *H = static_cast<const XT *>(a.xhot);
-	const int stride = a.G * VEC;
-	constexpr bool kBinary = std::is_void<WT>::value;
-	const bool runs = rg.slot == kNoSlot;
-	accum<A, VEC, NV> acc;
-	acc.zero();
-	uint32_t row = rg.row0;
-	uint32_t s = rg.e0 / U;
-	const uint32_t s_end = s + rg.len / U;
-	uint32_t raw[U];
-	ld_idx<U>(a.col, s, raw);
-	for (; s < s_end; s++) {
-		A w[U];
-		if constexpr (!kBinary) ld_w<WT, A, U>(a.val, s, w);
-		// issue this step's gathers
-		xvec<XT, VEC> x[U][NV];
-		A sc[U];
-		uint32_t ends = 0;
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			const uint32_t c = raw[u] & kIdxMask;
-			const bool hot = raw[u] & kHot;
-			const XT *xr = (hot ? H : X) + int64_t(c) * (hot ? int64_t(a.hot_ld) : a.ldx) + colbase;
-			const uint64_t pol = hot ? pol_hot : pol_cold;
-			if constexpr (NV == 1) {
-				// 16-byte lanes: every lane of a group owns a valid vector
-				x[u][0] = ld_x_hint<XT, VEC>(xr, pol);
-			} else {
-#pragma unroll
-				for (int v = 0; v < NV; v++)
-					if (v < a.nv && colbase + v * stride < a.k)
-						x[u][v] = ld_x_hint<XT, VEC>(xr + v * stride, pol);
-			}
-			if constexpr (SCALE_IN) sc[u] = hot ? A(1) : static_cast<const A *>(a.s_in)[c];
-			ends |= (raw[u] >> 31) << u;
-		}
-		// the next step's column ids load while the gathers are in flight
-		if (s + 1 < s_end) ld_idx<U>(a.col, s + 1, raw);
-		// add up in entry order; a set end flag closes the row
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-#pragma unroll
-			for (int v = 0; v < NV; v++)
-				if (NV == 1 || (v < a.nv && colbase + v * stride < a.k)) {
-					// (x * s_in) * w, rounded per step like scale_rows then SpMM;
-					// for hot entries x * s_in was rounded by the pack
-					if constexpr (SCALE_IN && !kBinary) acc.template add<XT, 2>(v, x[u][v], sc[u], w[u]);
-					else if constexpr (SCALE_IN) acc.template add<XT, 1>(v, x[u][v], sc[u], A(1));
-					else if constexpr (!kBinary) acc.template add<XT, 1>(v, x[u][v], w[u], A(1));
-					else acc.template add<XT, 0>(v, x[u][v], A(1), A(1));
-				}
-			const bool end = runs && ((ends >> u) & 1u);
-			if constexpr (EPI) {
-				static_assert(NV == 1 && VEC == 1 && std::is_same<A, float>::value, "PageRank: k = 1, FP32");
-				if (end && !((__ldg(e.heavy_mask + (row >> 5)) >> (row & 31)) & 1u))
-					pr_update(e, int64_t(row), acc.get(0, 0), cnt);
-			} else if constexpr (NV == 1) {
-				// branch-free row close: predicated store, select-reset
-				YT *Yp = static_cast<YT *>(a.Y) + int64_t(row) * a.ldy + colbase;
-				A so = A(1);
-				if constexpr (SCALE_OUT) so = end ? static_cast<const A *>(a.s_out)[row] : A(1);
-				YT out[VEC];
-#pragma unroll
-				for (int i = 0; i < VEC; i++) {
-					A t = acc.get(0, i);
-					if constexpr (SCALE_OUT) t = acc_mul(t, so);
-					out[i] = from_acc<YT, A>(t);
-				}
-				st_y_if<YT, VEC>(Yp, out, end);
-			} else {
-				if (end) store_row<YT, A, VEC, NV, SCALE_OUT>(a, int32_t(row), colbase, acc);
-			}
-			acc.zero_if(end);
-			row += end;
-		}
-	}
-	if (!runs) {
-		A *p = static_cast<A *>(a.partial) + int64_t(rg.slot) * kPartialStride;
-#pragma unroll
-		for (int v = 0; v < NV; v++)
-			if (v < a.nv && colbase + v * stride < a.k)
-#pragma unroll
-				for (int i = 0; i < VEC; i++) p[colbase + v * stride + i] = acc.get(v, i);
-	}
-}
-
-template <class XT, class YT, class A, class WT, int VEC, int NV, int U, bool SCALE_IN, bool SCALE_OUT,
-		bool EPI = false>
-__global__ void __launch_bounds__(kThreads, sizeof(XT) == 2 ? FMX_SPMM_MIN_BLOCKS_2B : FMX_SPMM_MIN_BLOCKS)
-spmm_kernel(const spmm_args a, const pr_epi e)
-{
-	if constexpr (EPI) {
-		if (e.state[1]) return;           // converged in an earlier iteration
-	}
-	const int lane = threadIdx.x & 31;
-	const uint32_t gw = (blockIdx.x * kThreads + threadIdx.x) >> 5;
-	const uint32_t nw = (gridDim.x * kThreads) >> 5;
-	const int G = a.G, R = a.R;
-	const int grp = lane / G;
-	if (grp >= R) return;
-	const int colbase = (lane - grp * G) * VEC;
-	const uint32_t gg = gw * uint32_t(R) + uint32_t(grp);
-	const uint32_t ng = nw * uint32_t(R);
-	const uint64_t pol_hot = policy_evict_last(), pol_cold = policy_evict_first();
-	unsigned cnt = 0;
-	for (uint32_t r = gg; r < a.n_ranges; r += ng)
-		run_range<XT, YT, A, WT, VEC, NV, U, SCALE_IN, SCALE_OUT, EPI>(a, a.ranges[r], colbase, pol_hot, pol_cold,
-				e, cnt);
-	if constexpr (EPI) {
-		// G = 1: every lane of the warp is a row group and reaches this point
-		cnt = __reduce_add_sync(0xffffffffu, cnt);
-		if (lane == 0 && cnt) atomicAdd(e.state, (unsigned long long)cnt);
-	}
-}
-
 // ---------------------------------------------------------------------------
-// 32-byte lanes (the main path for row panels of 32, 64 or 128 bytes).
+// The row kernel: lane groups walk ranges.
 //
-// A lane owns 32 bytes of every X row it gathers (8 FP32 or 16 BF16
-// elements), so a row panel of P bytes takes G = P / 32 lanes (1, 2 or 4) and
-// a warp runs 32 / G lane groups.  Each entry costs one 256-bit load per lane
-// and one decode per lane (the 16-byte-lane kernel spends a decode on every
-// 16 bytes); a warp-wide load still touches one 128-byte line per row.
-// Loads use no L2 policy: the measured gain of the hot/cold hints did not pay
-// for selecting them per entry.  The arithmetic is the 16-byte-lane kernel's
-// (products rounded, adds in entry order as packed FP32 pairs), so results
-// are bit-identical.
+// A lane owns VN elements of every X row it gathers, so a panel of k columns
+// takes G = k / VN lanes and a warp runs 32 / G groups.  Groups take ranges
+// round-robin and walk them U entries a step: all of a step's gathers, and
+// the next step's column ids, are in flight before its adds.  Any width runs
+// in whole lanes: VN is the widest unit that divides the rows (lane_width).
+//
+// What bounds it: the L1 data pipe (a gathered row costs about one data-pipe
+// cycle to return and half a cycle of tag output, whatever lanes ask for it)
+// and instruction issue.  Measured by ncu at R-MAT scale 22, k = 16 FP32: the
+// former 32-byte lanes with 4 gathers in flight kept the pipe 82 % busy at
+// 458 us with 106M wavefronts; 16-byte lanes with 8 in flight need 81M.  The
+// row close is a branch: predicated stores cost every entry the conversion.
+// Times of the former kernels -> this one (whole fmx_spmm, B200):
+//   FP32 k = 16, R-MAT scale 16 / 20 / 22 / 24   41 / 177 / 512 / 1855 ->
+//                                               27 / 130 / 411 / 1785 us
+//   FP64 k = 8, scale 22                         593 -> 430 us
+//   FP32 k = 10 / 33, scale 20                   427 / 1111 -> 156 / 684 us
+//   int64 k = 4 weighted, scale 20               177 -> 149 us
+//   D^-1/2 A D^-1/2, k = 16, symmetric scale 21  FP32 567 -> 471 us,
+//                                                BF16 531 -> 393 us
 // ---------------------------------------------------------------------------
-#ifndef FMX_WIDE_MIN_BLOCKS
-#define FMX_WIDE_MIN_BLOCKS 4
-#endif
-
 __device__ __forceinline__ void ld32_nc(const void *p, uint32_t (&r)[8])
 {
 	asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
 			: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
 			: "l"(p));
 }
-// 32-byte streaming store when `pred` holds (predicated, no branch).
-__device__ __forceinline__ void st32_if(void *p, const uint32_t (&v)[8], bool pred)
+
+// VN elements of T in one load (2 to 32 bytes).  Volatile: a step's loads
+// stay where they are written, all before the adds.
+template <class T, int VN>
+__device__ __forceinline__ xvec<T, VN> ld_n(const char *p)
 {
-	asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %9, 0;\n\t"
-			"@q st.global.cs.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n\t}"
-			:: "l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-			   "r"(uint32_t(pred)) : "memory");
+	xvec<T, VN> r;
+	if constexpr (VN * sizeof(T) == 32) {
+		uint32_t v[8];
+		ld32_nc(p, v);
+		memcpy(&r, v, 32);
+	} else if constexpr (VN * sizeof(T) == 16) {
+		uint32_t v[4];
+		asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
+		memcpy(&r, v, 16);
+	} else if constexpr (VN * sizeof(T) == 8) {
+		uint32_t v[2];
+		asm volatile("ld.global.nc.v2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
+		memcpy(&r, v, 8);
+	} else if constexpr (VN * sizeof(T) == 4) {
+		uint32_t v;
+		asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+		memcpy(&r, &v, 4);
+	} else {
+		static_assert(VN == 1 && sizeof(T) == 2, "one 2-byte element");
+		unsigned short v;
+		asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+		memcpy(&r, &v, 2);
+	}
+	return r;
 }
 
-// The VEC elements of one 32-byte load as FP32 (BF16 widened exactly).
-template <class XT, int VEC>
-__device__ __forceinline__ void widen(const uint32_t (&r)[8], float (&f)[VEC])
+// v = *p when `pred` holds (predicated, no branch)
+__device__ __forceinline__ void ld_if(float &v, const float *p, bool pred)
 {
-	if constexpr (sizeof(XT) == 4) {
+	asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+			: "+f"(v) : "l"(p), "r"(uint32_t(pred)));
+}
+__device__ __forceinline__ void ld_if(double &v, const double *p, bool pred)
+{
+	asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.f64 %0, [%1];\n\t}"
+			: "+d"(v) : "l"(p), "r"(uint32_t(pred)));
+}
+template <class A>
+__device__ __forceinline__ void ld_if(A &, const A *, bool) {}       // integers take no scales
+
+// U weights of consecutive entries
+template <class WT, class A, int U>
+__device__ __forceinline__ void ld_wn(const void *val, uint32_t e0, A (&w)[U])
+{
+	constexpr int per = int(16 / sizeof(WT));
+	const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const WT *>(val) + e0);
 #pragma unroll
-		for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[i]);
-	} else {
+	for (int q = 0; q < U / per; q++) {
+		const uint4 a = __ldg(p + q);
+		WT t[per];
+		memcpy(t, &a, 16);
 #pragma unroll
-		for (int i = 0; i < 8; i++) {
-			f[2 * i] = __uint_as_float(r[i] << 16);
-			f[2 * i + 1] = __uint_as_float(r[i] & 0xFFFF0000u);
-		}
+		for (int i = 0; i < per; i++) w[q * per + i] = A(t[i]);
 	}
 }
 
-template <class XT, class YT, class WT, int U, bool SCALE_IN, bool SCALE_OUT>
-__device__ __forceinline__ void run_range_wide(const spmm_args &a, const range_t rg, int colbase)
+// One range, U entries per step: the gathers (and scales, weights and the
+// next step's column ids) of a step are all issued before its adds.  Entries
+// of chunks carry no end flag, so only row runs store.
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
+__device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, int colbase)
 {
-	constexpr int VEC = int(32 / sizeof(XT));
 	constexpr bool kBinary = std::is_void<WT>::value;
+	static_assert(U % kStep == 0, "whole id loads");
 	const char *Xb = static_cast<const char *>(a.X) + size_t(colbase) * sizeof(XT);
 	const char *Hb = static_cast<const char *>(a.xhot) + size_t(colbase) * sizeof(XT);
-	const uint32_t xs = uint32_t(a.ldx) * uint32_t(sizeof(XT)), hs = uint32_t(a.hot_ld) * uint32_t(sizeof(XT));
-	char *Yb = static_cast<char *>(a.Y) + size_t(colbase) * sizeof(YT);
-	const uint64_t ys = uint64_t(a.ldy) * sizeof(YT);
-	const bool runs = rg.slot == kNoSlot;
-	uint64_t p[VEC / 2];
+	// 32-bit row strides (one wide multiply-add per address); one-element
+	// lanes also take the strides beyond 4 GB
+	typedef typename std::conditional<VN == 1, uint64_t, uint32_t>::type stride_t;
+	const stride_t xs = stride_t(a.ldx) * stride_t(sizeof(XT)), hs = stride_t(a.hot_ld) * stride_t(sizeof(XT));
+	YT *yp = static_cast<YT *>(a.Y) + int64_t(rg.row0) * a.ldy + colbase;
+	const A *sop = SO ? static_cast<const A *>(a.s_out) + rg.row0 : nullptr;
+	accum<A, VN, 1> acc;
+	acc.zero();
+	uint32_t e = rg.e0;
+	const uint32_t e_end = e + rg.len;
+	auto ids = [&](uint32_t at, uint32_t (&r)[U]) {
 #pragma unroll
-	for (int i = 0; i < VEC / 2; i++) p[i] = 0;
-	uint32_t row = rg.row0;
-	// pairs of 4-entry steps (a range is a whole number of kStep = 8
-	// entries): one 32-byte load of 8 column ids, and of 8 weights, per lane
-	// per pair, issued with the first step's gathers; the next pair's column
-	// ids load with the second step's gathers
-	static_assert(U == 4 && kStep == 2 * U, "pairs of 4-entry steps");
-	uint32_t s = rg.e0 / kStep;
-	const uint32_t s_end = s + rg.len / kStep;
-	uint32_t raw8[2 * U];
-	ld32_nc(a.col + size_t(s) * kStep, raw8);
-	for (; s < s_end; s++) {
-		uint32_t w8[2 * U];
-		if constexpr (!kBinary) ld32_nc(static_cast<const WT *>(a.val) + size_t(s) * kStep, w8);
+		for (int q = 0; q < U / kStep; q++) {
+			// past the end: entries of the zero row
+			uint32_t t[8] = {kHot, kHot, kHot, kHot, kHot, kHot, kHot, kHot};
+			if (at + kStep * q < e_end) ld32_nc(a.col + at + kStep * q, t);
 #pragma unroll
-		for (int half = 0; half < 2; half++) {
-		float w[U];
+			for (int i = 0; i < kStep; i++) r[kStep * q + i] = t[i];
+		}
+	};
+	uint32_t raw[U];
+	ids(e, raw);
+	while (true) {
+		xvec<XT, VN> x[U];
+		A sc[SI ? U : 1], w[kBinary ? 1 : U], so[SO ? U : 1];
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t c = raw[u] & kIdxMask;
+			const bool hot = raw[u] & kHot;
+			x[u] = ld_n<XT, VN>((hot ? Hb : Xb) + uint64_t(c) * (hot ? hs : xs));
+		}
+		// the scales that this step needs, loaded with its rows: s_in of cold
+		// entries (the pack's rows carry theirs) and s_out of the rows that
+		// close in it
+		uint32_t all = raw[0], any = raw[0];
+#pragma unroll
+		for (int u = 1; u < U; u++) {
+			all &= raw[u];
+			any |= raw[u];
+		}
+		// steps without a cold entry skip the scales (4-byte types: the second
+		// copy of the sums spills in the others, BF16 695 against 393 us at
+		// scale 21)
+		const bool cold = SI && (sizeof(XT) != 4 || !(all & kHot));
+		if constexpr (SI)
+			if (cold) {
+#pragma unroll
+				for (int u = 0; u < U; u++) {
+					sc[u] = A(1);
+					ld_if(sc[u], static_cast<const A *>(a.s_in) + (raw[u] & kIdxMask), !(raw[u] & kHot));
+				}
+			}
+		if constexpr (SO)
+			if (int32_t(any) < 0) {
+#pragma unroll
+				for (int u = 0; u < U; u++) {
+					ld_if(so[u], sop, raw[u] >> 31);
+					sop += raw[u] >> 31;
+				}
+			}
 		if constexpr (!kBinary) {
 #pragma unroll
-			for (int u = 0; u < U; u++) w[u] = __uint_as_float(w8[half * U + u]);
-		}
-		uint32_t xv[U][8];
-		float sc[U];
-		uint32_t ends = 0;
+			for (int q = 0; q < U / kStep; q++) {
+				A t[kStep] = {};
+				if (e + kStep * q < e_end) ld_wn<WT, A, kStep>(a.val, e + kStep * q, t);
 #pragma unroll
-		for (int u = 0; u < U; u++) {
-			const uint32_t rw = raw8[half * U + u];
-			const uint32_t c = rw & kIdxMask;
-			const bool hot = rw & kHot;
-			ld32_nc((hot ? Hb : Xb) + uint64_t(c) * (hot ? hs : xs), xv[u]);
-			if constexpr (SCALE_IN) sc[u] = hot ? 1.f : static_cast<const float *>(a.s_in)[c];
-			ends |= (rw >> 31) << u;
-		}
-		if (half == 1 && s + 1 < s_end) ld32_nc(a.col + size_t(s + 1) * kStep, raw8);
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			float f[VEC];
-			widen<XT, VEC>(xv[u], f);
-#pragma unroll
-			for (int i = 0; i < VEC / 2; i++) {
-				float t0 = f[2 * i], t1 = f[2 * i + 1];
-				// (x * s_in) * w, each product rounded, like scale_rows then SpMM
-				if constexpr (SCALE_IN) { t0 = __fmul_rn(t0, sc[u]); t1 = __fmul_rn(t1, sc[u]); }
-				if constexpr (!kBinary) { t0 = __fmul_rn(t0, w[u]); t1 = __fmul_rn(t1, w[u]); }
-				p[i] = add2(p[i], pack2(t0, t1));
+				for (int i = 0; i < kStep; i++) w[kStep * q + i] = t[i];
 			}
-			const bool end = runs && ((ends >> u) & 1u);
-			float so = 1.f;
-			if constexpr (SCALE_OUT) so = end ? static_cast<const float *>(a.s_out)[row] : 1.f;
-			float o[VEC];
+		}
+		e += U;
+		uint32_t nraw[U];
+		ids(e, nraw);
+		auto sums = [&](auto scaled) {
+			constexpr bool kSc = decltype(scaled)::value;
 #pragma unroll
-			for (int i = 0; i < VEC / 2; i++) {
-				unpack2(p[i], o[2 * i], o[2 * i + 1]);
-				if constexpr (SCALE_OUT) { o[2 * i] = __fmul_rn(o[2 * i], so); o[2 * i + 1] = __fmul_rn(o[2 * i + 1], so); }
-			}
-			char *yp = Yb + uint64_t(row) * ys;
-			if constexpr (sizeof(YT) == 4) {
+			for (int u = 0; u < U; u++) {
+				// (x * s_in) * w, rounded per step like scale_rows then SpMM
+				if constexpr (kSc && !kBinary) acc.template add<XT, 2>(0, x[u], sc[u], w[u]);
+				else if constexpr (kSc) acc.template add<XT, 1>(0, x[u], sc[u], A(1));
+				else if constexpr (!kBinary) acc.template add<XT, 1>(0, x[u], w[u], A(1));
+				else acc.template add<XT, 0>(0, x[u], A(1), A(1));
+				if (int32_t(raw[u]) < 0) {
+					YT out[VN];
 #pragma unroll
-				for (int h = 0; h < VEC / 8; h++) {
-					uint32_t v[8];
-#pragma unroll
-					for (int i = 0; i < 8; i++) v[i] = __float_as_uint(o[8 * h + i]);
-					st32_if(yp + 32 * h, v, end);
+					for (int i = 0; i < VN; i++) {
+						A v = acc.get(0, i);
+						if constexpr (SO) v = acc_mul(v, so[u]);
+						out[i] = from_acc<YT, A>(v);
+					}
+					st_y<YT, VN>(yp, out);
+					yp += a.ldy;
+					acc.zero();
 				}
-			} else {
-				uint32_t v[8];
-#pragma unroll
-				for (int i = 0; i < 8; i++) {
-					__nv_bfloat162 b2 = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-					memcpy(&v[i], &b2, 4);
-				}
-				st32_if(yp, v, end);
 			}
+		};
+		if constexpr (SI && sizeof(XT) != 4) {
+			sums(std::true_type{});
+		} else if constexpr (SI) {
+			if (cold) sums(std::true_type{});
+			else sums(std::false_type{});
+		} else {
+			sums(std::false_type{});
+		}
+		if (e >= e_end) break;
 #pragma unroll
-			for (int i = 0; i < VEC / 2; i++) p[i] = end ? 0ull : p[i];
-			row += end;
-		}
-		}
+		for (int u = 0; u < U; u++) raw[u] = nraw[u];
 	}
-	if (!runs) {
-		float *q = static_cast<float *>(a.partial) + int64_t(rg.slot) * kPartialStride + colbase;
+	if (rg.slot != kNoSlot) {
+		A *p = static_cast<A *>(a.partial) + int64_t(rg.slot) * kPartialStride + colbase;
 #pragma unroll
-		for (int i = 0; i < VEC / 2; i++) unpack2(p[i], q[2 * i], q[2 * i + 1]);
+		for (int i = 0; i < VN; i++) p[i] = acc.get(0, i);
 	}
 }
 
-template <class XT, class YT, class WT, int U, bool SCALE_IN, bool SCALE_OUT>
-__global__ void __launch_bounds__(kThreads, FMX_WIDE_MIN_BLOCKS) spmm_wide_kernel(const spmm_args a)
+// Threads and resident blocks per SM: at most 24 warps (FP32 rows in 16-byte
+// lanes: 24 warps 411 us, 20 warps 429 us at scale 22), fewer where the loads
+// in flight need the registers (spills cost more than the warps: BF16 with
+// 24 warps 801 us against 446 us with 20).
+constexpr int kLaneThreads = 128;
+constexpr int lane_blocks(int bytes, bool scaled, int esize)
 {
-	constexpr int VEC = int(32 / sizeof(XT));
+	return bytes == 32 ? (scaled ? 4 : 3) : (scaled && esize == 8) ? 4 : (scaled || esize == 2) ? 5 : 6;
+}
+// Entries per step: 16 in lanes of at most 8 bytes of an unweighted, unscaled
+// product (small or odd panels: R-MAT scale 18, k = 5, 39 against 43 us with
+// 8), else 8.
+constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 && esize >= 4 && plain ? 16 : 8; }
+
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
+__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT))))
+spmm_lane_kernel(const spmm_args a)
+{
 	const int lane = threadIdx.x & 31;
-	const uint32_t gw = (blockIdx.x * kThreads + threadIdx.x) >> 5;
-	const uint32_t nw = (gridDim.x * kThreads) >> 5;
 	const int G = a.G, R = a.R;
 	const int grp = lane / G;
 	if (grp >= R) return;
-	const int colbase = (lane - grp * G) * VEC;
-	const uint32_t gg = gw * uint32_t(R) + uint32_t(grp);
-	const uint32_t ng = nw * uint32_t(R);
-	for (uint32_t r = gg; r < a.n_ranges; r += ng)
-		run_range_wide<XT, YT, WT, U, SCALE_IN, SCALE_OUT>(a, a.ranges[r], colbase);
+	const int colbase = (lane - grp * G) * VN;
+	constexpr uint32_t wpb = kLaneThreads / 32;
+	const uint32_t wib = threadIdx.x >> 5;
+	const uint32_t ng = gridDim.x * wpb * uint32_t(R);
+	// full rounds give a block neighbouring ranges; the last, partial one is
+	// dealt out over the blocks (a round of neighbours left some SMs idle
+	// through the tail: 528 -> 488 us for the BF16 operator at scale 21)
+	const uint32_t g0 = (blockIdx.x * wpb + wib) * uint32_t(R) + uint32_t(grp);
+	const uint32_t g1 = (wib * gridDim.x + blockIdx.x) * uint32_t(R) + uint32_t(grp);
+	uint32_t base = 0;
+	for (; base + ng <= a.n_ranges; base += ng)
+		run_range<XT, YT, A, WT, VN, U, SI, SO>(a, a.ranges[base + g0], colbase);
+	if (base + g1 < a.n_ranges)
+		run_range<XT, YT, A, WT, VN, U, SI, SO>(a, a.ranges[base + g1], colbase);
 }
 
 // k = 1 (SpMV): a warp per range.  The 32 lanes load the range's column ids
@@ -1334,11 +1200,11 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 // ---------------------------------------------------------------------------
 
 template <class K>
-static unsigned persistent_blocks(K kernel, int device)
+static unsigned persistent_blocks(K kernel, int device, int threads)
 {
 	int sms = 0, per = 0;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kThreads, 0);
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
 	return unsigned(std::max(1, sms) * std::max(1, per));
 }
 
@@ -1346,19 +1212,15 @@ static unsigned persistent_blocks(K kernel, int device)
 // slots per kernel instantiation, indexed by device; racing first calls
 // compute the same value).
 template <class K>
-static unsigned cached_blocks(std::atomic<unsigned> &slot, K kernel, int device)
+static unsigned cached_blocks(std::atomic<unsigned> &slot, K kernel, int device, int threads)
 {
 	unsigned b = slot.load(std::memory_order_relaxed);
 	if (!b) {
-		b = persistent_blocks(kernel, device);
+		b = persistent_blocks(kernel, device, threads);
 		slot.store(b, std::memory_order_relaxed);
 	}
 	return b;
 }
-
-#ifndef FMX_SPMM_STEP
-#define FMX_SPMM_STEP 4                  // entries gathered per stream step (4 or 8)
-#endif
 
 // Run launch(args) over the part's ranges: once for a resident entry stream;
 // slice by slice for a streamed part.  Each slice is copied from pinned host
@@ -1398,61 +1260,54 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 	return FMX_OK;
 }
 
-template <class XT, class YT, class A, class WT, int VEC, int NV, bool SI, bool SO>
-static int launch_one(const gpu_part &p, const spmm_args &a, cudaStream_t st)
+template <class XT, class YT, class A, class WT, int VN, bool SI, bool SO>
+static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
-	auto kern = spmm_kernel<XT, YT, A, WT, VEC, NV, FMX_SPMM_STEP, SI, SO>;
+	constexpr int U = lane_step(VN * int(sizeof(XT)), int(sizeof(XT)), std::is_void<WT>::value && !SI && !SO);
+	auto kern = spmm_lane_kernel<XT, YT, A, WT, VN, U, SI, SO>;
 	static std::atomic<unsigned> blocks[64];
-	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device);
-	kern<<<b, kThreads, 0, st>>>(a, pr_epi{});
+	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kLaneThreads);
+	kern<<<b, kLaneThreads, 0, st>>>(a);
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
 }
 
-template <class XT, class YT, class WT, bool SI, bool SO>
-static int launch_wide(const gpu_part &p, const spmm_args &a, cudaStream_t st)
+template <class XT, class YT, class A, class WT, int VN>
+static int launch_lanes_scaled(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
-	auto kern = spmm_wide_kernel<XT, YT, WT, 4, SI, SO>;
-	static std::atomic<unsigned> blocks[64];
-	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device);
-	kern<<<b, kThreads, 0, st>>>(a);
-	CUDA_TRY(cudaGetLastError());
-	return FMX_OK;
+	if constexpr (std::is_floating_point<A>::value && (sizeof(XT) == 4 || VN * sizeof(XT) <= 16)) {
+		if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true>(p, a, st);
+		if (a.s_in) return launch_lanes<XT, YT, A, WT, VN, true, false>(p, a, st);
+		if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true>(p, a, st);
+	}
+	return launch_lanes<XT, YT, A, WT, VN, false, false>(p, a, st);
 }
 
-template <class XT, class YT, class A, class WT, int VEC, int NV>
-static int launch_t(const gpu_part &p, spmm_args a, bool sin, bool sout, cudaStream_t st, bool wide = false)
-{
-	if (int rc = launch_pack<XT, A>(p, static_cast<const XT *>(a.X), a.ldx, a.k, static_cast<XT *>(p.xhot), a.hot_ld,
-			sin ? static_cast<const A *>(a.s_in) : nullptr, st))
-		return rc;
-	int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
-		if constexpr (std::is_same<A, float>::value &&
-				(sizeof(XT) == 4 || (sizeof(YT) == 2 && std::is_void<WT>::value)) &&
-				(std::is_same<WT, void>::value || std::is_same<WT, float>::value)) {
-			if (wide) {
-				if (sin && sout) return launch_wide<XT, YT, WT, true, true>(p, sa, st);
-				if (sin) return launch_wide<XT, YT, WT, true, false>(p, sa, st);
-				if (sout) return launch_wide<XT, YT, WT, false, true>(p, sa, st);
-				return launch_wide<XT, YT, WT, false, false>(p, sa, st);
-			}
-		}
-		if (sin && sout) return launch_one<XT, YT, A, WT, VEC, NV, true, true>(p, sa, st);
-		if (sin) return launch_one<XT, YT, A, WT, VEC, NV, true, false>(p, sa, st);
-		if (sout) return launch_one<XT, YT, A, WT, VEC, NV, false, true>(p, sa, st);
-		return launch_one<XT, YT, A, WT, VEC, NV, false, false>(p, sa, st);
-	});
-	if (rc) return rc;
-	if (sout) rc = launch_fixup<YT, A, true>(p, static_cast<const A *>(a.partial), static_cast<YT *>(a.Y), a.ldy, a.k,
-			static_cast<const A *>(a.s_out), st);
-	else rc = launch_fixup<YT, A, false>(p, static_cast<const A *>(a.partial), static_cast<YT *>(a.Y), a.ldy, a.k,
-			nullptr, st);
-	if (rc) return rc;
-	return FMX_OK;
-}
+static bool aligned_to(const void *p, size_t n) { return (reinterpret_cast<uintptr_t>(p) % n) == 0; }
 
-static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-static bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
+// Elements per lane for a call: the widest unit of at most 16 bytes that
+// every X and Y row is made of and starts on (stores go in units of up to 16
+// bytes), or 32 bytes where that measured faster: FP32 with row scales (471
+// against 528 us at R-MAT scale 21, k = 16: the scales cost instructions per
+// entry, which wider lanes halve), and unscaled rows of 96 bytes or more
+// (FP32 k = 32 weighted 786 against 882 us, FP64 k = 16 701 against 784 us at
+// scale 22), but not shorter ones (k = 16 FP32 507 against 412 us).
+template <class XT, class YT>
+static int lane_width(const void *X, int64_t ldx, const void *Y, int64_t ldy, int64_t k, bool scaled)
+{
+	if (uint64_t(ldx) * sizeof(XT) >= (1ull << 32)) return 1;
+	auto fits = [&](int vn) {
+		return k % vn == 0 && ldx % vn == 0 && aligned_to(X, vn * sizeof(XT)) && (ldy * sizeof(YT)) % std::min<size_t>(16, vn * sizeof(YT)) == 0 &&
+				aligned_to(Y, std::min<size_t>(16, vn * sizeof(YT)));
+	};
+	constexpr int V32 = int(32 / sizeof(XT)), V16 = V32 / 2;
+	const bool f32 = std::is_same<XT, float>::value;
+	const int64_t row = std::min<int64_t>(k * int64_t(sizeof(XT)), kPanelBytes);
+	if (sizeof(XT) != 2 && (scaled ? f32 : row >= 96) && fits(V32)) return V32;
+	int vn = V16;
+	while (vn > 1 && !fits(vn)) vn /= 2;
+	return vn;
+}
 
 // Run one orientation over all column panels (kPanelBytes of X row each).
 // k = 1 without row scales: pack, the warp-per-range SpMV, fixup.
@@ -1469,7 +1324,7 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 	a.Y = Y;
 	a.partial = partial;
 	a.ldx = ldx; a.ldy = ldy; a.k = 1;
-	a.G = 1; a.R = 32; a.nv = 1;
+	a.G = 1; a.R = 32;
 	a.n_ranges = p.n_ranges;
 	const unsigned pb = unsigned(std::min<uint64_t>((uint64_t(p.n_hot) + 256) / 256, 148ull * 16));
 	pack_hot_kernel<T, T, false><<<pb, 256, 0, st>>>(p.hot_col, p.n_hot, X, ldx, 1, static_cast<T *>(xhot), 1,
@@ -1477,7 +1332,7 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 	CUDA_TRY(cudaGetLastError());
 	auto kern = spmv_kernel<T, WT, EPI>;
 	static std::atomic<unsigned> blocks[64];
-	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device);
+	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kThreads);
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
 			kern<<<b, kThreads, 0, st>>>(sa, e);
 			CUDA_TRY(cudaGetLastError());
@@ -1489,62 +1344,49 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 
 template <class XT, class YT, class A, class WT>
 static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int64_t ldy, int64_t k,
-		const void *sin, const void *sout, cudaStream_t st)
+		const void *sin, const void *sout, cudaStream_t st, void *xhot = nullptr, void *partial = nullptr)
 {
+	if (!xhot) xhot = p.xhot;
+	if (!partial) partial = p.partial;
 	if constexpr (std::is_same<XT, A>::value && std::is_same<YT, A>::value && std::is_floating_point<A>::value) {
 		if (k == 1 && !sin && !sout)
-			return run_spmv<A, WT, false>(p, static_cast<const A *>(X), ldx, static_cast<A *>(Y), ldy, st);
+			return run_spmv<A, WT, false>(p, static_cast<const A *>(X), ldx, static_cast<A *>(Y), ldy, st, pr_epi{}, xhot,
+					partial);
 	}
-	constexpr int VEC = int(16 / sizeof(XT));
-	constexpr int kPanel = kPanelBytes / int(sizeof(XT));
-	// 16-byte vectors along k when every X and Y row starts 16-byte aligned
-	// and k is a multiple of VEC; otherwise scalar lanes.
-	const bool vec_ok = (k % VEC == 0) && (ldx % VEC == 0) && (ldy % VEC == 0) &&
-			aligned16(X) && aligned16(Y) && (VEC * sizeof(YT)) % 8 == 0;
-	for (int64_t c0 = 0; c0 < k; c0 += kPanel) {
-		const int kp = int(std::min<int64_t>(kPanel, k - c0));
+	const int vn = lane_width<XT, YT>(X, ldx, Y, ldy, k, sin || sout);
+	constexpr int V32 = int(32 / sizeof(XT));
+	// column panels of at most kPanelBytes of X row, and 32 lanes
+	const int panel = std::min(kPanelBytes / int(sizeof(XT)), 32 * vn);
+	for (int64_t c0 = 0; c0 < k; c0 += panel) {
+		const int kp = int(std::min<int64_t>(panel, k - c0));
 		spmm_args a{};
 		a.col = p.col; a.val = p.val; a.ranges = p.ranges;
 		a.X = static_cast<const XT *>(X) + c0;
-		a.xhot = p.xhot;
+		a.xhot = xhot;
 		a.hot_ld = kp;                // packed rows back to back (two 64-byte rows per line)
 		a.Y = static_cast<YT *>(Y) + c0;
-		a.s_in = sin; a.s_out = sout; a.partial = p.partial;
+		a.s_in = sin; a.s_out = sout; a.partial = partial;
 		a.ldx = ldx; a.ldy = ldy; a.k = kp;
 		a.n_ranges = p.n_ranges;
-		int rc;
-		// 32-byte lanes: FP32 accumulation, a panel of whole 32-byte lanes,
-		// X, Y and the packed rows 32-byte aligned
-		// (BF16 rows of 16 elements take the 16-byte lanes: measured at R-MAT
-		// scale 24, k = 16, one 32-byte lane per row loads an index group per
-		// lane and ran 2.2 ms against 1.8 ms)
-		// FP32, and unweighted BF16 with BF16 output (the eigensolver's
-		// correction SpMMs: 0.82 against 0.89 ms per call at scale 22,
-		// k = 16); BF16 into FP32 and weighted BF16 keep the 16-byte lanes,
-		// where the wider accumulators spill
-		constexpr bool kWideBf16 = sizeof(YT) == 2 && std::is_void<WT>::value;
-		const bool wide = std::is_same<A, float>::value && (sizeof(XT) == 4 || kWideBf16) && vec_ok &&
-				(kp * sizeof(XT)) % 32 == 0 &&
-				(ldx * sizeof(XT)) % 32 == 0 && (ldy * sizeof(YT)) % 32 == 0 && aligned32(a.X) && aligned32(a.Y);
-		if (wide) {
-			a.G = int(kp * sizeof(XT) / 32);     // 1, 2 or 4
-			a.R = 32 / a.G;
-			a.nv = 1;
-			rc = launch_t<XT, YT, A, WT, VEC, 1>(p, a, sin, sout, st, true);
-		} else if (vec_ok) {
-			a.G = kp / VEC;           // <= 8
-			a.R = 32 / a.G;
-			a.nv = 1;
-			rc = launch_t<XT, YT, A, WT, VEC, 1>(p, a, sin, sout, st);
-		} else {
-			int g = 1;
-			while (g < 32 && g * 4 < kp) g *= 2;
-			a.G = g;
-			a.R = 32 / g;
-			a.nv = (kp + g - 1) / g;   // <= 4
-			rc = launch_t<XT, YT, A, WT, 1, 4>(p, a, sin, sout, st);
-		}
-		if (rc) return rc;
+		a.G = kp / vn;
+		a.R = 32 / a.G;
+		if (int rc = launch_pack<XT, A>(p, static_cast<const XT *>(a.X), ldx, kp, static_cast<XT *>(xhot), kp,
+				static_cast<const A *>(sin), st))
+			return rc;
+		if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
+				switch (vn) {
+				case 1: return launch_lanes_scaled<XT, YT, A, WT, 1>(p, sa, st);
+				case 2: return launch_lanes_scaled<XT, YT, A, WT, 2>(p, sa, st);
+				case 4: return launch_lanes_scaled<XT, YT, A, WT, 4>(p, sa, st);
+				}
+				if constexpr (V32 >= 8) return launch_lanes_scaled<XT, YT, A, WT, 8>(p, sa, st);
+				return set_error(FMX_ERR_UNSUPPORTED, "no kernel for lanes of %d elements", vn);
+			}))
+			return rc;
+		const A *so = static_cast<const A *>(sout);
+		if (int rc = sout ? launch_fixup<YT, A, true>(p, static_cast<const A *>(partial), static_cast<YT *>(a.Y), ldy, kp, so, st)
+				: launch_fixup<YT, A, false>(p, static_cast<const A *>(partial), static_cast<YT *>(a.Y), ldy, kp, nullptr, st))
+			return rc;
 	}
 	return FMX_OK;
 }
@@ -2208,49 +2050,6 @@ static int noalloc_scratch(int device, void **ptr)
 	return FMX_OK;
 }
 
-template <class WT>
-static int run_noalloc(const gpu_part &p, const float *X, int64_t ldx, float *Y, int64_t ldy, int64_t k,
-		void *xhot, void *partial, cudaStream_t st)
-{
-	// the kernels fmx_spmm runs for the same call, on the fixed scratch
-	if (k == 1) return run_spmv<float, WT, false>(p, X, ldx, Y, ldy, st, pr_epi{}, xhot, partial);
-	constexpr int VEC = 4;
-	constexpr int kPanel = kPanelBytes / int(sizeof(float));
-	const bool vec_ok = (k % VEC == 0) && (ldx % VEC == 0) && (ldy % VEC == 0) && aligned16(X) && aligned16(Y);
-	for (int64_t c0 = 0; c0 < k; c0 += kPanel) {
-		const int kp = int(std::min<int64_t>(kPanel, k - c0));
-		spmm_args a{};
-		a.col = p.col; a.val = p.val; a.ranges = p.ranges;
-		a.X = X + c0;
-		a.xhot = xhot;
-		a.hot_ld = kp;
-		a.Y = Y + c0;
-		a.partial = partial;
-		a.ldx = ldx; a.ldy = ldy; a.k = kp;
-		a.n_ranges = p.n_ranges;
-		int rc = launch_pack<float, float>(p, X + c0, ldx, kp, static_cast<float *>(xhot), kp, nullptr, st);
-		if (rc) return rc;
-		if (vec_ok) {
-			a.G = kp / VEC;
-			a.R = 32 / a.G;
-			a.nv = 1;
-			rc = launch_one<float, float, float, WT, VEC, 1, false, false>(p, a, st);
-		} else {
-			int g = 1;
-			while (g < 32 && g * 4 < kp) g *= 2;
-			a.G = g;
-			a.R = 32 / g;
-			a.nv = (kp + g - 1) / g;
-			rc = launch_one<float, float, float, WT, 1, 4, false, false>(p, a, st);
-		}
-		if (rc) return rc;
-		const int frc = launch_fixup<float, float, false>(p, static_cast<const float *>(partial), Y + c0, ldy, kp,
-				nullptr, st);
-		if (frc) return frc;
-	}
-	return FMX_OK;
-}
-
 } // namespace fmx
 
 extern "C" int fmx_spmm_noalloc(const fmx_matrix *m, const float *X, int64_t ldx, float *Y, int64_t ldy,
@@ -2279,8 +2078,10 @@ extern "C" int fmx_spmm_noalloc(const fmx_matrix *m, const float *X, int64_t ldx
 		void *xhot = base;
 		void *partial = static_cast<char *>(base) + hot_bytes;
 		cudaStream_t st = static_cast<cudaStream_t>(stream);
-		rc = (p.prim == FMX_P_BOOL) ? run_noalloc<void>(p, X, ldx, Y, ldy, k, xhot, partial, st)
-		                            : run_noalloc<float>(p, X, ldx, Y, ldy, k, xhot, partial, st);
+		// the kernels fmx_spmm runs for the same call, on the fixed scratch
+		rc = (p.prim == FMX_P_BOOL)
+				? run_typed<float, float, float, void>(p, X, ldx, Y, ldy, k, nullptr, nullptr, st, xhot, partial)
+				: run_typed<float, float, float, float>(p, X, ldx, Y, ldy, k, nullptr, nullptr, st, xhot, partial);
 	}
 	if (cur != p.device) cudaSetDevice(cur);
 	return rc;

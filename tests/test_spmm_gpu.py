@@ -249,6 +249,45 @@ def test_spmv_kernel_matches_lane_group_kernel(torch_cuda, dtype):
         assert torch.equal(Y3[:, :1], Y1) and bool((Y3[:, 1:] == 7).all())
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64", "int32", "int64", "bfloat16"])
+@pytest.mark.parametrize("k", [2, 3, 5, 7, 12, 15, 24, 31, 32, 33, 40, 65])
+def test_lane_widths(torch_cuda, dtype, k):
+    """Every lane width and remainder of the row kernel: whole and odd panels,
+    operands that start off the vector grid (a column slice of a wider
+    block), rows of 0 to 256 entries, with and without row scales.  Integer
+    operands and power-of-two scales keep every sum exact, so each element
+    must equal the oracle's."""
+    torch = torch_cuda
+    tdt = getattr(torch, dtype)
+    n = 3001
+    src, dst = _graph(n, 15000, 40 + k, ((5, 256), (2999, 255), (77, 8), (78, 9)))
+    idx, mat = oracle.build_image(src, dst, None, block=(1024, 1024), dedup=True)
+    m = sparse_matrix.create(matrix_image.from_bytes(idx, mat), None, device=0)
+    rng = np.random.default_rng(k)
+    X = rng.integers(-8, 9, (n, k))
+    R = oracle.spmm(idx, mat, X.astype(np.float64))
+    scales = [(None, None)]
+    if tdt.is_floating_point:
+        s = np.ldexp(1.0, rng.integers(-2, 3, n))
+        sdt = torch.float64 if tdt == torch.float64 else torch.float32
+        sc = torch.from_numpy(s).to("cuda", sdt)
+        scales += [(sc, None), (None, sc), (sc, sc)]
+    for off, pad in ((0, 0), (1, 2), (4, 4)):
+        Xw = torch.zeros((n, off + k + pad), dtype=tdt, device="cuda")
+        Xw[:, off:off + k] = torch.from_numpy(X).to("cuda", tdt)
+        for si, so in scales:
+            Yw = torch.full((n, off + k + pad), 77, dtype=torch.float32 if tdt == torch.bfloat16 else tdt, device="cuda")
+            assert m.multiply(Xw[:, off:off + k], Yw[:, off:off + k], si, so), _lib.last_error()
+            want = R
+            if si is not None:
+                want = oracle.spmm(idx, mat, X * s[:, None])
+            if so is not None:
+                want = want * s[:, None]
+            got = Yw.cpu().double().numpy()
+            assert np.array_equal(got[:, off:off + k], want), (off, si is not None, so is not None)
+            assert (got[:, :off] == 77).all() and (got[:, off + k:] == 77).all()
+
+
 def test_host_buffers_e2e(torch_cuda):
     src, dst = _graph(5000, 40000, 21)
     idx, mat = oracle.build_image(src, dst, None, block=(1024, 1024), dedup=True)
