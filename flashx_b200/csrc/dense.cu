@@ -1101,44 +1101,72 @@ gram_dmma_kernel(const float *__restrict__ X, int64_t ldx, int M, const float *_
 // ---------------------------------------------------------------------------
 
 // T = R^{-1} with G = R^T R (upper Cholesky).  info = 0, or the 1-based
-// column whose pivot was not positive.  One CTA of 64 threads.
-__global__ void chol_inv_kernel(const double *__restrict__ G, int b, double *__restrict__ T, int *info)
+// column whose pivot was not positive.  One CTA, LDL^T by rows with the same
+// operations applied to the identity: a row i > k holds what is left of G's
+// upper triangle after step k and, left of it, its row of L^{-1}, so that
+// R^{-1} = L^{-T} D^{-1/2} needs no back substitution.
+//
+// What bounds it: the chain of b steps (a shared-memory read, an FP64
+// division, two FP64 multiply-adds and a barrier each, about 250 cycles).
+// Every element is a thread's own, so a step costs one barrier; the former left-looking form walked a dot product of up to k
+// dependent multiply-adds per pivot and per column, and inverted R column by
+// column on one thread each: 17.5 us at b = 16.
+//
+// With rel > 0, rel * max(diag G) is added to the diagonal of G first (the
+// shift of shifted CholQR), as a kernel of its own did before.
+constexpr int kCholThreads = 1024;
+__global__ void __launch_bounds__(kCholThreads) chol_inv_kernel(const double *__restrict__ G, int b,
+		double *__restrict__ T, int *info, double rel)
 {
-	extern __shared__ double dyn[];                  // two 64 x 65 FP64 matrices
-	double (*R)[65] = reinterpret_cast<double (*)[65]>(dyn);
-	double (*Ti)[65] = reinterpret_cast<double (*)[65]>(dyn + 64 * 65);
-	const int t = threadIdx.x;
-	for (int i = t; i < b * b; i += blockDim.x) R[i / b][i % b] = G[i];
+	extern __shared__ double dyn[];                  // b x (b + 1) FP64
+	const int ld = b + 1;
+	const int t = threadIdx.x, nt = blockDim.x;
+	double shift = 0;
+	if (rel > 0) {
+		for (int i = 0; i < b; i++) shift = fmax(shift, G[i * b + i]);
+		shift *= rel;
+	}
+	// a thread keeps its elements (one up to b = 32, four at b = 64) in
+	// registers; a row goes to shared memory when it becomes the pivot row
+	constexpr int Q = 64 * 64 / kCholThreads;
+	double v[Q];
+	int ei[Q], ej[Q];
+#pragma unroll
+	for (int q = 0; q < Q; q++) {
+		const int e = t + q * nt;
+		ei[q] = e < b * b ? e / b : -1;
+		ej[q] = e < b * b ? e - ei[q] * b : 0;
+		v[q] = ei[q] < 0 || ej[q] < ei[q] ? 0.0 : G[e] + (ei[q] == ej[q] ? shift : 0.0);
+		if (ei[q] == 0) dyn[ej[q]] = v[q];
+	}
 	__syncthreads();
-	__shared__ int bad;
-	if (t == 0) bad = 0;
-	__syncthreads();
-	for (int k = 0; k < b; k++) {
-		if (t == 0) {
-			double d = R[k][k];
-			for (int p = 0; p < k; p++) d -= R[p][k] * R[p][k];
-			if (!(d > 0) && !bad) bad = k + 1;
-			R[k][k] = d > 0 ? sqrt(d) : 1.0;
+	int bad = 0;
+	for (int k = 0; k + 1 < b; k++) {
+		const double *rk = dyn + k * ld;
+		double d = rk[k];
+		if (!(d > 0)) {
+			if (!bad) bad = k + 1;
+			d = 1.0;
 		}
-		__syncthreads();
-		for (int j = k + 1 + t; j < b; j += blockDim.x) {
-			double s = R[k][j];
-			for (int p = 0; p < k; p++) s -= R[p][k] * R[p][j];
-			R[k][j] = s / R[k][k];
+		const double inv = 1.0 / d;
+#pragma unroll
+		for (int q = 0; q < Q; q++) {
+			const int i = ei[q], j = ej[q];
+			// right of the diagonal: G's rows; left, up to column k: the rows
+			// of L^{-1}, whose diagonal is 1
+			if (i > k && (j <= k || j >= i)) v[q] = fma(-(rk[i] * inv), j == k ? 1.0 : rk[j], v[q]);
+			if (i == k + 1) dyn[i * ld + j] = v[q];
 		}
 		__syncthreads();
 	}
-	// inverse of the upper-triangular R, column by column
-	for (int j = t; j < b; j += blockDim.x) {
-		for (int i = b - 1; i >= 0; i--) {
-			if (i > j) { Ti[i][j] = 0; continue; }
-			double s = (i == j) ? 1.0 : 0.0;
-			for (int p = i + 1; p <= j; p++) s -= R[i][p] * Ti[p][j];
-			Ti[i][j] = s / R[i][i];
-		}
+	const double dl = dyn[(b - 1) * ld + b - 1];
+	if (!(dl > 0) && !bad) bad = b;
+	for (int e = t; e < b * b; e += nt) {
+		const int i = e / b, j = e - i * b;
+		const double d = dyn[j * ld + j];
+		const double rs = d > 0 ? 1.0 / sqrt(d) : 1.0;
+		T[e] = i > j ? 0.0 : (i == j ? rs : dyn[j * ld + i] * rs);
 	}
-	__syncthreads();
-	for (int i = t; i < b * b; i += blockDim.x) T[i] = Ti[i / b][i % b];
 	if (t == 0) *info = bad;
 }
 
@@ -1819,6 +1847,16 @@ int sms(int device)
 }
 
 } // namespace dense
+
+int dense_chol_inv_shifted(const double *G, int b, double *T, int *info, double rel, void *stream)
+{
+	// one element per thread up to b = 32
+	const int nt = std::min(dense::kCholThreads, (b * b + 31) / 32 * 32);
+	dense::chol_inv_kernel<<<1, nt, size_t(b) * (b + 1) * sizeof(double), static_cast<cudaStream_t>(stream)>>>(G, b, T, info, rel);
+	DCUDA_TRY(cudaGetLastError());
+	return FMX_OK;
+}
+
 } // namespace fmx
 
 using namespace fmx;
@@ -1968,11 +2006,7 @@ int fmx_dense_chol_inv(const double *G, int b, double *T, int *info, void *strea
 {
 	if (!G || !T || !info) return set_error(FMX_ERR_INVAL, "null argument");
 	if (b < 1 || b > 64) return set_error(FMX_ERR_UNSUPPORTED, "b in 1..64");
-	const int smem = 2 * 64 * 65 * int(sizeof(double));
-	DCUDA_TRY(cudaFuncSetAttribute(chol_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-	chol_inv_kernel<<<1, 64, smem, static_cast<cudaStream_t>(stream)>>>(G, b, T, info);
-	DCUDA_TRY(cudaGetLastError());
-	return FMX_OK;
+	return fmx::dense_chol_inv_shifted(G, b, T, info, 0.0, stream);
 }
 
 int fmx_dense_sym_eig(const double *H, int b, double *w, double *V, void *stream)

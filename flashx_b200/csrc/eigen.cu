@@ -594,17 +594,6 @@ __global__ void reduce_parts_kernel(const double *__restrict__ part, int nparts,
 	}
 }
 
-// G += rel * max(diag G) * I  (the shift of shifted CholQR: keeps the
-// Cholesky factor defined for numerically rank-deficient blocks)
-__global__ void shift_diag_kernel(double *G, int b, double rel)
-{
-	if (threadIdx.x == 0 && blockIdx.x == 0) {
-		double m = 0;
-		for (int i = 0; i < b; i++) m = fmax(m, G[i * b + i]);
-		for (int i = 0; i < b; i++) G[i * b + i] += rel * m;
-	}
-}
-
 __global__ void f64_to_f32_kernel(const double *a, float *o, int count)
 {
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) o[i] = float(a[i]);
@@ -798,11 +787,9 @@ struct solver {
 		float *outs[2] = {tmp, Q};
 		for (int p = 0; p < 2; p++) {
 			E_TRY(fmx_dense_gram(FMX_DENSE_F64, in, b, b, in, b, b, n, gpart, G, nullptr, st));
-			if (p == 0) {
-				shift_diag_kernel<<<1, 1, 0, st>>>(G, b, 1e-13);
-				ECUDA_TRY(cudaGetLastError());
-			}
-			E_TRY(fmx_dense_chol_inv(G, b, T, info + p, st));
+			// the first pass's shift keeps the factor defined for numerically
+			// rank-deficient blocks
+			E_TRY(dense_chol_inv_shifted(G, b, T, info + p, p == 0 ? 1e-13 : 0.0, st));
 			// The Gram stays FP64 in both modes: the filtered block can be
 			// ill-conditioned and the Cholesky needs its accuracy.  The update
 			// runs on the tensor cores in the low-precision phase (139 us at

@@ -91,6 +91,8 @@ int default_threads();
 // Stream-ordered workspace from the current device's library pool (freed
 // memory stays reserved for the next call; fmx_release_cached returns it).
 cudaError_t work_alloc(void **p, size_t bytes, cudaStream_t st);
+// fmx_dense_chol_inv of G + rel * max(diag G) * I (the shift of shifted CholQR)
+int dense_chol_inv_shifted(const double *G, int b, double *T, int *info, double rel, void *stream);
 
 // The device a matrix lives on.
 int matrix_device(const fmx_matrix *m);

@@ -175,13 +175,26 @@ __global__ void __launch_bounds__(kThreads) relu_grad_kernel(float *__restrict__
 	}
 }
 
-__global__ void sum_parts_kernel(const float *__restrict__ part, int nparts, int len, float *__restrict__ out)
+// out[j] = sum over the CTAs' partials.  A block takes 8 columns (32-byte
+// sectors), 128 threads share a column's partials and their sums are combined
+// by a fixed tree.  (One thread per column walking all 1184 partials took 48 us
+// at n = 100k.)
+__global__ void __launch_bounds__(1024) sum_parts_kernel(const float *__restrict__ part, int nparts, int len,
+		float *__restrict__ out)
 {
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-		float s = 0.f;
-		for (int p = 0; p < nparts; p++) s += part[size_t(p) * len + i];
-		out[i] = s;
+	__shared__ float red[128][8];
+	const int c = threadIdx.x & 7, r = threadIdx.x >> 3;
+	const int col = blockIdx.x * 8 + c;
+	float s = 0.f;
+	if (col < len)
+		for (int p = r; p < nparts; p += 128) s += part[size_t(p) * len + col];
+	red[r][c] = s;
+	__syncthreads();
+	for (int w = 64; w > 0; w >>= 1) {
+		if (r < w) red[r][c] += red[r + w][c];
+		__syncthreads();
 	}
+	if (r == 0 && col < len) out[col] = red[0][c];
 }
 
 // out (cols x rows) = in^T (rows x cols), small
@@ -204,41 +217,35 @@ __global__ void f32_to_f64_kernel(const float *a, double *o, int count)
 __global__ void __launch_bounds__(kThreads) loss_kernel(const double *__restrict__ G, const double *__restrict__ M,
 		int nev, float *__restrict__ P1, float *__restrict__ P2, double *__restrict__ loss)
 {
-	__shared__ double R[kOut][kOut], Ri[kOut][kOut], Gi[kOut][kOut], K[kMaxNev][kOut];
-	__shared__ double fred[kThreads];
+	__shared__ double A[kOut][kOut + 1], Gi[kOut][kOut], K[kMaxNev][kOut];
+	__shared__ double fred[kThreads / 32];
+	static_assert(kThreads == kOut * kOut, "a thread per element");
 	const int t = threadIdx.x;
-	if (t == 0) {
-		double tr = 0;
-		for (int i = 0; i < kOut; i++) tr += G[i * kOut + i];
-		const double shift = 1e-12 * (tr > 0 ? tr : 1.0);
-		// upper Cholesky G = R^T R
-		for (int k = 0; k < kOut; k++) {
-			double dkk = G[k * kOut + k] + shift;
-			for (int p = 0; p < k; p++) dkk -= R[p][k] * R[p][k];
-			R[k][k] = sqrt(dkk > shift ? dkk : shift);
-			for (int j = k + 1; j < kOut; j++) {
-				double s = G[k * kOut + j];
-				for (int p = 0; p < k; p++) s -= R[p][k] * R[p][j];
-				R[k][j] = s / R[k][k];
-			}
-			for (int j = 0; j < k; j++) R[k][j] = 0;
-		}
-		// Ri = R^-1 (upper triangular), column by column
-		for (int j = 0; j < kOut; j++)
-			for (int i = kOut - 1; i >= 0; i--) {
-				if (i > j) { Ri[i][j] = 0; continue; }
-				double s = (i == j) ? 1.0 : 0.0;
-				for (int p = i + 1; p <= j; p++) s -= R[i][p] * Ri[p][j];
-				Ri[i][j] = s / R[i][i];
-			}
-	}
+	const int ei = t / kOut, ej = t % kOut;
+	// G + shift = L D L^T, the row operations applied to the identity too
+	// (one element per thread, one barrier a step; the former Cholesky and
+	// inverse on one thread took 60 of the kernel's 68 us)
+	double tr = 0;
+	for (int i = 0; i < kOut; i++) tr += G[i * kOut + i];
+	const double shift = 1e-12 * (tr > 0 ? tr : 1.0);
+	double v = ej < ei ? 0.0 : G[t] + (ei == ej ? shift : 0.0);
+	if (ei == 0) A[0][ej] = v;
 	__syncthreads();
-	// Gi = Ri Ri^T
-	for (int e = t; e < kOut * kOut; e += kThreads) {
-		const int i = e / kOut, j = e % kOut;
+	for (int k = 0; k + 1 < kOut; k++) {
+		const double d = A[k][k] > shift ? A[k][k] : shift;
+		const double inv = 1.0 / d;
+		if (ei > k && (ej <= k || ej >= ei)) v = fma(-(A[k][ei] * inv), ej == k ? 1.0 : A[k][ej], v);
+		if (ei == k + 1) A[ei][ej] = v;
+		__syncthreads();
+	}
+	// Gi = L^-T D^-1 L^-1
+	{
 		double s = 0;
-		for (int p = 0; p < kOut; p++) s += Ri[i][p] * Ri[j][p];
-		Gi[i][j] = s;
+		for (int p = max(ei, ej); p < kOut; p++) {
+			const double d = A[p][p] > shift ? A[p][p] : shift;
+			s += (p == ei ? 1.0 : A[p][ei]) * (p == ej ? 1.0 : A[p][ej]) / d;
+		}
+		Gi[ei][ej] = s;
 	}
 	__syncthreads();
 	// K = M Gi
@@ -251,7 +258,8 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const double *__restrict
 	__syncthreads();
 	double f = 0;
 	for (int e = t; e < nev * kOut; e += kThreads) f += K[e / kOut][e % kOut] * M[e];
-	fred[t] = f;
+	for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+	if ((t & 31) == 0) fred[t / 32] = f;
 	const double sc = 2.0 / double(nev);
 	for (int e = t; e < nev * kOut; e += kThreads) P1[e] = float(-sc * K[e / kOut][e % kOut]);
 	for (int e = t; e < kOut * kOut; e += kThreads) {
@@ -263,7 +271,7 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const double *__restrict
 	__syncthreads();
 	if (t == 0) {
 		double s = 0;
-		for (int i = 0; i < kThreads; i++) s += fred[i];
+		for (int i = 0; i < kThreads / 32; i++) s += fred[i];
 		*loss = 1.0 - s / double(nev);
 	}
 }
@@ -551,7 +559,7 @@ int fmx_gnn_loss_grad(fmx_gnn *g, const fmx_matrix *m, const float *scale, const
 	// layer 1: H = relu(Z W1 + b1)
 	relu_grad_kernel<<<rparts, kThreads, 0, st>>>(dH, H, n, bpart);
 	GCUDA_TRY(cudaGetLastError());
-	sum_parts_kernel<<<1, kH, 0, st>>>(bpart, rparts, kH, g->g + kOffB1);
+	sum_parts_kernel<<<(kH + 7) / 8, 1024, 0, st>>>(bpart, rparts, kH, g->g + kOffB1);
 	GCUDA_TRY(cudaGetLastError());
 	G_TRY(fmx_dense_gram(precision, Z, kZ, kZ, dH, kH, kH, n, gpart, g->g + kOffW1, g->err, st));
 	if (loss) GCUDA_TRY(cudaMemcpyAsync(loss, dloss, sizeof(double), cudaMemcpyDeviceToHost, st));
