@@ -925,174 +925,210 @@ tc_gram_kernel(const float *__restrict__ X, int64_t ldx, int M, const float *__r
 	if (warp == 0) tmem_dealloc(tmem, ncols);
 }
 
-// G[i] = sum over the partials of part[p][i]: one warp per element, lane l
-// adding partials l, l + 32, ... and the lanes combined by a fixed xor tree
-// (deterministic for a given number of partials)
+// G[i] = sum over the partials of part[p][i]: a block takes 4 neighbouring
+// elements (32-byte sectors of FP64), 64 threads share an element's partials
+// and their sums are combined by a fixed tree (deterministic for a given
+// number of partials)
 template <class T>
-__global__ void gram_reduce_kernel(const T *part, int nparts, int MN, T *G)
+__global__ void __launch_bounds__(256) gram_reduce_kernel(const T *part, int nparts, int MN, T *G)
 {
-	const int lane = threadIdx.x & 31;
-	const int warps = int((gridDim.x * blockDim.x) >> 5);
-	for (int i = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < MN; i += warps) {
-		T s = 0;
-		for (int p = lane; p < nparts; p += 32) s += part[size_t(p) * MN + i];
-		for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		if (lane == 0) G[i] = s;
+	__shared__ T red[64][4];
+	const int c = threadIdx.x & 3, r = threadIdx.x >> 2;
+	const int i = blockIdx.x * 4 + c;
+	T s = 0;
+	if (i < MN) {
+#pragma unroll 4
+		for (int p = r; p < nparts; p += 64) s += part[size_t(p) * MN + i];
 	}
-}
-
-// ---------------------------------------------------------------------------
-// FP64 Gram on CUDA cores: part[cta] = sum over the CTA's rows of x^T w (FP64)
-// Each thread owns a 4 x 4 block of G and every `groups`-th row: per row it
-// loads its 4 columns of x and of w straight from global memory (16-byte
-// loads when the leading dimensions allow, L1-shared by the threads of the
-// same row) and does 16 FP64 FMAs; four rows are in flight per thread.  The
-// row groups' blocks are added in a fixed order at the end (deterministic).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float4 ld4_guard(const float *p, int c, int lim, bool vec)
-{
-	if (vec && c + 3 < lim) return *reinterpret_cast<const float4 *>(p + c);
-	float4 v;
-	v.x = c < lim ? p[c] : 0.f;
-	v.y = c + 1 < lim ? p[c + 1] : 0.f;
-	v.z = c + 2 < lim ? p[c + 2] : 0.f;
-	v.w = c + 3 < lim ? p[c + 3] : 0.f;
-	return v;
-}
-
-__global__ void __launch_bounds__(256)
-gram_f64_kernel(const float *__restrict__ X, int64_t ldx, int M, const float *__restrict__ W, int64_t ldw, int N,
-		int64_t n, double *__restrict__ part)
-{
-	__shared__ double red[256 * 16];
-	const int tid = threadIdx.x;
-	const int nbi = (M + 3) / 4, nbj = (N + 3) / 4, nblk = nbi * nbj;    // <= 256
-	const int groups = 256 / nblk;
-	const int blk = tid % nblk, grp = tid / nblk;
-	const int bi = blk / nbj, bj = blk % nbj;
-	const bool active = grp < groups;
-	const bool vx = (ldx % 4) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-	const bool vw = (ldw % 4) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
-	double acc[4][4];
-#pragma unroll
-	for (int a = 0; a < 4; a++)
-#pragma unroll
-		for (int c = 0; c < 4; c++) acc[a][c] = 0;
-	if (active) {
-		const int64_t stride = int64_t(gridDim.x) * groups;
-		int64_t row = int64_t(blockIdx.x) * groups + grp;
-		for (; row + 3 * stride < n; row += 4 * stride) {
-			float4 a[4], c[4];
-#pragma unroll
-			for (int u = 0; u < 4; u++) {
-				a[u] = ld4_guard(X + (row + u * stride) * ldx, 4 * bi, M, vx);
-				c[u] = ld4_guard(W + (row + u * stride) * ldw, 4 * bj, N, vw);
-			}
-#pragma unroll
-			for (int u = 0; u < 4; u++) {
-				const double av[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, cv[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
-#pragma unroll
-				for (int p = 0; p < 4; p++)
-#pragma unroll
-					for (int q = 0; q < 4; q++) acc[p][q] = fma(av[p], cv[q], acc[p][q]);
-			}
-		}
-		for (; row < n; row += stride) {
-			const float4 a = ld4_guard(X + row * ldx, 4 * bi, M, vx);
-			const float4 c = ld4_guard(W + row * ldw, 4 * bj, N, vw);
-			const double av[4] = {a.x, a.y, a.z, a.w}, cv[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-			for (int p = 0; p < 4; p++)
-#pragma unroll
-				for (int q = 0; q < 4; q++) acc[p][q] = fma(av[p], cv[q], acc[p][q]);
-		}
-#pragma unroll
-		for (int p = 0; p < 4; p++)
-#pragma unroll
-			for (int q = 0; q < 4; q++) red[(size_t(grp) * nblk + blk) * 16 + p * 4 + q] = acc[p][q];
-	}
+	red[r][c] = s;
 	__syncthreads();
-	for (int pr = tid; pr < M * N; pr += 256) {
-		const int i = pr / N, j = pr % N;
-		const int b2 = (i / 4) * nbj + j / 4, e = (i % 4) * 4 + j % 4;
-		double sum = 0;
-		for (int g = 0; g < groups; g++) sum += red[(size_t(g) * nblk + b2) * 16 + e];
-		part[size_t(blockIdx.x) * M * N + pr] = sum;
+	for (int w = 32; w > 0; w >>= 1) {
+		if (r < w) red[r][c] += red[r + w][c];
+		__syncthreads();
 	}
+	if (r == 0 && i < MN) G[i] = red[0][c];
 }
 
-// FP64 Gram for M, N <= 16 on the FP64 tensor path (mma.sync m8n8k4 .f64):
-// a warp takes 4 rows per step (the MMA's K).  Lane (g = lane / 4,
-// t = lane % 4) holds x[r][g] and x[r][8 + g] for r = row + t (A fragments
-// of the two 8-row halves of x^T) and the same of w (B fragments), so every
-// input element is loaded and converted once; 4 MMAs update the 2 x 2 tiles
-// of G.  Products of FP32 inputs are exact in FP64.  The 8 warps' tiles are
-// added in warp order (deterministic for a fixed grid).
+// FP64 Gram on the FP64 tensor path (mma.sync m8n8k4 .f64): a warp takes 4
+// rows per MMA (its K) and a block of up to 32 x 32 columns of G.  Lane
+// (g = lane / 4, t = lane % 4) loads VM neighbouring columns of row r + t of X,
+// from column g * VM on, in one load of up to 16 bytes, and VN of W: its m-th
+// value is the A element of the tile of G's rows {g * VM + m}, so the columns
+// are dealt to the tiles with stride VM and no value is loaded or converted
+// twice.  Products of FP32 inputs are exact in FP64.  SYM (W = X): one operand
+// is loaded and only the tiles on and above the diagonal are multiplied.  Wider
+// blocks (M or N > 32) are shared out over the warps of the CTA.
+//
+// What bounds it: bytes in flight, then the DMMA pipe.  With 4-byte loads of 8
+// rows per trip the 16-column Gram at n = 4.2M took 231 us (one operand) and
+// 262 us (two); the DMMA pipe needs about 54 us, HBM 41 and 82 us.  Now 73 and
+// 107 us; 32 columns at n = 2.1M (formerly on CUDA cores) 511 -> 111 and 540 ->
+// 167 us, 64 columns at n = 1.0M 1083 -> 300 us.
 __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b)
 {
 	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
 			: "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(256)
-gram_dmma_kernel(const float *__restrict__ X, int64_t ldx, int M, const float *__restrict__ W, int64_t ldw, int N,
-		int64_t n, double *__restrict__ part)
+// V columns of a row from column c on.  vec: the rows are whole units of V
+// floats, and the load is unconditional (from the last unit where c lies
+// beyond the row: the caller zeroes those lanes), so that a trip's loads
+// leave together.
+template <int V>
+__device__ __forceinline__ void gram_load(const float *row, int c, int lim, bool vec, float (&v)[V])
 {
-	__shared__ double red[8][16 * 16];
+	if (vec) {
+		const float *p = row + min(c, lim - V);
+		if constexpr (V == 4) {
+			const float4 f = __ldcs(reinterpret_cast<const float4 *>(p));
+			v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+		} else if constexpr (V == 2) {
+			const float2 f = __ldcs(reinterpret_cast<const float2 *>(p));
+			v[0] = f.x; v[1] = f.y;
+		} else {
+			v[0] = __ldcs(p);
+		}
+		return;
+	}
+#pragma unroll
+	for (int i = 0; i < V; i++) v[i] = c + i < lim ? row[c + i] : 0.f;
+}
+
+// 4-row steps per trip: two operands of 16 columns at n = 4.2M 107 us with 2,
+// 116 with 4, 126 with 8; of 32 columns at n = 2.1M (127 registers, two CTAs per
+// SM) 167 with 2, 174 with 1, 181 with 4.  One operand: 16 columns 79 us with
+// 4, 77 with 5, 73 with 8 (5 holds a third fewer registers); 32 columns 111
+// with 4, 122 with 2.
+constexpr int gram_steps(int vm, int vn, bool sym)
+{
+	return vm * vn > 4 ? (sym ? 4 : 2) : vm * vn == 1 ? 8 : (sym ? 5 : 2);
+}
+
+template <int VM, int VN, bool SYM>
+__global__ void __launch_bounds__(256, VM * VN == 16 ? 2 : 0)
+gram_dmma_kernel(const float *__restrict__ X, int64_t ldx, int M, const float *__restrict__ W, int64_t ldw, int N,
+		int64_t n, double *__restrict__ part, int nmb, int nnb, bool vx, bool vw)
+{
+	extern __shared__ double gsum[];                 // M x N (a copy per warp up to 16 x 16)
+	constexpr int U = gram_steps(VM, VN, SYM);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int g = lane >> 2, t = lane & 3;
-	double c[2][2][2];
+	const int nblk = nmb * nnb;                      // 1, 2 or 4
+	const int mb = (warp % nblk) / nnb, nb = (warp % nblk) % nnb;
+	const int rg = warp / nblk, RG = 8 / nblk;       // row groups
+	const int cx = mb * 8 * VM + g * VM, cw = nb * 8 * VN + g * VN;
+	double c[VM][VN][2];
 #pragma unroll
-	for (int mi = 0; mi < 2; mi++)
+	for (int m = 0; m < VM; m++)
 #pragma unroll
-		for (int ni = 0; ni < 2; ni++) c[mi][ni][0] = c[mi][ni][1] = 0.0;
-	const int64_t steps = (n + 3) / 4;
-	const int64_t nw = int64_t(gridDim.x) * 8;
-	int64_t q = int64_t(blockIdx.x) * 8 + warp;
-	// two steps per trip: all loads first
-	for (; q + nw < steps; q += 2 * nw) {
-		double a[2][2], bb[2][2];
+		for (int q = 0; q < VN; q++) c[m][q][0] = c[m][q][1] = 0.0;
+	const int64_t stride = int64_t(gridDim.x) * RG * (4 * U);
+	int64_t r0 = (int64_t(blockIdx.x) * RG + rg) * (4 * U) + t;
+	auto load = [&](int64_t row, float (&a)[U][VM], float (&b)[U][VN]) {
 #pragma unroll
-		for (int u = 0; u < 2; u++) {
-			const int64_t r = 4 * (q + u * nw) + t;
-			const bool rv = r < n;
-			a[u][0] = (rv && g < M) ? double(X[r * ldx + g]) : 0.0;
-			a[u][1] = (rv && 8 + g < M) ? double(X[r * ldx + 8 + g]) : 0.0;
-			bb[u][0] = (rv && g < N) ? double(W[r * ldw + g]) : 0.0;
-			bb[u][1] = (rv && 8 + g < N) ? double(W[r * ldw + 8 + g]) : 0.0;
+		for (int u = 0; u < U; u++) {
+			const int64_t r = min(row + 4 * u, n - 1);       // rows beyond n are zeroed below
+			gram_load<VM>(X + r * ldx, cx, M, vx, a[u]);
+			if constexpr (!SYM) gram_load<VN>(W + r * ldw, cw, N, vw, b[u]);
+		}
+	};
+	float a[U][VM], b[U][VN];
+	if (r0 - t < n) load(r0, a, b);
+	for (; r0 - t < n; r0 += stride) {
+		float an[U][VM], bn[U][VN];
+		load(r0 + stride, an, bn);
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			double da[VM], db[VN];
+			// both operands: zero times what the clamped loads left may be NaN
+			const bool live = r0 + 4 * u < n, ax = live && cx < M, aw = live && cw < N;
+#pragma unroll
+			for (int m = 0; m < VM; m++) da[m] = ax ? double(a[u][m]) : 0.0;
+#pragma unroll
+			for (int q = 0; q < VN; q++) db[q] = SYM ? da[q % VM] : (aw ? double(b[u][q]) : 0.0);
+#pragma unroll
+			for (int m = 0; m < VM; m++)
+#pragma unroll
+				for (int q = SYM ? m : 0; q < VN; q++) dmma_8x8x4(c[m][q], da[m], db[q]);
 		}
 #pragma unroll
-		for (int u = 0; u < 2; u++)
+		for (int u = 0; u < U; u++) {
 #pragma unroll
-			for (int mi = 0; mi < 2; mi++)
+			for (int m = 0; m < VM; m++) a[u][m] = an[u][m];
 #pragma unroll
-				for (int ni = 0; ni < 2; ni++) dmma_8x8x4(c[mi][ni], a[u][mi], bb[u][ni]);
+			for (int q = 0; q < VN; q++) b[u][q] = SYM ? 0.f : bn[u][q];
+		}
 	}
-	for (; q < steps; q += nw) {
-		const int64_t r = 4 * q + t;
-		const bool rv = r < n;
-		const double a0 = (rv && g < M) ? double(X[r * ldx + g]) : 0.0;
-		const double a1 = (rv && 8 + g < M) ? double(X[r * ldx + 8 + g]) : 0.0;
-		const double b0 = (rv && g < N) ? double(W[r * ldw + g]) : 0.0;
-		const double b1 = (rv && 8 + g < N) ? double(W[r * ldw + 8 + g]) : 0.0;
-		dmma_8x8x4(c[0][0], a0, b0);
-		dmma_8x8x4(c[0][1], a0, b1);
-		dmma_8x8x4(c[1][0], a1, b0);
-		dmma_8x8x4(c[1][1], a1, b1);
+	// the warps' tiles added in warp order: lane (g, t) holds G's rows
+	// cx + m and columns (2 t + i) VN + q of its block
+	const int MN = M * N;
+	auto tiles = [&](auto put) {
+#pragma unroll
+		for (int m = 0; m < VM; m++)
+#pragma unroll
+			for (int q = SYM ? m : 0; q < VN; q++)
+#pragma unroll
+				for (int i = 0; i < 2; i++) {
+					const int row = cx + m, col = nb * 8 * VN + (2 * t + i) * VN + q;
+					if (row < M && col < N) {
+						put(row * N + col, c[m][q][i]);
+						if (SYM && q > m) put(col * N + row, c[m][q][i]);
+					}
+				}
+	};
+	if constexpr (VM <= 2 && VN <= 2) {
+		// one block of at most 16 x 16: a copy per warp
+		tiles([&](int e, double v) { gsum[warp * MN + e] = v; });
+		__syncthreads();
+		for (int e = tid; e < MN; e += 256) {
+			double s = gsum[e];
+			for (int w = 1; w < 8; w++) s += gsum[w * MN + e];
+			part[size_t(blockIdx.x) * MN + e] = s;
+		}
+	} else {
+		for (int e = tid; e < MN; e += 256) gsum[e] = 0.0;
+		__syncthreads();
+		for (int w = 0; w < 8; w++) {
+			if (warp == w) tiles([&](int e, double v) { gsum[e] += v; });
+			__syncthreads();
+		}
+		for (int e = tid; e < MN; e += 256) part[size_t(blockIdx.x) * MN + e] = gsum[e];
 	}
-	// D fragment: G[8 mi + g][8 ni + 2 t + i]
-#pragma unroll
-	for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-		for (int ni = 0; ni < 2; ni++)
-#pragma unroll
-			for (int i = 0; i < 2; i++) red[warp][(8 * mi + g) * 16 + 8 * ni + 2 * t + i] = c[mi][ni][i];
-	__syncthreads();
-	for (int pr = tid; pr < M * N; pr += 256) {
-		const int i = pr / N, j = pr % N;
-		double sum = red[0][i * 16 + j];
-		for (int w = 1; w < 8; w++) sum += red[w][i * 16 + j];
-		part[size_t(blockIdx.x) * M * N + pr] = sum;
+}
+
+template <int VM, int VN, bool SYM>
+static void launch_gram_dmma(int parts, cudaStream_t st, const float *X, int64_t ldx, int M, const float *W, int64_t ldw,
+		int N, int64_t n, double *part)
+{
+	auto vec = [](const float *p, int64_t ld, int cols, int v) {
+		return cols % v == 0 && ld % v == 0 && (reinterpret_cast<uintptr_t>(p) & (4 * v - 1)) == 0;
+	};
+	const size_t smem = size_t(M) * N * sizeof(double) * (VM <= 2 && VN <= 2 ? 8 : 1);
+	gram_dmma_kernel<VM, VN, SYM><<<parts, 256, smem, st>>>(X, ldx, M, W, ldw, N, n, part,
+			(M + 8 * VM - 1) / (8 * VM), (N + 8 * VN - 1) / (8 * VN), vec(X, ldx, M, VM), vec(W, ldw, N, VN));
+}
+
+// Columns per lane: 1, 2 or 4 for up to 8, 16 or more columns.
+static void gram_dmma(int parts, cudaStream_t st, const float *X, int64_t ldx, int M, const float *W, int64_t ldw, int N,
+		int64_t n, double *part)
+{
+	const int vm = M <= 8 ? 1 : (M <= 16 ? 2 : 4), vn = N <= 8 ? 1 : (N <= 16 ? 2 : 4);
+	if (X == W && ldx == ldw && M == N && M <= 32) {
+		if (vm == 1) launch_gram_dmma<1, 1, true>(parts, st, X, ldx, M, W, ldw, N, n, part);
+		else if (vm == 2) launch_gram_dmma<2, 2, true>(parts, st, X, ldx, M, W, ldw, N, n, part);
+		else launch_gram_dmma<4, 4, true>(parts, st, X, ldx, M, W, ldw, N, n, part);
+		return;
+	}
+	switch (10 * vm + vn) {
+	case 11: return launch_gram_dmma<1, 1, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 12: return launch_gram_dmma<1, 2, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 14: return launch_gram_dmma<1, 4, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 21: return launch_gram_dmma<2, 1, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 22: return launch_gram_dmma<2, 2, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 24: return launch_gram_dmma<2, 4, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 41: return launch_gram_dmma<4, 1, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	case 42: return launch_gram_dmma<4, 2, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
+	default: return launch_gram_dmma<4, 4, false>(parts, st, X, ldx, M, W, ldw, N, n, part);
 	}
 }
 
@@ -1940,12 +1976,9 @@ int fmx_dense_gram(int precision, const float *X, int64_t ldx, int M, const floa
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
 	const int parts = fmx_dense_gram_parts(precision, n);
 	if (precision == FMX_DENSE_F64) {
-		if (M <= 16 && N <= 16)
-			gram_dmma_kernel<<<parts, 256, 0, st>>>(X, ldx, M, W, ldw, N, n, static_cast<double *>(part));
-		else
-			gram_f64_kernel<<<parts, 256, 0, st>>>(X, ldx, M, W, ldw, N, n, static_cast<double *>(part));
+		gram_dmma(parts, st, X, ldx, M, W, ldw, N, n, static_cast<double *>(part));
 		DCUDA_TRY(cudaGetLastError());
-		gram_reduce_kernel<double><<<(M * N + 7) / 8, 256, 0, st>>>(static_cast<const double *>(part), parts, M * N,
+		gram_reduce_kernel<double><<<(M * N + 3) / 4, 256, 0, st>>>(static_cast<const double *>(part), parts, M * N,
 				static_cast<double *>(G));
 		DCUDA_TRY(cudaGetLastError());
 		return FMX_OK;
@@ -1959,7 +1992,7 @@ int fmx_dense_gram(int precision, const float *X, int64_t ldx, int M, const floa
 		DCUDA_TRY(cudaFuncSetAttribute(tc_gram_x3s_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kX3Smem)));
 		tc_gram_x3s_kernel<<<parts / 2, kX3Threads, kX3Smem, st>>>(X, W, n, static_cast<float *>(part), err);
 		DCUDA_TRY(cudaGetLastError());
-		gram_reduce_kernel<float><<<(M * N + 7) / 8, 256, 0, st>>>(static_cast<const float *>(part), parts, M * N,
+		gram_reduce_kernel<float><<<(M * N + 3) / 4, 256, 0, st>>>(static_cast<const float *>(part), parts, M * N,
 				static_cast<float *>(G));
 		DCUDA_TRY(cudaGetLastError());
 		return FMX_OK;
@@ -1979,7 +2012,7 @@ int fmx_dense_gram(int precision, const float *X, int64_t ldx, int M, const floa
 			kern<<<tf32 ? parts / 2 : parts, pipe_threads(P.NG), P.smem, st>>>(X, ldx, M, W, ldw, N, nullptr, 0, nullptr, 0,
 					static_cast<float *>(part), n, err);
 			DCUDA_TRY(cudaGetLastError());
-			gram_reduce_kernel<float><<<(M * N + 7) / 8, 256, 0, st>>>(static_cast<const float *>(part), parts, M * N,
+			gram_reduce_kernel<float><<<(M * N + 3) / 4, 256, 0, st>>>(static_cast<const float *>(part), parts, M * N,
 					static_cast<float *>(G));
 			DCUDA_TRY(cudaGetLastError());
 			return FMX_OK;
@@ -1996,7 +2029,7 @@ int fmx_dense_gram(int precision, const float *X, int64_t ldx, int M, const floa
 		tc_gram_kernel<false><<<parts, 128, smem, st>>>(X, ldx, M, W, ldw, N, n, static_cast<float *>(part), err);
 	}
 	DCUDA_TRY(cudaGetLastError());
-	gram_reduce_kernel<float><<<(M * N + 7) / 8, 256, 0, st>>>(static_cast<const float *>(part), parts, M * N,
+	gram_reduce_kernel<float><<<(M * N + 3) / 4, 256, 0, st>>>(static_cast<const float *>(part), parts, M * N,
 			static_cast<float *>(G));
 	DCUDA_TRY(cudaGetLastError());
 	return FMX_OK;

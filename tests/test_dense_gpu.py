@@ -88,6 +88,31 @@ def _gram_case(torch_cuda, prec, n, M, N, ldx, ldw):
     assert float((G.double() - ref).abs().max()) <= TOL[prec] * scale * (1 if prec != _lib.DENSE_F64 else 10)
 
 
+@pytest.mark.parametrize("n,M,N,ldx,ldw", [(1, 16, 16, 16, 16), (3, 8, 8, 8, 8), (5, 32, 32, 32, 32), (17, 9, 17, 9, 17),
+                                           (33, 24, 24, 24, 24), (4099, 31, 33, 40, 36), (20001, 48, 8, 48, 8),
+                                           (70003, 64, 40, 64, 64), (100001, 15, 2, 16, 3)])
+def test_gram_f64_tiles(torch_cuda, n, M, N, ldx, ldw):
+    """The FP64 tensor-path Gram at the edges of its tiles and trips: row
+    remainders, columns that fill no lane unit, blocks shared over warps; NaN
+    beyond the columns must not leak in.  One operand (the symmetric form)
+    must equal the two-operand form of a copy to FP64 rounding."""
+    torch = torch_cuda
+    _gram_case(torch, _lib.DENSE_F64, n, M, N, ldx, ldw)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    Xf = torch.full((n, ldx + 4), float("nan"), device="cuda")
+    Xf[:, :M] = torch.randn((n, M), generator=g, device="cuda")
+    Xc = Xf.clone()
+    part = torch.empty(_lib.lib.fmx_dense_gram_parts(_lib.DENSE_F64, n) * M * M, dtype=torch.float64, device="cuda")
+    G = [torch.full((M, M), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2)]
+    for W, out in ((Xf, G[0]), (Xc, G[1])):
+        assert _lib.lib.fmx_dense_gram(_lib.DENSE_F64, Xf.data_ptr(), ldx + 4, M, W.data_ptr(), ldx + 4, M, n,
+                                       part.data_ptr(), out.data_ptr(), None, _stream(torch)) == 0
+    ref = Xf[:, :M].double().T @ Xf[:, :M].double()
+    tol = 1e-12 * float(ref.abs().max())
+    assert float((G[0] - ref).abs().max()) <= tol and float((G[1] - ref).abs().max()) <= tol
+    assert torch.equal(G[0], G[0].T)
+
+
 @pytest.mark.parametrize("b", [1, 4, 16, 33, 64])
 def test_chol_inv(torch_cuda, b):
     torch = torch_cuda
