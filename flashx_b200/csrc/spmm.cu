@@ -48,7 +48,8 @@
 // row is written exactly once.  Two row kernels share that scheme:
 //   spmm_lane_kernel  every panel: a lane owns 2 to 32 bytes of each gathered
 //                     row, 8 or 16 gathers in flight per lane
-//   spmv_kernel       k = 1: a warp per range, gathers staged in shared memory
+//   spmv_kernel       k = 1 of small matrices and PageRank: a warp per range,
+//                     gathers staged in shared memory
 // Each call first packs the hot rows: pack_hot_vec_kernel in 16-byte units,
 // pack_hot_kernel one element per thread (k = 1 and rows of odd widths).
 #include "fmx_internal.h"
@@ -486,7 +487,28 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 				}
 			}
 		};
-		if constexpr (SI && sizeof(XT) != 4) {
+		bool done = false;
+		if constexpr (VN == 1) {
+			if (rg.slot != kNoSlot) {
+				// a chunk may be added in any fixed order: the step's terms
+				// by a tree (the error of one long running sum is larger)
+				A t[U];
+#pragma unroll
+				for (int u = 0; u < U; u++) {
+					t[u] = to_acc<A>(x[u].v[0]);
+					if constexpr (SI) { if (cold) t[u] = acc_mul(t[u], sc[u]); }
+					if constexpr (!kBinary) t[u] = acc_mul(t[u], w[u]);
+				}
+#pragma unroll
+				for (int d = 1; d < U; d *= 2)
+#pragma unroll
+					for (int u = 0; u + d < U; u += 2 * d) t[u] = acc_add(t[u], t[u + d]);
+				acc.s[0][0] = acc_add(acc.s[0][0], t[0]);
+				done = true;
+			}
+		}
+		if (done) {
+		} else if constexpr (SI && sizeof(XT) != 4) {
 			sums(std::true_type{});
 		} else if constexpr (SI) {
 			if (cold) sums(std::true_type{});
@@ -549,9 +571,8 @@ spmm_lane_kernel(const spmm_args a)
 // order, with one running sum per row and every add rounded, which is the
 // lane-group kernel's arithmetic: rows of up to 256 entries come out
 // identical.  A chunk of a longer row is added up by the whole warp (each
-// lane its own entries, then a fixed xor tree) into its partial slot.  (The lane-group
-// kernel at k = 1 gives each lane a whole range and waits on one step of 4
-// gathers at a time.)
+// lane its own entries, then a fixed xor tree) into its partial slot.
+// (spmv_by_warps says which matrices come here.)
 constexpr int kSpmvMax = 512;            // most entries of one range
 static_assert(((kRange - 1 + kExactMax + kStep - 1) / kStep) * kStep <= uint32_t(kSpmvMax) &&
 		kChunk <= uint32_t(kSpmvMax), "a range fits the SpMV kernel's staging");
@@ -1309,6 +1330,24 @@ static int lane_width(const void *X, int64_t ldx, const void *Y, int64_t ldy, in
 	return vn;
 }
 
+// k = 1: the warp-per-range kernel while its grid (64 warps per SM) takes the
+// ranges in one round, where its short chain wins (R-MAT scale 16: 18.9
+// against 20.6 us); beyond that a lane per range in the row kernel, which
+// issues a third of the instructions per entry (scale 18 / 20 / 22 / 24: 38 /
+// 111 / 325 / 1400 against 29 / 66 / 251 / 1150 us).  Decided on the whole
+// part, so that a streamed matrix takes the resident one's kernels.
+static bool spmv_by_warps(const gpu_part &p)
+{
+	static std::atomic<unsigned> sms[64];
+	unsigned n = sms[p.device & 63].load(std::memory_order_relaxed);
+	if (!n) {
+		int v = 0;
+		cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, p.device);
+		sms[p.device & 63].store(n = unsigned(std::max(v, 1)), std::memory_order_relaxed);
+	}
+	return p.n_ranges <= n * 64;
+}
+
 // Run one orientation over all column panels (kPanelBytes of X row each).
 // k = 1 without row scales: pack, the warp-per-range SpMV, fixup.
 // `xhot` and `partial` default to the part's own scratch.
@@ -1349,7 +1388,7 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 	if (!xhot) xhot = p.xhot;
 	if (!partial) partial = p.partial;
 	if constexpr (std::is_same<XT, A>::value && std::is_same<YT, A>::value && std::is_floating_point<A>::value) {
-		if (k == 1 && !sin && !sout)
+		if (k == 1 && !sin && !sout && spmv_by_warps(p))
 			return run_spmv<A, WT, false>(p, static_cast<const A *>(X), ldx, static_cast<A *>(Y), ldy, st, pr_epi{}, xhot,
 					partial);
 	}
