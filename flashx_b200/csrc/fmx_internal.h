@@ -126,24 +126,35 @@ int matrix_from_csr(const host_csr &a, const host_csr *at, int device, fmx_matri
 // ---- fused PageRank iteration ----------------------------------------------
 // The update of fm::alg::PageRank (PageRank.cpp:110-123) applied where the
 // SpMV on A^T closes a row: p2 = out * d + teleport; converged += |pr1 - p2|
-// < eps; pr = p2; in_next = p2 / deg; pr1 = in_next * deg.  state[0] counts
-// this iteration's converged vertices, state[1] is the done flag (set once
-// every vertex converged or the iteration cap is reached; the kernels of
-// later iterations then return at once), state[2] the iterations run.
+// < eps; pr = p2; in_next = p2 / deg; pr1 = in_next * deg.  A hot column's next
+// input also goes to its slot of the next hot pack (slot[row], 0: none).
+// state[0] counts this iteration's converged vertices, state[1] is the done
+// flag (set once every vertex converged or the iteration cap is reached; the
+// kernels of later iterations then return at once), state[2] the iterations
+// run, state[3] the blocks of the iteration's last kernel that are through:
+// the last of them applies the loop test (when `finish` is set).
 struct pr_epi {
 	const float *deg;
 	const uint32_t *heavy_mask;    // bit per row summed by the fixup (chunked rows)
-	float *pr, *pr1, *in_next;
+	const uint32_t *slot;
+	float *pr, *pr1, *in_next, *xhot_next;
 	unsigned long long *state;
 	float damping, teleport, eps;
+	int finish;
 	unsigned long long n, max_iters;
 };
-// One iteration on the transpose part of `mt`: SpMV of `in` with the update
-// fused, then the iteration's convergence test on the device.
-int pagerank_iteration(const fmx_matrix *mt, const float *in, const pr_epi &e, cudaStream_t st);
-// Set heavy_mask (ceil(nrows / 32) words, zeroed by the caller) from mt's
-// chunked rows.
-int pagerank_heavy_mask(const fmx_matrix *mt, uint32_t *mask, cudaStream_t st);
+// One iteration on the transpose part of `mt`: the SpMV of `in` (its hot
+// pack in xhot) with the update fused, or, where k = 1 takes the row kernel,
+// into `out` (nrows floats) with the update in a pass of its own; then the
+// iteration's convergence test on the device.
+int pagerank_iteration(const fmx_matrix *mt, const float *in, float *xhot, float *out, const pr_epi &e, cudaStream_t st);
+// Whether pagerank_iteration needs `out`.
+bool pagerank_needs_out(const fmx_matrix *mt);
+// Hot columns of mt's part (a pack holds one value more: slot 0 is zero).
+uint64_t pagerank_hot(const fmx_matrix *mt);
+// Set heavy_mask (ceil(nrows / 32) words) from mt's chunked rows and slot
+// (nrows words) from its hot columns; both zeroed by the caller.
+int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, cudaStream_t st);
 
 } // namespace fmx
 

@@ -12,15 +12,18 @@
 //     converged = #{ |pr1 - pr2| < 0.001 / n }        (:94, :118-123)
 //     pr  = pr2
 //
-// One iteration is one pass: the SpMV on the transpose (k = 1) applies the
-// damping, counts the converged vertices and writes the next input where it
-// closes each row (rows summed in chunks get the same update in the fixup
-// kernel), and a one-thread kernel runs the loop test on the device.  The
-// input is double-buffered (other rows still gather this iteration's input
-// while the next one is written).  Iterations are queued in batches with one
-// host read of the loop state per batch; an iteration queued after the loop
-// ended returns at once, so the result and the count match a loop that
-// tests on the host after every iteration.
+// One iteration of a small matrix is one pass: the SpMV on the transpose
+// (k = 1) applies the damping, counts the converged vertices and writes the
+// next input, and its hot pack, where it closes each row (rows summed in chunks
+// get the same update in the fixup kernel); the last block of the last kernel
+// applies the loop test.  Larger ones run the row kernel and the update as a
+// pass over the rows.  Input and pack are double-buffered (other rows still
+// gather this iteration's while the next ones are written).  What bounds a
+// small iteration is its kernels' latency: with a pack and a loop-test kernel
+// of their own R-MAT scale 16 took 26 us per iteration.  Iterations are
+// queued in batches, one batch ahead of the host's read of the loop state; an
+// iteration queued after the loop ended returns at once, so the result and
+// the count match a loop that tests on the host after every iteration.
 #include "fmx_internal.h"
 
 #include <cuda_runtime.h>
@@ -52,9 +55,10 @@ __global__ void fill_kernel(float *p, int64_t n, float v)
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) p[i] = v;
 }
 
-// deg = max(deg, 1); pr = p0; in = pr / deg; pr1 = in * deg
+// deg = max(deg, 1); pr = p0; in = pr / deg (and its slot of the hot pack);
+// pr1 = in * deg
 __global__ void init_kernel(float *__restrict__ deg, float *__restrict__ pr, float *__restrict__ in,
-		float *__restrict__ pr1, int64_t n, float p0)
+		float *__restrict__ pr1, const uint32_t *__restrict__ slot, float *__restrict__ xhot, int64_t n, float p0)
 {
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
 		const float d = fmaxf(deg[i], 1.0f);
@@ -62,6 +66,7 @@ __global__ void init_kernel(float *__restrict__ deg, float *__restrict__ pr, flo
 		pr[i] = p0;
 		const float x = __fdiv_rn(p0, d);
 		in[i] = x;
+		if (slot[i]) xhot[slot[i]] = x;
 		pr1[i] = __fmul_rn(x, d);
 	}
 }
@@ -106,8 +111,8 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	} g{mt, static_cast<cudaStream_t>(stream), {}};
 	cudaStream_t st = g.st;
 	const int64_t n = int64_t(nr);
-	float *deg, *in0, *in1, *pr1;
-	uint32_t *mask;
+	float *deg, *in0, *in1, *pr1, *xh0, *xh1, *out = nullptr;
+	uint32_t *mask, *slot;
 	unsigned long long *state;
 	auto alloc = [&](void **q, size_t bytes) -> int {
 		cudaError_t e = work_alloc(q, std::max<size_t>(bytes, 16), st);
@@ -117,11 +122,20 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	};
 	const size_t mask_words = size_t((n + 31) / 32);
 	for (float **b : {&deg, &in0, &in1, &pr1}) P_TRY(alloc(reinterpret_cast<void **>(b), size_t(n) * sizeof(float)));
-	P_TRY(alloc(reinterpret_cast<void **>(&mask), mask_words * sizeof(uint32_t)));
-	P_TRY(alloc(reinterpret_cast<void **>(&state), 3 * sizeof(unsigned long long)));
-	// the loop state comes back through three pinned words per host thread
+	// one block of zeroed words: the loop state, the two hot packs (their slot
+	// 0 stays zero), the mask and the slots
+	const size_t pack = size_t(pagerank_hot(mt)) + 1;
+	const size_t zbytes = 8 * sizeof(unsigned long long) + (2 * pack + mask_words + size_t(n)) * sizeof(uint32_t);
+	P_TRY(alloc(reinterpret_cast<void **>(&state), zbytes));
+	xh0 = reinterpret_cast<float *>(state + 8);
+	xh1 = xh0 + pack;
+	mask = reinterpret_cast<uint32_t *>(xh1 + pack);
+	slot = mask + mask_words;
+	if (pagerank_needs_out(mt)) P_TRY(alloc(reinterpret_cast<void **>(&out), size_t(n) * sizeof(float)));
+	// the loop state comes back through pinned words per host thread, one set
+	// per batch in flight
 	static thread_local unsigned long long *hstate = nullptr;
-	if (!hstate) PCUDA_TRY(cudaMallocHost(&hstate, 3 * sizeof(unsigned long long)));
+	if (!hstate) PCUDA_TRY(cudaMallocHost(&hstate, 2 * 4 * sizeof(unsigned long long)));
 	const unsigned gb = grid_for(n);
 	fill_kernel<<<gb, kThreads, 0, st>>>(in1, n, 1.0f);
 	PCUDA_TRY(cudaGetLastError());
@@ -130,6 +144,7 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	pr_epi e{};
 	e.deg = deg;
 	e.heavy_mask = mask;
+	e.slot = slot;
 	e.pr = pr;
 	e.pr1 = pr1;
 	e.state = state;
@@ -138,24 +153,37 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	e.eps = float(0.001 / double(n));
 	e.n = uint64_t(n);
 	e.max_iters = max_iters;
-	init_kernel<<<gb, kThreads, 0, st>>>(deg, pr, in0, pr1, n, p0);
+	PCUDA_TRY(cudaMemsetAsync(state, 0, zbytes, st));
+	P_TRY(pagerank_maps(mt, mask, slot, st));
+	init_kernel<<<gb, kThreads, 0, st>>>(deg, pr, in0, pr1, slot, xh0, n, p0);
 	PCUDA_TRY(cudaGetLastError());
-	PCUDA_TRY(cudaMemsetAsync(mask, 0, mask_words * sizeof(uint32_t), st));
-	PCUDA_TRY(cudaMemsetAsync(state, 0, 3 * sizeof(unsigned long long), st));
-	P_TRY(pagerank_heavy_mask(mt, mask, st));
-	uint64_t it = 0, queued = 0;
-	while (n > 0 && queued < max_iters) {
-		const uint64_t batch = std::min<uint64_t>(kBatch, max_iters - queued);
-		for (uint64_t b = 0; b < batch; b++, queued++) {
-			const float *in = (queued & 1) ? in1 : in0;
-			e.in_next = (queued & 1) ? in0 : in1;
-			P_TRY(pagerank_iteration(mt, in, e, st));
+	struct events {
+		cudaEvent_t e[2] = {nullptr, nullptr};
+		~events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+	} ev;
+	for (cudaEvent_t &x : ev.e) PCUDA_TRY(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+	uint64_t it = 0, queued = 0, batches = 0, read = 0;
+	bool done = n == 0 || max_iters == 0;
+	while (!done) {
+		// queue a batch, then read the state of the one before
+		if (queued < max_iters) {
+			const uint64_t batch = std::min<uint64_t>(kBatch, max_iters - queued);
+			for (uint64_t b = 0; b < batch; b++, queued++) {
+				const bool odd = queued & 1;
+				e.in_next = odd ? in0 : in1;
+				e.xhot_next = odd ? xh0 : xh1;
+				P_TRY(pagerank_iteration(mt, odd ? in1 : in0, odd ? xh1 : xh0, out, e, st));
+			}
+			PCUDA_TRY(cudaMemcpyAsync(hstate + 4 * (batches & 1), state, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+			PCUDA_TRY(cudaEventRecord(ev.e[batches & 1], st));
+			batches++;
+			if (batches - read < 2 && queued < max_iters) continue;
 		}
-		PCUDA_TRY(cudaMemcpyAsync(hstate, state, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-		PCUDA_TRY(cudaStreamSynchronize(st));
-		it = hstate[2];
-		if (hstate[1]) break;
+		PCUDA_TRY(cudaEventSynchronize(ev.e[read & 1]));
+		it = hstate[4 * (read & 1) + 2];
+		done = hstate[4 * (read & 1) + 1] || (++read == batches && queued >= max_iters);
 	}
+	PCUDA_TRY(cudaStreamSynchronize(st));
 	if (iters) *iters = it;
 	return FMX_OK;
 }

@@ -312,7 +312,23 @@ __device__ __forceinline__ void pr_update(const pr_epi &e, int64_t row, float ou
 	const float d = e.deg[row];
 	const float x = __fdiv_rn(p2, d);
 	e.in_next[row] = x;
+	const uint32_t s = __ldg(e.slot + row);
+	if (s) e.xhot_next[s] = x;
 	e.pr1[row] = __fmul_rn(x, d);
+}
+
+// The loop test (PageRank.cpp:96,124-129) by the last block of an iteration's
+// last kernel, every thread of which comes here.
+__device__ __forceinline__ void pr_finish(const pr_epi &e)
+{
+	__syncthreads();
+	if (threadIdx.x != 0) return;
+	__threadfence();
+	if (atomicAdd(e.state + 3, 1ull) != gridDim.x - 1) return;
+	__threadfence();
+	e.state[3] = 0;
+	const unsigned long long it = ++e.state[2], converged = atomicExch(e.state, 0ull);
+	if (converged >= e.n || it >= e.max_iters) e.state[1] = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -690,7 +706,22 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 	if constexpr (EPI) {
 		cnt = __reduce_add_sync(0xffffffffu, cnt);
 		if (lane == 0 && cnt) atomicAdd(e.state, (unsigned long long)cnt);
+		if (e.finish) pr_finish(e);
 	}
+}
+
+// The update of one PageRank iteration over `out` = A^T in.
+__global__ void __launch_bounds__(kThreads) pr_apply_kernel(const float *__restrict__ out, int64_t n, const pr_epi e)
+{
+	dep_wait();
+	dep_launch();
+	if (e.state[1]) return;
+	unsigned cnt = 0;
+	for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads)
+		pr_update(e, i, out[i], cnt);
+	cnt = __reduce_add_sync(0xffffffffu, cnt);
+	if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(e.state, (unsigned long long)cnt);
+	pr_finish(e);
 }
 
 // Pack the hot columns' X rows of this panel behind a zero row:
@@ -916,6 +947,9 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const heavy_row *heavy,
 		} else if (mine && part == 0) {
 			fix_store<YT, A, SCALE_OUT, EPI>(h, t, nv, Y, ldy, vec ? 4 * u : u, s_out, e);
 		}
+	}
+	if constexpr (EPI) {
+		if (e.finish) pr_finish(e);
 	}
 }
 
@@ -1355,7 +1389,7 @@ static bool spmv_by_warps(const gpu_part &p)
 // `xhot` and `partial` default to the part's own scratch.
 template <class T, class WT, bool EPI>
 static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ldy, cudaStream_t st,
-		const pr_epi &e = pr_epi{}, void *xhot = nullptr, void *partial = nullptr)
+		const pr_epi &e = pr_epi{}, void *xhot = nullptr, void *partial = nullptr, bool packed = false)
 {
 	if (!xhot) xhot = p.xhot;
 	if (!partial) partial = p.partial;
@@ -1367,16 +1401,21 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 	a.ldx = ldx; a.ldy = ldy; a.k = 1;
 	a.G = 1; a.R = 32;
 	a.n_ranges = p.n_ranges;
-	const unsigned pb = unsigned(std::min<uint64_t>((uint64_t(p.n_hot) + 256) / 256, 148ull * 16));
-	pack_hot_kernel<T, T, false><<<pb, 256, 0, st>>>(p.hot_col, p.n_hot, X, ldx, 1, static_cast<T *>(xhot), 1,
-			nullptr);
-	CUDA_TRY(cudaGetLastError());
+	if (!packed) {
+		const unsigned pb = unsigned(std::min<uint64_t>((uint64_t(p.n_hot) + 256) / 256, 148ull * 16));
+		pack_hot_kernel<T, T, false><<<pb, 256, 0, st>>>(p.hot_col, p.n_hot, X, ldx, 1, static_cast<T *>(xhot), 1,
+				nullptr);
+		CUDA_TRY(cudaGetLastError());
+	}
+	// the loop test belongs to the iteration's last kernel
+	pr_epi es = e;
+	es.finish = e.finish && !p.n_heavy;
 	auto kern = spmv_kernel<T, WT, EPI>;
 	static std::atomic<unsigned> blocks[64];
 	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kThreads);
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
-			if (p.streamed) kern<<<b, kThreads, 0, st>>>(sa, e);
-			else CUDA_TRY(launch_dep(kern, b, kThreads, st, sa, e));
+			if (p.streamed) kern<<<b, kThreads, 0, st>>>(sa, es);
+			else CUDA_TRY(launch_dep(kern, b, kThreads, st, sa, es));
 			CUDA_TRY(cudaGetLastError());
 			return FMX_OK;
 		}))
@@ -1488,7 +1527,7 @@ int spmm_part(const gpu_part &p, int xt, const void *X, int64_t ldx, int yt, voi
 // Fused PageRank iteration (SpMV on A^T with the update at each row close)
 // ---------------------------------------------------------------------------
 
-// The iteration's convergence test (PageRank.cpp:96,124-129): one thread.
+// The same loop test as a kernel, for streamed parts (several SpMV launches).
 __global__ void pr_finish_kernel(unsigned long long *state, unsigned long long n, unsigned long long max_iters)
 {
 	if (threadIdx.x == 0 && !state[1]) {
@@ -1496,6 +1535,11 @@ __global__ void pr_finish_kernel(unsigned long long *state, unsigned long long n
 		if (state[0] >= n || it >= max_iters) state[1] = 1;
 		state[0] = 0;
 	}
+}
+
+__global__ void hot_slot_kernel(const int32_t *hot_col, uint32_t n_hot, uint32_t *slot)
+{
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_hot; i += gridDim.x * blockDim.x) slot[hot_col[i]] = i + 1;
 }
 
 __global__ void heavy_mask_kernel(const heavy_row *heavy, uint32_t n_heavy, uint32_t *mask)
@@ -1506,31 +1550,56 @@ __global__ void heavy_mask_kernel(const heavy_row *heavy, uint32_t n_heavy, uint
 	}
 }
 
-int pagerank_heavy_mask(const fmx_matrix *mt, uint32_t *mask, cudaStream_t st)
+int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, cudaStream_t st)
 {
 	const gpu_part &p = *mt->a;
-	if (!p.n_heavy) return FMX_OK;
-	heavy_mask_kernel<<<unsigned(std::min<uint32_t>((p.n_heavy + 255) / 256, 1024)), 256, 0, st>>>(p.heavy,
-			p.n_heavy, mask);
+	auto grid = [](uint32_t n) { return unsigned(std::min<uint32_t>((n + 255) / 256, 1024)); };
+	if (p.n_heavy) heavy_mask_kernel<<<grid(p.n_heavy), 256, 0, st>>>(p.heavy, p.n_heavy, mask);
+	CUDA_TRY(cudaGetLastError());
+	if (p.n_hot) hot_slot_kernel<<<grid(p.n_hot), 256, 0, st>>>(p.hot_col, p.n_hot, slot);
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
 }
+
+uint64_t pagerank_hot(const fmx_matrix *mt) { return mt->a->n_hot; }
+bool pagerank_needs_out(const fmx_matrix *mt) { return !spmv_by_warps(*mt->a); }
 
 template <class WT>
-static int pr_iteration_typed(const gpu_part &p, const float *in, const pr_epi &e, cudaStream_t st)
+static int pr_iteration_typed(const gpu_part &p, const float *in, float *xhot, float *out, pr_epi e, cudaStream_t st)
 {
-	// the update writes pr, pr1 and the next input instead of Y
-	if (int rc = run_spmv<float, WT, true>(p, in, 1, nullptr, 1, st, e)) return rc;
-	pr_finish_kernel<<<1, 32, 0, st>>>(e.state, e.n, e.max_iters);
-	CUDA_TRY(cudaGetLastError());
+	if (spmv_by_warps(p)) {
+		// the update writes pr, pr1, the next input and its hot pack instead of Y
+		e.finish = !p.streamed;
+		if (int rc = run_spmv<float, WT, true>(p, in, 1, nullptr, 1, st, e, xhot, nullptr, true)) return rc;
+		if (p.streamed) {
+			pr_finish_kernel<<<1, 32, 0, st>>>(e.state, e.n, e.max_iters);
+			CUDA_TRY(cudaGetLastError());
+		}
+		return FMX_OK;
+	}
+	// the row kernel of fmx_spmm at k = 1, then the update over all rows: a row
+	// close there would wait on its own loads of deg and pr1
+	spmm_args a{};
+	a.col = p.col; a.val = p.val; a.ranges = p.ranges;
+	a.X = in; a.xhot = xhot; a.hot_ld = 1;
+	a.Y = out; a.partial = p.partial;
+	a.ldx = a.ldy = 1; a.k = 1; a.G = 1; a.R = 32;
+	a.n_ranges = p.n_ranges;
+	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
+			return launch_lanes<float, float, float, WT, 1, false, false>(p, sa, st);
+		}))
+		return rc;
+	if (int rc = launch_fixup<float, float, false>(p, static_cast<const float *>(p.partial), out, 1, 1, nullptr, st)) return rc;
+	const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((p.nrows + kThreads - 1) / kThreads, 148ull * 8)));
+	CUDA_TRY(launch_dep(pr_apply_kernel, g, kThreads, st, out, int64_t(p.nrows), e));
 	return FMX_OK;
 }
 
-int pagerank_iteration(const fmx_matrix *mt, const float *in, const pr_epi &e, cudaStream_t st)
+int pagerank_iteration(const fmx_matrix *mt, const float *in, float *xhot, float *out, const pr_epi &e, cudaStream_t st)
 {
 	const gpu_part &p = *mt->a;
-	if (p.prim == FMX_P_BOOL) return pr_iteration_typed<void>(p, in, e, st);
-	if (p.prim == FMX_P_FLOAT) return pr_iteration_typed<float>(p, in, e, st);
+	if (p.prim == FMX_P_BOOL) return pr_iteration_typed<void>(p, in, xhot, out, e, st);
+	if (p.prim == FMX_P_FLOAT) return pr_iteration_typed<float>(p, in, xhot, out, e, st);
 	return set_error(FMX_ERR_TYPE, "PageRank: binary or float-weighted matrices");
 }
 
