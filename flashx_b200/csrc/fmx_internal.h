@@ -132,11 +132,15 @@ int matrix_from_csr(const host_csr &a, const host_csr *at, int device, fmx_matri
 // flag (set once every vertex converged or the iteration cap is reached; the
 // kernels of later iterations then return at once), state[2] the iterations
 // run, state[3] the blocks of the iteration's last kernel that are through:
-// the last of them applies the loop test (when `finish` is set).
+// the last of them applies the loop test (when `finish` is set).  A chunked row
+// is updated by the warp whose chunk arrives last.
 struct pr_epi {
 	const float *deg;
 	const uint32_t *heavy_mask;    // bit per row summed by the fixup (chunked rows)
 	const uint32_t *slot;
+	const void *heavy;             // the part's chunked rows (heavy_row[])
+	const uint32_t *chunk_heavy;   // a chunk's row in that list
+	uint32_t *arrived;             // chunks of each such row summed in this iteration
 	float *pr, *pr1, *in_next, *xhot_next;
 	unsigned long long *state;
 	float damping, teleport, eps;
@@ -150,11 +154,14 @@ struct pr_epi {
 int pagerank_iteration(const fmx_matrix *mt, const float *in, float *xhot, float *out, const pr_epi &e, cudaStream_t st);
 // Whether pagerank_iteration needs `out`.
 bool pagerank_needs_out(const fmx_matrix *mt);
-// Hot columns of mt's part (a pack holds one value more: slot 0 is zero).
-uint64_t pagerank_hot(const fmx_matrix *mt);
-// Set heavy_mask (ceil(nrows / 32) words) from mt's chunked rows and slot
-// (nrows words) from its hot columns; both zeroed by the caller.
-int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, cudaStream_t st);
+// Hot columns of mt's part (a pack holds one value more: slot 0 is zero), its
+// chunked rows and their chunks.
+void pagerank_sizes(const fmx_matrix *mt, uint64_t *hot, uint64_t *heavy, uint64_t *chunks);
+// Set heavy_mask (ceil(nrows / 32) words) and chunk_heavy from mt's chunked
+// rows, whose list is *heavy, and slot (nrows words) from its hot columns;
+// mask and slot zeroed by the caller.
+int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, uint32_t *chunk_heavy, const void **heavy,
+		cudaStream_t st);
 
 } // namespace fmx
 

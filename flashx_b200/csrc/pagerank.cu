@@ -15,12 +15,11 @@
 // One iteration of a small matrix is one pass: the SpMV on the transpose
 // (k = 1) applies the damping, counts the converged vertices and writes the
 // next input, and its hot pack, where it closes each row (rows summed in chunks
-// get the same update in the fixup kernel); the last block of the last kernel
-// applies the loop test.  Larger ones run the row kernel and the update as a
+// by the warp whose chunk arrives last); the last block applies the loop test.  Larger ones run the row kernel and the update as a
 // pass over the rows.  Input and pack are double-buffered (other rows still
 // gather this iteration's while the next ones are written).  What bounds a
-// small iteration is its kernels' latency: with a pack and a loop-test kernel
-// of their own R-MAT scale 16 took 26 us per iteration.  Iterations are
+// small iteration is its kernels' latency: as four launches (pack, SpMV,
+// fixup, loop test) R-MAT scale 16 took 27 us per iteration.  Iterations are
 // queued in batches, one batch ahead of the host's read of the loop state; an
 // iteration queued after the loop ended returns at once, so the result and
 // the count match a loop that tests on the host after every iteration.
@@ -112,7 +111,7 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	cudaStream_t st = g.st;
 	const int64_t n = int64_t(nr);
 	float *deg, *in0, *in1, *pr1, *xh0, *xh1, *out = nullptr;
-	uint32_t *mask, *slot;
+	uint32_t *mask, *slot, *arrived, *chunk_heavy;
 	unsigned long long *state;
 	auto alloc = [&](void **q, size_t bytes) -> int {
 		cudaError_t e = work_alloc(q, std::max<size_t>(bytes, 16), st);
@@ -123,14 +122,18 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	const size_t mask_words = size_t((n + 31) / 32);
 	for (float **b : {&deg, &in0, &in1, &pr1}) P_TRY(alloc(reinterpret_cast<void **>(b), size_t(n) * sizeof(float)));
 	// one block of zeroed words: the loop state, the two hot packs (their slot
-	// 0 stays zero), the mask and the slots
-	const size_t pack = size_t(pagerank_hot(mt)) + 1;
-	const size_t zbytes = 8 * sizeof(unsigned long long) + (2 * pack + mask_words + size_t(n)) * sizeof(uint32_t);
+	// 0 stays zero), the mask, the slots and the arrival counts
+	uint64_t n_hot = 0, n_heavy = 0, n_chunks = 0;
+	pagerank_sizes(mt, &n_hot, &n_heavy, &n_chunks);
+	const size_t pack = size_t(n_hot) + 1;
+	const size_t zbytes = 8 * sizeof(unsigned long long) + (2 * pack + mask_words + size_t(n) + n_heavy) * sizeof(uint32_t);
 	P_TRY(alloc(reinterpret_cast<void **>(&state), zbytes));
+	P_TRY(alloc(reinterpret_cast<void **>(&chunk_heavy), n_chunks * sizeof(uint32_t)));
 	xh0 = reinterpret_cast<float *>(state + 8);
 	xh1 = xh0 + pack;
 	mask = reinterpret_cast<uint32_t *>(xh1 + pack);
 	slot = mask + mask_words;
+	arrived = slot + n;
 	if (pagerank_needs_out(mt)) P_TRY(alloc(reinterpret_cast<void **>(&out), size_t(n) * sizeof(float)));
 	// the loop state comes back through pinned words per host thread, one set
 	// per batch in flight
@@ -145,6 +148,8 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	e.deg = deg;
 	e.heavy_mask = mask;
 	e.slot = slot;
+	e.chunk_heavy = chunk_heavy;
+	e.arrived = arrived;
 	e.pr = pr;
 	e.pr1 = pr1;
 	e.state = state;
@@ -154,7 +159,7 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	e.n = uint64_t(n);
 	e.max_iters = max_iters;
 	PCUDA_TRY(cudaMemsetAsync(state, 0, zbytes, st));
-	P_TRY(pagerank_maps(mt, mask, slot, st));
+	P_TRY(pagerank_maps(mt, mask, slot, chunk_heavy, &e.heavy, st));
 	init_kernel<<<gb, kThreads, 0, st>>>(deg, pr, in0, pr1, slot, xh0, n, p0);
 	PCUDA_TRY(cudaGetLastError());
 	struct events {

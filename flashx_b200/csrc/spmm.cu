@@ -620,14 +620,57 @@ constexpr int kSpmvMax = 512;            // most entries of one range
 static_assert(((kRange - 1 + kExactMax + kStep - 1) / kStep) * kStep <= uint32_t(kSpmvMax) &&
 		kChunk <= uint32_t(kSpmvMax), "a range fits the SpMV kernel's staging");
 
+// A chunk of a PageRank row: the warp whose chunk arrives last adds the row's
+// partials, in spmm_fixup_kernel's order at k = 1 (the same parts, the same
+// tree), and updates the row, which saves the iteration a kernel.  Partials
+// are read past the L1.
+__device__ __forceinline__ void pr_chunk(const pr_epi &e, float *partial, uint32_t slot, float acc, int lane, unsigned &cnt)
+{
+	uint32_t h = 0, old = 0;
+	if (lane == 0) {
+		__stcg(partial + int64_t(slot) * kPartialStride, acc);
+		__threadfence();
+		h = e.chunk_heavy[slot];
+		old = atomicAdd(e.arrived + h, 1u);
+	}
+	h = __shfl_sync(0xffffffffu, h, 0);
+	old = __shfl_sync(0xffffffffu, old, 0);
+	const heavy_row hr = static_cast<const heavy_row *>(e.heavy)[h];
+	if (old != hr.count - 1) return;
+	__threadfence();
+	const float *pc = partial + int64_t(hr.first) * kPartialStride;
+	auto sums = [&](uint32_t part, uint32_t P) {
+		float s0 = 0.f, s1 = 0.f;
+		uint32_t c = part;
+		for (; c + P < hr.count; c += 2u * P) {
+			s0 = acc_add(s0, __ldcg(pc + int64_t(c) * kPartialStride));
+			s1 = acc_add(s1, __ldcg(pc + int64_t(c + P) * kPartialStride));
+		}
+		if (c < hr.count) s0 = acc_add(s0, __ldcg(pc + int64_t(c) * kPartialStride));
+		return acc_add(s0, s1);
+	};
+	auto tree = [&](float v, int lanes) {
+		for (int o = 1; o < lanes; o <<= 1) v = acc_add(v, __shfl_xor_sync(0xffffffffu, v, o));
+		return v;
+	};
+	float v;
+	if (hr.count > kBlockChunks) {
+		v = tree(sums(uint32_t(lane), 256), 32);
+		for (uint32_t w = 1; w < 8; w++) v = acc_add(v, tree(sums(w * 32 + uint32_t(lane), 256), 32));
+	} else if (hr.count > kLongChunks) {
+		v = tree(sums(uint32_t(lane), 32), 32);
+	} else {
+		v = tree(sums(uint32_t(lane & 1), 2), 2);
+	}
+	if (lane == 0) {
+		e.arrived[h] = 0;
+		pr_update(e, hr.row, v, cnt);
+	}
+}
+
 template <class T, class WT, bool EPI>
 __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const pr_epi e)
 {
-	dep_wait();
-	dep_launch();
-	if constexpr (EPI) {
-		if (e.state[1]) return;           // converged in an earlier iteration
-	}
 	constexpr int kWarps = kThreads / 32;
 	constexpr int J = kSpmvMax / 32;
 	constexpr bool kBinary = std::is_void<WT>::value;
@@ -640,6 +683,16 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 	const T *H = static_cast<const T *>(a.xhot);
 	const uint64_t pol_hot = policy_evict_last(), pol_cold = policy_evict_first();
 	unsigned cnt = 0;
+	// the matrix does not change: the first range's ids load while the kernel
+	// before this one still runs
+	bool waited = false, done = false;
+	auto wait = [&]() {
+		if (waited) return;
+		dep_wait();
+		dep_launch();
+		waited = true;
+		if constexpr (EPI) done = e.state[1] != 0;    // converged in an earlier iteration
+	};
 	for (uint32_t r = gw; r < a.n_ranges; r += nw) {
 		const range_t rg = a.ranges[r];
 		const bool runs = rg.slot == kNoSlot;
@@ -649,6 +702,7 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			const uint32_t i = uint32_t(j * 32 + lane);
 			raw[j] = i < rg.len ? __ldcs(a.col + rg.e0 + i) : 0u;
 		}
+		wait();
 		T t[J];
 #pragma unroll
 		for (int j = 0; j < J; j++) {
@@ -680,6 +734,9 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			sval[wib][i] = t[j];
 		}
 		__syncwarp();
+		if constexpr (EPI) {
+			if (done) break;
+		}
 		if (runs) {
 			for (int q = lane; q < nrow; q += 32) {
 				const int b0 = q ? int(send[wib][q - 1]) + 1 : 0, b1 = send[wib][q];
@@ -699,11 +756,14 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			for (int j = 0; j < J; j++) acc = acc_add(acc, t[j]);
 #pragma unroll
 			for (int o = 16; o > 0; o >>= 1) acc = acc_add(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-			if (lane == 0) static_cast<T *>(a.partial)[int64_t(rg.slot) * kPartialStride] = acc;
+			if constexpr (EPI) pr_chunk(e, static_cast<float *>(a.partial), rg.slot, acc, lane, cnt);
+			else if (lane == 0) static_cast<T *>(a.partial)[int64_t(rg.slot) * kPartialStride] = acc;
 		}
 		__syncwarp();
 	}
+	wait();
 	if constexpr (EPI) {
+		if (done) return;
 		cnt = __reduce_add_sync(0xffffffffu, cnt);
 		if (lane == 0 && cnt) atomicAdd(e.state, (unsigned long long)cnt);
 		if (e.finish) pr_finish(e);
@@ -870,36 +930,27 @@ __device__ __forceinline__ void chunk_sums(const A *pc, uint32_t part, uint32_t 
 // others, each of the first n_long (more than kLongChunks chunks) gets a warp
 // with P = 32 / L; the rest go 32 / (2 L) rows to a warp with P = 2 (one row
 // and P = 1 when L = 32).  Deterministic, with many loads in flight.
-template <class YT, class A, bool SCALE_OUT, bool EPI>
+template <class YT, class A, bool SCALE_OUT>
 __device__ __forceinline__ void fix_store(const heavy_row &h, const A (&v)[4], int nv, YT *Y, int64_t ldy, int col,
-		const A *s_out, const pr_epi &e)
+		const A *s_out)
 {
-	if constexpr (EPI) {
-		unsigned c = 0;
-		pr_update(e, h.row, v[0], c);
-		if (c) atomicAdd(e.state, 1ull);
-	} else {
-		A so = A(1);
-		if constexpr (SCALE_OUT) so = s_out[h.row];
-		YT *y = Y + int64_t(h.row) * ldy + col;
-		for (int i = 0; i < nv; i++) {
-			A x = v[i];
-			if constexpr (SCALE_OUT) x = acc_mul(x, so);
-			y[i] = from_acc<YT, A>(x);
-		}
+	A so = A(1);
+	if constexpr (SCALE_OUT) so = s_out[h.row];
+	YT *y = Y + int64_t(h.row) * ldy + col;
+	for (int i = 0; i < nv; i++) {
+		A x = v[i];
+		if constexpr (SCALE_OUT) x = acc_mul(x, so);
+		y[i] = from_acc<YT, A>(x);
 	}
 }
 
-template <class YT, class A, bool SCALE_OUT, bool EPI = false>
+template <class YT, class A, bool SCALE_OUT>
 __global__ void __launch_bounds__(256) spmm_fixup_kernel(const heavy_row *heavy, uint32_t n_heavy, uint32_t n_block,
-		uint32_t n_long, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, int L, const pr_epi e)
+		uint32_t n_long, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, int L)
 {
 	__shared__ A red[8][32][4];
 	dep_wait();
 	dep_launch();
-	if constexpr (EPI) {
-		if (e.state[1]) return;
-	}
 	constexpr bool kVec4 = std::is_same<A, float>::value;
 	const bool vec = kVec4 && (k % 4) == 0;
 	const int units = vec ? k / 4 : k, nv = vec ? 4 : 1;
@@ -941,21 +992,17 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const heavy_row *heavy,
 					v[i] = red[0][lane][i];
 					for (int q = 1; q < 8; q++) v[i] = acc_add(v[i], red[q][lane][i]);
 				}
-				fix_store<YT, A, SCALE_OUT, EPI>(h, v, nv, Y, ldy, vec ? 4 * u : u, s_out, e);
+				fix_store<YT, A, SCALE_OUT>(h, v, nv, Y, ldy, vec ? 4 * u : u, s_out);
 			}
 			__syncthreads();
 		} else if (mine && part == 0) {
-			fix_store<YT, A, SCALE_OUT, EPI>(h, t, nv, Y, ldy, vec ? 4 * u : u, s_out, e);
+			fix_store<YT, A, SCALE_OUT>(h, t, nv, Y, ldy, vec ? 4 * u : u, s_out);
 		}
-	}
-	if constexpr (EPI) {
-		if (e.finish) pr_finish(e);
 	}
 }
 
-template <class YT, class A, bool SCALE_OUT, bool EPI = false>
-static int launch_fixup(const gpu_part &p, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out,
-		cudaStream_t st, const pr_epi &e = pr_epi{})
+template <class YT, class A, bool SCALE_OUT>
+static int launch_fixup(const gpu_part &p, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, cudaStream_t st)
 {
 	if (!p.n_heavy) return FMX_OK;
 	const bool vec = std::is_same<A, float>::value && (k % 4) == 0;
@@ -968,11 +1015,11 @@ static int launch_fixup(const gpu_part &p, const A *partial, YT *Y, int64_t ldy,
 	const uint64_t per_warp = uint64_t(32 / (L * (L < 32 ? 2 : 1)));    // short rows per warp
 	const uint64_t warps = n_long + (n_short + per_warp - 1) / per_warp;
 	const unsigned grid = nb + unsigned((warps + 7) / 8);
-	auto kern = spmm_fixup_kernel<YT, A, SCALE_OUT, EPI>;
+	auto kern = spmm_fixup_kernel<YT, A, SCALE_OUT>;
 	if (p.streamed)
-		kern<<<grid, 256, 0, st>>>(p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L, e);
+		kern<<<grid, 256, 0, st>>>(p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L);
 	else
-		CUDA_TRY(launch_dep(kern, grid, 256, st, p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L, e));
+		CUDA_TRY(launch_dep(kern, grid, 256, st, p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L));
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
 }
@@ -1407,20 +1454,18 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 				nullptr);
 		CUDA_TRY(cudaGetLastError());
 	}
-	// the loop test belongs to the iteration's last kernel
-	pr_epi es = e;
-	es.finish = e.finish && !p.n_heavy;
 	auto kern = spmv_kernel<T, WT, EPI>;
 	static std::atomic<unsigned> blocks[64];
 	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kThreads);
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
-			if (p.streamed) kern<<<b, kThreads, 0, st>>>(sa, es);
-			else CUDA_TRY(launch_dep(kern, b, kThreads, st, sa, es));
+			if (p.streamed) kern<<<b, kThreads, 0, st>>>(sa, e);
+			else CUDA_TRY(launch_dep(kern, b, kThreads, st, sa, e));
 			CUDA_TRY(cudaGetLastError());
 			return FMX_OK;
 		}))
 		return rc;
-	return launch_fixup<T, T, false, EPI>(p, static_cast<const T *>(partial), Y, ldy, 1, nullptr, st, e);
+	if constexpr (EPI) return FMX_OK;          // the kernel's last warp of a heavy row finished it
+	return launch_fixup<T, T, false>(p, static_cast<const T *>(partial), Y, ldy, 1, nullptr, st);
 }
 
 template <class XT, class YT, class A, class WT>
@@ -1537,6 +1582,12 @@ __global__ void pr_finish_kernel(unsigned long long *state, unsigned long long n
 	}
 }
 
+__global__ void chunk_heavy_kernel(const heavy_row *heavy, uint32_t n_heavy, uint32_t *chunk_heavy)
+{
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_heavy; i += gridDim.x * blockDim.x)
+		for (uint32_t c = 0; c < heavy[i].count; c++) chunk_heavy[heavy[i].first + c] = i;
+}
+
 __global__ void hot_slot_kernel(const int32_t *hot_col, uint32_t n_hot, uint32_t *slot)
 {
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_hot; i += gridDim.x * blockDim.x) slot[hot_col[i]] = i + 1;
@@ -1550,18 +1601,27 @@ __global__ void heavy_mask_kernel(const heavy_row *heavy, uint32_t n_heavy, uint
 	}
 }
 
-int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, cudaStream_t st)
+int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, uint32_t *chunk_heavy, const void **heavy,
+		cudaStream_t st)
 {
 	const gpu_part &p = *mt->a;
+	*heavy = p.heavy;
 	auto grid = [](uint32_t n) { return unsigned(std::min<uint32_t>((n + 255) / 256, 1024)); };
 	if (p.n_heavy) heavy_mask_kernel<<<grid(p.n_heavy), 256, 0, st>>>(p.heavy, p.n_heavy, mask);
+	CUDA_TRY(cudaGetLastError());
+	if (p.n_heavy) chunk_heavy_kernel<<<grid(p.n_heavy), 256, 0, st>>>(p.heavy, p.n_heavy, chunk_heavy);
 	CUDA_TRY(cudaGetLastError());
 	if (p.n_hot) hot_slot_kernel<<<grid(p.n_hot), 256, 0, st>>>(p.hot_col, p.n_hot, slot);
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
 }
 
-uint64_t pagerank_hot(const fmx_matrix *mt) { return mt->a->n_hot; }
+void pagerank_sizes(const fmx_matrix *mt, uint64_t *hot, uint64_t *heavy, uint64_t *chunks)
+{
+	*hot = mt->a->n_hot;
+	*heavy = mt->a->n_heavy;
+	*chunks = mt->a->n_partials;
+}
 bool pagerank_needs_out(const fmx_matrix *mt) { return !spmv_by_warps(*mt->a); }
 
 template <class WT>
