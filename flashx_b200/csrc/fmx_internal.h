@@ -2,6 +2,7 @@
 // libfmx.  Not installed; the public surface is include/fmx.h.
 #pragma once
 
+#include <functional>
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
@@ -93,6 +94,21 @@ int default_threads();
 cudaError_t work_alloc(void **p, size_t bytes, cudaStream_t st);
 // fmx_dense_chol_inv of G + rel * max(diag G) * I (the shift of shifted CholQR)
 int dense_chol_inv_shifted(const double *G, int b, double *T, int *info, double rel, void *stream);
+
+// Host rows of `width` bytes, `pitch` apart, and their place on the device,
+// back to back.
+struct host_copy {
+	void *dev, *host;
+	size_t width, pitch, rows;
+};
+// Copies `in` to the device, calls run() (which enqueues on st) and copies
+// `out` back; pageable memory goes through pinned slots on several host
+// threads.  All on st; on return the result has arrived where the copies of
+// `out` were pageable, else st may still be running.
+int run_host_copies(int device, cudaStream_t st, const host_copy &in, const host_copy &out,
+		const std::function<int()> &run);
+// Hands the pinned slots of `device` back.
+void release_host_slots(int device);
 
 // The device a matrix lives on.
 int matrix_device(const fmx_matrix *m);

@@ -110,6 +110,7 @@ struct gpu_part {
 	std::mutex stage_mu;
 	void *stage_x = nullptr, *stage_y = nullptr;
 	size_t stage_xb = 0, stage_yb = 0;
+	cudaStream_t stage_st = nullptr;
 	// fmx_spmm_host_async (guarded by stage_mu): a ring of two staging slots
 	// (grow-only), one stream for the copies of X in and one for the copies
 	// of Y out, so each direction runs back to back; per slot, events for X
@@ -139,7 +140,7 @@ struct gpu_part {
 			for (cudaEvent_t e : {a.x_ready, a.spmm_done, a.y_out})
 				if (e) cudaEventDestroy(e);
 		}
-		for (cudaStream_t s : {h2d_st, d2h_st})
+		for (cudaStream_t s : {h2d_st, d2h_st, stage_st})
 			if (s) cudaStreamDestroy(s);
 		if (copy_st) cudaStreamDestroy(copy_st);
 		cudaSetDevice(cur);

@@ -60,6 +60,7 @@ extern "C" int fmx_release_cached(int device)
 		std::lock_guard<std::mutex> g(pool_mu);
 		pool = pools[device];
 	}
+	release_host_slots(device);
 	if (!pool) return FMX_OK;
 	cudaError_t e = cudaMemPoolTrimTo(pool, 0);
 	if (e != cudaSuccess) return set_error(FMX_ERR_CUDA, "cudaMemPoolTrimTo failed: %s", cudaGetErrorString(e));

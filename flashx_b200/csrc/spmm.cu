@@ -1982,24 +1982,20 @@ int fmx_spmm_host(const fmx_matrix *m, int x_type, const void *X_host, int64_t l
 	};
 	rc = grow(p.stage_x, p.stage_xb, xb);
 	if (!rc) rc = grow(p.stage_y, p.stage_yb, yb);
-	cudaStream_t st = nullptr;
-	if (!rc && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) rc = set_error(FMX_ERR_CUDA, "stream creation failed");
-	// one linear copy each way when the rows are contiguous (a pitched copy
-	// of 64-byte rows moves far below the link rate)
-	auto copy = [&](void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows,
-			cudaMemcpyKind kind) {
-		if (dpitch == width && spitch == width) return cudaMemcpyAsync(dst, src, width * rows, kind, st);
-		return cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, kind, st);
-	};
-	if (!rc && copy(p.stage_x, k * xs, X_host, ldx * xs, k * xs, p.ncols, cudaMemcpyHostToDevice) != cudaSuccess)
-		rc = set_error(FMX_ERR_CUDA, "copy of X to the device failed");
-	if (!rc) rc = spmm_part(p, x_type, p.stage_x, k, y_type, p.stage_y, k, k, nullptr, nullptr, st);
-	if (!rc && copy(Y_host, ldy * ys, p.stage_y, k * ys, k * ys, p.nrows, cudaMemcpyDeviceToHost) != cudaSuccess)
-		rc = set_error(FMX_ERR_CUDA, "copy of Y to the host failed");
-	if (st) {
+	if (!rc && !p.stage_st && cudaStreamCreateWithFlags(&p.stage_st, cudaStreamNonBlocking) != cudaSuccess)
+		rc = set_error(FMX_ERR_CUDA, "stream creation failed");
+	if (!rc) {
+		cudaStream_t st = p.stage_st;
+		try {
+			rc = run_host_copies(p.device, st, {p.stage_x, const_cast<void *>(X_host), k * xs, ldx * xs, p.ncols},
+					{p.stage_y, Y_host, k * ys, ldy * ys, p.nrows}, [&] {
+						return spmm_part(p, x_type, p.stage_x, k, y_type, p.stage_y, k, k, nullptr, nullptr, st);
+					});
+		} catch (const std::exception &e) {
+			rc = set_error(FMX_ERR_OOM, "host copies: %s", e.what());
+		}
 		cudaError_t e = cudaStreamSynchronize(st);
 		if (!rc && e != cudaSuccess) rc = set_error(FMX_ERR_CUDA, "SpMM failed: %s", cudaGetErrorString(e));
-		cudaStreamDestroy(st);
 	}
 	cudaSetDevice(cur);
 	return rc;

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import oracle
-from flashx_b200 import _lib, matrix_image, sparse_matrix, create_2d_matrix
+from flashx_b200 import release_cached, _lib, matrix_image, sparse_matrix, create_2d_matrix
 from flashx_b200.graphs import rmat_edges
 
 pytestmark = pytest.mark.gpu
@@ -294,6 +294,40 @@ def test_host_buffers_e2e(torch_cuda):
     m = sparse_matrix.create(matrix_image.from_bytes(idx, mat), None)
     X = np.random.default_rng(1).integers(-8, 9, (5000, 16)).astype(np.float32)
     assert np.array_equal(m.multiply_host(X), oracle.spmm(idx, mat, X))
+
+
+@pytest.mark.parametrize("n,k,pad,dtype", [(70001, 5, 0, "float32"), (70001, 5, 3, "float32"), (262144, 1, 0, "float64"),
+                                           (33333, 33, 7, "float64"), (1 << 18, 16, 0, "float32"), (150000, 2, 1, "int32")])
+def test_host_buffers_through_pinned_slots(torch_cuda, n, k, pad, dtype):
+    """Pageable operands of more than 1 MB go through pinned slots on several
+    threads: chunk remainders, strided rows, repeated calls, calls of two
+    threads at once (the second copies directly) and after the slots were
+    handed back, each equal to the device product bit for bit."""
+    import threading
+    torch = torch_cuda
+    src, dst = _graph(n, 4 * n, 31)
+    mats = [sparse_matrix.create(matrix_image.build(src, dst, None, nrows=n, ncols=n, dedup=True), None)
+            for _ in range(2)]
+    code = {"float32": _lib.F32, "float64": _lib.F64, "int32": _lib.I32}[dtype]
+    rng = np.random.default_rng(n)
+    X = _dense(rng, (n, k + pad), np.dtype(dtype).type)
+    want = mats[0].multiply(torch.from_numpy(np.ascontiguousarray(X[:, :k])).cuda()).cpu().numpy()
+    got = [np.full((n, k + pad), 7, dtype=dtype) for _ in range(4)]
+
+    def call(m, y):
+        rc = _lib.lib.fmx_spmm_host(m.handle, code, X.ctypes.data, k + pad, code, y.ctypes.data, k + pad, k)
+        assert rc == _lib.FMX_OK, _lib.last_error()
+
+    call(mats[0], got[0])
+    release_cached(0)
+    call(mats[0], got[1])
+    th = [threading.Thread(target=call, args=(m, y)) for m, y in zip(mats, got[2:])]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for y in got:
+        assert np.array_equal(y[:, :k], want) and (y[:, k:] == 7).all()
 
 
 def test_host_buffers_async_two_streams(torch_cuda):
