@@ -34,6 +34,7 @@ constexpr uint32_t kRange = FMX_RANGE_ENTRIES;  // most target entries per multi
 #endif
 constexpr uint32_t kRangeMin = FMX_RANGE_MIN;   // fewest: small matrices get shorter runs, so that they
                                                 // still fill the grid
+constexpr uint32_t kRangeFine = 32;     // runs of the fine list (fine_entries)
 // lane groups of a full grid at k = 16 (148 SMs x 32 warps x 16 groups)
 // times the runs each should get before runs shrink below kRange
 constexpr uint64_t kRangeFill = uint64_t(FMX_RANGE_FILL_PER_GROUP) * 148 * 32 * 16;
@@ -85,6 +86,8 @@ struct gpu_part {
 	uint32_t n_exact = 0;                // rows summed in the reference's order
 	range_t *ranges = nullptr;
 	uint32_t n_ranges = 0;
+	range_t *fine = nullptr;             // the row kernel's list where it is a finer one (fine_entries)
+	uint32_t n_fine = 0;
 	heavy_row *heavy = nullptr;
 	uint32_t n_heavy = 0;
 	uint32_t n_long_heavy = 0;           // the first heavy rows, of more than kLongChunks chunks
@@ -96,7 +99,8 @@ struct gpu_part {
 	// streamed part: the entry stream stays in pinned host memory and each
 	// SpMM copies it slice by slice into two device slots (copy_st), the
 	// kernel of one slice overlapping the copy of the next
-	struct slice_t { uint64_t e0, e1; uint32_t r0, nr; };   // entries [e0, e1), ranges [r0, r0 + nr)
+	// entries [e0, e1), ranges [r0, r0 + nr), fine ranges [f0, f0 + nf)
+	struct slice_t { uint64_t e0, e1; uint32_t r0, nr, f0, nf; };
 	bool streamed = false;
 	uint32_t *h_col = nullptr;
 	void *h_val = nullptr;
@@ -126,7 +130,7 @@ struct gpu_part {
 		int cur = 0;
 		cudaGetDevice(&cur);
 		cudaSetDevice(device);
-		void *ps[] = {col, val, hot_col, xhot, ranges, heavy, partial, stage_x, stage_y, slot_col[0], slot_col[1],
+		void *ps[] = {col, val, hot_col, xhot, ranges, fine, heavy, partial, stage_x, stage_y, slot_col[0], slot_col[1],
 				slot_val[0], slot_val[1]};
 		for (void *p : ps)
 			if (p) cudaFree(p);
@@ -178,6 +182,22 @@ __host__ __device__ inline uint32_t range_entries(uint64_t total)
 	r = r < kRangeMin ? kRangeMin : (r > kRange ? kRange : r);
 	return uint32_t(r / kStep * kStep);
 }
+
+// Small matrices (runs of kRangeMin) are cut finer for the row kernel: its lane
+// groups walk a range 8 or 16 entries at a time, one memory latency each, and
+// their grid has room for more ranges than runs of kRangeMin give (whole SpMM,
+// k = 16: block model of n = 50k 24.1 us with 128-entry runs, 16.3 us with 32;
+// symmetric R-MAT scale 16 in BF16 45.5 against 37.0 us).
+// The segments of the stream are then the fine runs, and the list that
+// the warp-per-range kernel takes is made of the runs of kRangeMin, which are
+// whole fine runs since kRangeFine divides kRangeMin.  The run size of the
+// fine list, or the other list's where there is only one:
+__host__ __device__ inline uint32_t fine_entries(uint64_t total)
+{
+	const uint32_t r = range_entries(total);
+	return r == kRangeMin ? kRangeFine : r;
+}
+static_assert(kRangeMin % kRangeFine == 0 && kRangeFine % kStep == 0, "whole fine runs in a run");
 
 // Device-resident CSR (rows ascending, columns in entry order); the
 // pointers are owned by `own` and released on `st` when it is destroyed.

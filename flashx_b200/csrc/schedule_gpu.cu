@@ -173,6 +173,34 @@ __global__ void ranges_kernel(const uint32_t *perm, uint32_t nseg, const uint64_
 	}
 }
 
+// flag[s] = 1 for a segment that starts a range of the coarse list: a fine run
+// whose lens before it enter a new multiple of the coarse run size, or a chunk
+__global__ void coarse_flag_kernel(const uint64_t *seg_L0, const uint32_t *seg_slot, uint32_t nseg, uint32_t coarse,
+		uint32_t *flag)
+{
+	GRID_STRIDE(s, uint64_t(nseg) + 1)
+		flag[s] = s < nseg && (s == 0 || seg_slot[s] != kNoSlot || seg_L0[s] / coarse != seg_L0[s - 1] / coarse);
+}
+
+// its first row, slot and stream offset (the last offset is the stream's end)
+__global__ void coarse_seg_kernel(const uint32_t *flag, const uint32_t *idx, const uint64_t *at, const uint32_t *seg_row0,
+		const uint32_t *seg_slot, uint32_t nseg, uint64_t *c_at, uint32_t *c_row0, uint32_t *c_slot)
+{
+	GRID_STRIDE(s, uint64_t(nseg) + 1) {
+		if (s < nseg && !flag[s]) continue;
+		const uint32_t c = idx[s];
+		c_at[c] = at[s];
+		if (s == nseg) continue;
+		c_row0[c] = seg_row0[s];
+		c_slot[c] = seg_slot[s];
+	}
+}
+
+__global__ void coarse_len_kernel(const uint64_t *c_at, uint32_t n, uint32_t *c_plen)
+{
+	GRID_STRIDE(i, n) c_plen[i] = uint32_t(c_at[i + 1] - c_at[i]);
+}
+
 __global__ void fill_stream_kernel(uint32_t *col, uint64_t total, uint64_t padded)
 {
 	GRID_STRIDE(i, padded) col[i] = i < total ? (0u | kHot) : 0u;
@@ -358,7 +386,8 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	TRY(excl_scan(t, hflag, hidx, n + 1));
 	uint64_t total_len = 0;
 	TRY(fetch(L + n, total_len, st));
-	start_kernel<<<grid(n + 1), kT, 0, st>>>(L, n, range_entries(total_len), start);
+	const uint32_t run = fine_entries(total_len), coarse = range_entries(total_len);
+	start_kernel<<<grid(n + 1), kT, 0, st>>>(L, n, run, start);
 	SCUDA_TRY(cudaGetLastError());
 	TRY(excl_scan(t, start, sidx, n + 1));
 	uint32_t s_run = 0, n_chunks = 0, n_heavy = 0;
@@ -388,18 +417,42 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	if (total >= (1ull << 32) - 64)
 		return set_error(FMX_ERR_UNSUPPORTED, "%llu stream entries: offsets are 32-bit", (unsigned long long)total);
 
-	// 4. ranges, longest first
+	// 4. ranges, longest first: the segments, and with a fine list the whole
+	// runs too (consecutive fine runs of one bucket of the coarse size)
 	uint32_t *lk0, *lk1, *lv0, *lv1;
 	TRY(t.get(&lk0, nseg)); TRY(t.get(&lk1, nseg)); TRY(t.get(&lv0, nseg)); TRY(t.get(&lv1, nseg));
 	uint64_t &bytes = p->bytes;
-	TRY(dalloc(&p->ranges, nseg, bytes));
-	if (nseg) {
-		len_keys_kernel<<<grid(nseg), kT, 0, st>>>(seg_plen, uint32_t(nseg), lk0, lv0);
+	auto sorted_ranges = [&](range_t **out_ranges, uint64_t count, const uint64_t *s_at, const uint32_t *s_plen,
+			const uint32_t *s_row0, const uint32_t *s_slot) -> int {
+		TRY(dalloc(out_ranges, count, bytes));
+		if (!count) return FMX_OK;
+		len_keys_kernel<<<grid(count), kT, 0, st>>>(s_plen, uint32_t(count), lk0, lv0);
 		SCUDA_TRY(cudaGetLastError());
 		const uint32_t *lk = lk0, *perm = lv0;
-		TRY(sort_pairs(t, lk0, lk1, lv0, lv1, nseg, kLenBits, &lk, &perm));
-		ranges_kernel<<<grid(nseg), kT, 0, st>>>(perm, uint32_t(nseg), at, seg_plen, seg_row0, seg_slot, p->ranges);
+		TRY(sort_pairs(t, lk0, lk1, lv0, lv1, count, kLenBits, &lk, &perm));
+		ranges_kernel<<<grid(count), kT, 0, st>>>(perm, uint32_t(count), s_at, s_plen, s_row0, s_slot, *out_ranges);
 		SCUDA_TRY(cudaGetLastError());
+		return FMX_OK;
+	};
+	uint64_t n_coarse = nseg;
+	if (run == coarse) {
+		TRY(sorted_ranges(&p->ranges, nseg, at, seg_plen, seg_row0, seg_slot));
+	} else {
+		TRY(sorted_ranges(&p->fine, nseg, at, seg_plen, seg_row0, seg_slot));
+		uint32_t *cflag, *cidx, *c_row0, *c_plen, *c_slot;
+		uint64_t *c_at;
+		TRY(t.get(&cflag, nseg + 1)); TRY(t.get(&cidx, nseg + 1)); TRY(t.get(&c_row0, nseg)); TRY(t.get(&c_plen, nseg));
+		TRY(t.get(&c_slot, nseg)); TRY(t.get(&c_at, nseg + 1));
+		coarse_flag_kernel<<<grid(nseg + 1), kT, 0, st>>>(seg_L0, seg_slot, uint32_t(nseg), coarse, cflag);
+		SCUDA_TRY(cudaGetLastError());
+		TRY(excl_scan(t, cflag, cidx, nseg + 1));
+		uint32_t nc32 = 0;
+		TRY(fetch(cidx + nseg, nc32, st));
+		n_coarse = nc32;
+		coarse_seg_kernel<<<grid(nseg + 1), kT, 0, st>>>(cflag, cidx, at, seg_row0, seg_slot, uint32_t(nseg), c_at, c_row0, c_slot);
+		if (n_coarse) coarse_len_kernel<<<grid(n_coarse), kT, 0, st>>>(c_at, uint32_t(n_coarse), c_plen);
+		SCUDA_TRY(cudaGetLastError());
+		TRY(sorted_ranges(&p->ranges, n_coarse, c_at, c_plen, c_row0, c_slot));
 	}
 
 	// 5. the stream (plus kStep entries so that index prefetches stay in bounds)
@@ -437,7 +490,8 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	p->hot_entries = hc[2];
 	p->n_long_heavy = uint32_t(hc[3]);
 	p->n_block_heavy = uint32_t(hc[4]);
-	p->n_ranges = uint32_t(nseg);
+	p->n_ranges = uint32_t(n_coarse);
+	p->n_fine = run == coarse ? 0 : uint32_t(nseg);
 	p->n_heavy = n_heavy;
 	p->n_partials = n_chunks;
 	TRY(dalloc(reinterpret_cast<char **>(&p->partial), size_t(n_chunks) * kPartialStride * 8, bytes));

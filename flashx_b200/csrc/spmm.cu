@@ -619,6 +619,9 @@ spmm_lane_kernel(const spmm_args a)
 constexpr int kSpmvMax = 512;            // most entries of one range
 static_assert(((kRange - 1 + kExactMax + kStep - 1) / kStep) * kStep <= uint32_t(kSpmvMax) &&
 		kChunk <= uint32_t(kSpmvMax), "a range fits the SpMV kernel's staging");
+// ... and so does a run of kRangeMin with its fine runs padded one by one
+static_assert(kRangeMin - 1 + kExactMax + ((kRangeMin - 1 + kExactMax) / kRangeFine + 2) * (kStep - 1) <= uint32_t(kSpmvMax),
+		"a run of fine runs fits the SpMV kernel's staging");
 
 // A chunk of a PageRank row: the warp whose chunk arrives last adds the row's
 // partials, in spmm_fixup_kernel's order at k = 1 (the same parts, the same
@@ -1140,21 +1143,23 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 	// part.h, which make_part_device follows too).  Each segment starts at a
 	// multiple of kStep in the stream and is padded to one.
 	const uint32_t zero_entry = 0u | kHot;          // slot 0: the zero row
-	struct seg_t { uint64_t row0, row1; uint32_t b, e; uint32_t slot; uint64_t at; uint32_t len; };
+	struct seg_t { uint64_t row0, row1; uint32_t b, e; uint32_t slot; uint64_t at; uint32_t len; uint64_t run; };
 	std::vector<seg_t> segs;
 	std::vector<heavy_row> heavy;
 	uint32_t n_exact = 0;
+	bool has_fine = false;
 	{
 		uint64_t total = 0;
 		for (uint64_t r = 0; r < n; r++) total += seg_row_len(csr.row_ptr[r + 1] - csr.row_ptr[r]);
-		const uint32_t run = range_entries(total);
+		const uint32_t run = fine_entries(total), coarse = range_entries(total);
+		has_fine = run != coarse;
 		uint64_t L = 0, bucket = ~0ull;           // lens of the rows before r
 		for (uint64_t r = 0; r < n; r++) {
 			const uint32_t d = csr.row_ptr[r + 1] - csr.row_ptr[r];
 			const uint32_t len = seg_row_len(d);
 			n_exact += (d >= 1 && d <= kExactMax);
 			if (L / run != bucket) {
-				segs.push_back({r, r + 1, 0, 0, kNoSlot, 0, 0});
+				segs.push_back({r, r + 1, 0, 0, kNoSlot, 0, 0, L / coarse});
 				bucket = L / run;
 			} else {
 				segs.back().row1 = r + 1;
@@ -1171,7 +1176,7 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 		heavy.push_back({int32_t(r), slots, cnt});
 		for (uint32_t c = 0; c < cnt; c++) {
 			const uint32_t b = uint32_t(uint64_t(d) * c / cnt), e = uint32_t(uint64_t(d) * (c + 1) / cnt);
-			segs.push_back({r, r + 1, b, e, slots + c, 0, e - b});
+			segs.push_back({r, r + 1, b, e, slots + c, 0, e - b, 0});
 		}
 		slots += cnt;
 	}
@@ -1183,29 +1188,46 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 	}
 	if (total >= (1ull << 32) - 64)
 		return set_error(FMX_ERR_UNSUPPORTED, "%llu stream entries: offsets are 32-bit", (unsigned long long)total);
-	std::vector<range_t> ranges(segs.size());
-	for (size_t i = 0; i < segs.size(); i++)
-		ranges[i] = {uint32_t(segs[i].at), segs[i].len, uint32_t(segs[i].row0), segs[i].slot};
+	// the segments as ranges, and the list of whole runs (equal to them without
+	// a fine list); starts[i]: the first segment of the i-th whole run
+	std::vector<range_t> fine(segs.size()), ranges;
+	std::vector<size_t> starts;
+	for (size_t i = 0; i < segs.size(); i++) {
+		const seg_t &g = segs[i];
+		fine[i] = {uint32_t(g.at), g.len, uint32_t(g.row0), g.slot};
+		if (i && has_fine && g.slot == kNoSlot && segs[i - 1].run == g.run) {
+			ranges.back().len += g.len;
+		} else {
+			ranges.push_back(fine[i]);
+			starts.push_back(i);
+		}
+	}
+	starts.push_back(segs.size());
 	// largest ranges first, so that round-robin assignment balances the groups
-	// (within each slice of a streamed part: a slice is whole segments in
-	// stream order, at least slice_entries entries but the last)
+	// (within each slice of a streamed part: a slice is whole runs in stream
+	// order, at least slice_entries entries but the last)
 	auto by_len = [](const range_t &x, const range_t &y) { return x.len > y.len; };
 	if (slice_entries) {
 		p->streamed = true;
 		uint64_t e0 = 0;
 		size_t i0 = 0;
-		for (size_t i = 0; i < segs.size(); i++) {
-			const uint64_t e1 = segs[i].at + segs[i].len;
-			if (e1 - e0 >= slice_entries || i + 1 == segs.size()) {
-				p->slices.push_back({e0, e1, uint32_t(i0), uint32_t(i + 1 - i0)});
-				std::stable_sort(ranges.begin() + i0, ranges.begin() + i + 1, by_len);
+		for (size_t i = 0; i < ranges.size(); i++) {
+			const uint64_t e1 = uint64_t(ranges[i].e0) + ranges[i].len;
+			if (e1 - e0 >= slice_entries || i + 1 == ranges.size()) {
+				const size_t f0 = starts[i0], f1 = starts[i + 1];
+				p->slices.push_back({e0, e1, uint32_t(i0), uint32_t(i + 1 - i0), uint32_t(f0), uint32_t(f1 - f0)});
+				std::stable_sort(fine.begin() + f0, fine.begin() + f1, by_len);
 				e0 = e1;
 				i0 = i + 1;
 			}
 		}
+		for (const auto &sl : p->slices)
+			std::stable_sort(ranges.begin() + sl.r0, ranges.begin() + sl.r0 + sl.nr, by_len);
 	} else {
+		std::stable_sort(fine.begin(), fine.end(), by_len);
 		std::stable_sort(ranges.begin(), ranges.end(), by_len);
 	}
+	if (!has_fine) fine.clear();
 
 	// the entry stream (plus kStep entries so that index prefetches stay in bounds)
 	const size_t padded = total + kStep;
@@ -1262,6 +1284,7 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 	}
 	if (!rc) rc = upload(&p->hot_col, hot_col.data(), hot_col.size(), bytes);
 	if (!rc) rc = upload(&p->ranges, ranges.data(), ranges.size(), bytes);
+	if (!rc) rc = upload(&p->fine, fine.data(), fine.size(), bytes);
 	// longest first (the fixup gives each long row a warp and packs the short
 	// ones several to a warp); ties keep row order
 	std::stable_sort(heavy.begin(), heavy.end(), [](const heavy_row &x, const heavy_row &y) { return x.count > y.count; });
@@ -1273,6 +1296,7 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 	p->n_hot = uint32_t(hot_col.size());
 	p->n_exact = n_exact;
 	p->n_ranges = uint32_t(ranges.size());
+	p->n_fine = uint32_t(fine.size());
 	p->n_heavy = uint32_t(heavy.size());
 	p->n_partials = slots;
 	auto scratch = [&](void **ptr, size_t sz, const char *what) {
@@ -1332,6 +1356,7 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 {
 	if (!p.streamed) return launch(a);
 	gpu_part &q = const_cast<gpu_part &>(p);
+	const bool fine = p.fine && a.ranges == p.fine;
 	CUDA_TRY(cudaEventRecord(q.ev_start, st));
 	CUDA_TRY(cudaStreamWaitEvent(q.copy_st, q.ev_start, 0));
 	for (size_t i = 0; i < p.slices.size(); i++) {
@@ -1349,8 +1374,8 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 		a.col = q.slot_col[b] - sl.e0;
 		a.val = p.esize ? static_cast<const void *>(static_cast<const char *>(q.slot_val[b]) - sl.e0 * p.esize)
 				: nullptr;
-		a.ranges = p.ranges + sl.r0;
-		a.n_ranges = sl.nr;
+		a.ranges = fine ? p.fine + sl.f0 : p.ranges + sl.r0;
+		a.n_ranges = fine ? sl.nf : sl.nr;
 		if (int rc = launch(a)) return rc;
 		CUDA_TRY(cudaEventRecord(q.ev_free[b], st));
 	}
@@ -1486,14 +1511,14 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 	for (int64_t c0 = 0; c0 < k; c0 += panel) {
 		const int kp = int(std::min<int64_t>(panel, k - c0));
 		spmm_args a{};
-		a.col = p.col; a.val = p.val; a.ranges = p.ranges;
+		a.col = p.col; a.val = p.val; a.ranges = p.fine ? p.fine : p.ranges;
 		a.X = static_cast<const XT *>(X) + c0;
 		a.xhot = xhot;
 		a.hot_ld = kp;                // packed rows back to back (two 64-byte rows per line)
 		a.Y = static_cast<YT *>(Y) + c0;
 		a.s_in = sin; a.s_out = sout; a.partial = partial;
 		a.ldx = ldx; a.ldy = ldy; a.k = kp;
-		a.n_ranges = p.n_ranges;
+		a.n_ranges = p.fine ? p.n_fine : p.n_ranges;
 		a.G = kp / vn;
 		a.R = 32 / a.G;
 		if (int rc = launch_pack<XT, A>(p, static_cast<const XT *>(a.X), ldx, kp, static_cast<XT *>(xhot), kp,
@@ -1640,11 +1665,11 @@ static int pr_iteration_typed(const gpu_part &p, const float *in, float *xhot, f
 	// the row kernel of fmx_spmm at k = 1, then the update over all rows: a row
 	// close there would wait on its own loads of deg and pr1
 	spmm_args a{};
-	a.col = p.col; a.val = p.val; a.ranges = p.ranges;
+	a.col = p.col; a.val = p.val; a.ranges = p.fine ? p.fine : p.ranges;
 	a.X = in; a.xhot = xhot; a.hot_ld = 1;
 	a.Y = out; a.partial = p.partial;
 	a.ldx = a.ldy = 1; a.k = 1; a.G = 1; a.R = 32;
-	a.n_ranges = p.n_ranges;
+	a.n_ranges = p.fine ? p.n_fine : p.n_ranges;
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
 			return launch_lanes<float, float, float, WT, 1, false, false>(p, sa, st);
 		}))
@@ -2121,9 +2146,9 @@ int fmx_matrix_layout_digest(const fmx_matrix *m, int transpose, uint64_t *diges
 	for (const range_t &r : rg) total = std::max<uint64_t>(total, uint64_t(r.e0) + r.len);
 	const size_t padded = size_t(total) + kStep;
 	const uint64_t counts[] = {p.nrows, p.ncols, p.nnz, p.n_hot, p.n_exact, p.n_ranges, p.n_heavy, p.n_long_heavy,
-			p.n_block_heavy, p.n_partials, p.hot_entries};
+			p.n_block_heavy, p.n_partials, p.hot_entries, p.n_fine};
 	mix_host(counts, sizeof(counts));
-	for (int rc : {mix(p.ranges, rg.size() * sizeof(range_t)), mix(p.col, padded * sizeof(uint32_t)),
+	for (int rc : {mix(p.ranges, rg.size() * sizeof(range_t)), mix(p.fine, size_t(p.n_fine) * sizeof(range_t)), mix(p.col, padded * sizeof(uint32_t)),
 			mix(p.val, p.esize ? padded * p.esize : 0), mix(p.heavy, size_t(p.n_heavy) * sizeof(heavy_row)),
 			mix(p.hot_col, size_t(p.n_hot) * sizeof(int32_t))})
 		if (rc) return rc;
@@ -2137,7 +2162,7 @@ int fmx_matrix_schedule(const fmx_matrix *m, uint64_t *n_light_rows, uint64_t *n
 	if (!m || !m->a) return set_error(FMX_ERR_INVAL, "null matrix");
 	const gpu_part &p = *m->a;
 	if (n_light_rows) *n_light_rows = p.n_exact;
-	if (n_split_tasks) *n_split_tasks = p.n_ranges;
+	if (n_split_tasks) *n_split_tasks = p.fine ? p.n_fine : p.n_ranges;
 	if (n_heavy_rows) *n_heavy_rows = p.n_heavy;
 	if (kernels_per_spmm)
 		*kernels_per_spmm = 2 + (p.n_heavy ? 1 : 0);
