@@ -312,13 +312,36 @@ static int excl_scan(tmp &t, const TI *in, TO *out, uint64_t n)
 	return FMX_OK;
 }
 
-template <class T>
-static int fetch(const T *dev, T &host, cudaStream_t st)
-{
-	SCUDA_TRY(cudaMemcpyAsync(&host, dev, sizeof(T), cudaMemcpyDeviceToHost, st));
-	SCUDA_TRY(cudaStreamSynchronize(st));
-	return FMX_OK;
-}
+// Counts come back through pinned words (one set per host thread): several
+// copies share one wait, where each copy into pageable memory is a wait of its
+// own.
+struct counts_back {
+	cudaStream_t st;
+	unsigned long long *w = nullptr;
+	int n = 0;
+	explicit counts_back(cudaStream_t s) : st(s) {}
+	int init()
+	{
+		static thread_local unsigned long long *pinned = nullptr;
+		if (!pinned) SCUDA_TRY(cudaMallocHost(&pinned, 16 * sizeof(unsigned long long)));
+		w = pinned;
+		return FMX_OK;
+	}
+	template <class T>
+	int ask(const T *dev)
+	{
+		w[n] = 0;
+		SCUDA_TRY(cudaMemcpyAsync(w + n, dev, sizeof(T), cudaMemcpyDeviceToHost, st));
+		n++;
+		return FMX_OK;
+	}
+	int wait()
+	{
+		SCUDA_TRY(cudaStreamSynchronize(st));
+		n = 0;
+		return FMX_OK;
+	}
+};
 
 template <class T>
 static int dalloc(T **p, size_t count, uint64_t &bytes)
@@ -368,11 +391,6 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	SCUDA_TRY(cudaGetLastError());
 	const uint32_t *hkey = hk0, *hot_sorted = hv0;
 	if (nc) TRY(sort_pairs(t, hk0, hk1, hv0, hv1, nc, kDegBits, &hkey, &hot_sorted));
-	unsigned long long ncand = 0;
-	TRY(fetch(cnt + 0, ncand, st));
-	const uint32_t nhot = uint32_t(std::min<unsigned long long>(kHotMax, ncand));
-	if (nhot) slot_kernel<<<grid(nhot), kT, 0, st>>>(hot_sorted, nhot, slot_of);
-	SCUDA_TRY(cudaGetLastError());
 
 	// 2. rows
 	uint64_t *lens, *L;
@@ -384,16 +402,25 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	TRY(excl_scan(t, lens, L, n + 1));
 	TRY(excl_scan(t, chunks, cfirst, n + 1));
 	TRY(excl_scan(t, hflag, hidx, n + 1));
-	uint64_t total_len = 0;
-	TRY(fetch(L + n, total_len, st));
+	counts_back back(st);
+	TRY(back.init());
+	TRY(back.ask(cnt + 0));
+	TRY(back.ask(L + n));
+	TRY(back.ask(cfirst + n));
+	TRY(back.ask(hidx + n));
+	TRY(back.wait());
+	const uint32_t nhot = uint32_t(std::min<unsigned long long>(kHotMax, back.w[0]));
+	const uint64_t total_len = back.w[1];
+	const uint32_t n_chunks = uint32_t(back.w[2]), n_heavy = uint32_t(back.w[3]);
+	if (nhot) slot_kernel<<<grid(nhot), kT, 0, st>>>(hot_sorted, nhot, slot_of);
+	SCUDA_TRY(cudaGetLastError());
 	const uint32_t run = fine_entries(total_len), coarse = range_entries(total_len);
 	start_kernel<<<grid(n + 1), kT, 0, st>>>(L, n, run, start);
 	SCUDA_TRY(cudaGetLastError());
 	TRY(excl_scan(t, start, sidx, n + 1));
-	uint32_t s_run = 0, n_chunks = 0, n_heavy = 0;
-	SCUDA_TRY(cudaMemcpyAsync(&s_run, sidx + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-	SCUDA_TRY(cudaMemcpyAsync(&n_chunks, cfirst + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-	TRY(fetch(hidx + n, n_heavy, st));
+	TRY(back.ask(sidx + n));
+	TRY(back.wait());
+	const uint32_t s_run = uint32_t(back.w[0]);
 	const uint64_t nseg = uint64_t(s_run) + n_chunks;
 
 	// 3. segments
@@ -412,13 +439,28 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	SCUDA_TRY(cudaMemsetAsync(seg_plen + nseg, 0, sizeof(uint32_t), st));
 	SCUDA_TRY(cudaGetLastError());
 	TRY(excl_scan(t, seg_plen, at, nseg + 1));
-	uint64_t total = 0;
-	TRY(fetch(at + nseg, total, st));
+	// a fine list: the whole runs too (consecutive fine runs of one bucket of
+	// the coarse size)
+	const bool has_fine = run != coarse;
+	uint32_t *cflag = nullptr, *cidx = nullptr, *c_row0 = nullptr, *c_plen = nullptr, *c_slot = nullptr;
+	uint64_t *c_at = nullptr;
+	if (has_fine) {
+		TRY(t.get(&cflag, nseg + 1)); TRY(t.get(&cidx, nseg + 1)); TRY(t.get(&c_row0, nseg)); TRY(t.get(&c_plen, nseg));
+		TRY(t.get(&c_slot, nseg)); TRY(t.get(&c_at, nseg + 1));
+		coarse_flag_kernel<<<grid(nseg + 1), kT, 0, st>>>(seg_L0, seg_slot, uint32_t(nseg), coarse, cflag);
+		SCUDA_TRY(cudaGetLastError());
+		TRY(excl_scan(t, cflag, cidx, nseg + 1));
+		coarse_seg_kernel<<<grid(nseg + 1), kT, 0, st>>>(cflag, cidx, at, seg_row0, seg_slot, uint32_t(nseg), c_at, c_row0, c_slot);
+		SCUDA_TRY(cudaGetLastError());
+	}
+	TRY(back.ask(at + nseg));
+	if (has_fine) TRY(back.ask(cidx + nseg));
+	TRY(back.wait());
+	const uint64_t total = back.w[0], n_coarse = has_fine ? back.w[1] : nseg;
 	if (total >= (1ull << 32) - 64)
 		return set_error(FMX_ERR_UNSUPPORTED, "%llu stream entries: offsets are 32-bit", (unsigned long long)total);
 
-	// 4. ranges, longest first: the segments, and with a fine list the whole
-	// runs too (consecutive fine runs of one bucket of the coarse size)
+	// 4. ranges, longest first: the segments, and with a fine list the whole runs
 	uint32_t *lk0, *lk1, *lv0, *lv1;
 	TRY(t.get(&lk0, nseg)); TRY(t.get(&lk1, nseg)); TRY(t.get(&lv0, nseg)); TRY(t.get(&lv1, nseg));
 	uint64_t &bytes = p->bytes;
@@ -434,22 +476,8 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 		SCUDA_TRY(cudaGetLastError());
 		return FMX_OK;
 	};
-	uint64_t n_coarse = nseg;
-	if (run == coarse) {
-		TRY(sorted_ranges(&p->ranges, nseg, at, seg_plen, seg_row0, seg_slot));
-	} else {
-		TRY(sorted_ranges(&p->fine, nseg, at, seg_plen, seg_row0, seg_slot));
-		uint32_t *cflag, *cidx, *c_row0, *c_plen, *c_slot;
-		uint64_t *c_at;
-		TRY(t.get(&cflag, nseg + 1)); TRY(t.get(&cidx, nseg + 1)); TRY(t.get(&c_row0, nseg)); TRY(t.get(&c_plen, nseg));
-		TRY(t.get(&c_slot, nseg)); TRY(t.get(&c_at, nseg + 1));
-		coarse_flag_kernel<<<grid(nseg + 1), kT, 0, st>>>(seg_L0, seg_slot, uint32_t(nseg), coarse, cflag);
-		SCUDA_TRY(cudaGetLastError());
-		TRY(excl_scan(t, cflag, cidx, nseg + 1));
-		uint32_t nc32 = 0;
-		TRY(fetch(cidx + nseg, nc32, st));
-		n_coarse = nc32;
-		coarse_seg_kernel<<<grid(nseg + 1), kT, 0, st>>>(cflag, cidx, at, seg_row0, seg_slot, uint32_t(nseg), c_at, c_row0, c_slot);
+	TRY(sorted_ranges(has_fine ? &p->fine : &p->ranges, nseg, at, seg_plen, seg_row0, seg_slot));
+	if (has_fine) {
 		if (n_coarse) coarse_len_kernel<<<grid(n_coarse), kT, 0, st>>>(c_at, uint32_t(n_coarse), c_plen);
 		SCUDA_TRY(cudaGetLastError());
 		TRY(sorted_ranges(&p->ranges, n_coarse, c_at, c_plen, c_row0, c_slot));
@@ -482,22 +510,21 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	TRY(dalloc(&p->hot_col, nhot, bytes));
 	if (nhot) SCUDA_TRY(cudaMemcpyAsync(p->hot_col, hot_sorted, nhot * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
 
-	unsigned long long hc[5] = {};
-	SCUDA_TRY(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
-	SCUDA_TRY(cudaStreamSynchronize(st));
+	TRY(dalloc(reinterpret_cast<char **>(&p->partial), size_t(n_chunks) * kPartialStride * 8, bytes));
+	TRY(dalloc(reinterpret_cast<char **>(&p->xhot), size_t(nhot + 1) * kPanelBytes, bytes));
+	SCUDA_TRY(cudaMemsetAsync(p->xhot, 0, size_t(nhot + 1) * kPanelBytes, st));
+	for (int q = 1; q < 5; q++) TRY(back.ask(cnt + q));
+	TRY(back.wait());
+	const unsigned long long *hc = back.w - 1;   // n_exact, hot_entries, n_long, n_block
 	p->n_hot = nhot;
 	p->n_exact = uint32_t(hc[1]);
 	p->hot_entries = hc[2];
 	p->n_long_heavy = uint32_t(hc[3]);
 	p->n_block_heavy = uint32_t(hc[4]);
 	p->n_ranges = uint32_t(n_coarse);
-	p->n_fine = run == coarse ? 0 : uint32_t(nseg);
+	p->n_fine = has_fine ? uint32_t(nseg) : 0;
 	p->n_heavy = n_heavy;
 	p->n_partials = n_chunks;
-	TRY(dalloc(reinterpret_cast<char **>(&p->partial), size_t(n_chunks) * kPartialStride * 8, bytes));
-	TRY(dalloc(reinterpret_cast<char **>(&p->xhot), size_t(nhot + 1) * kPanelBytes, bytes));
-	SCUDA_TRY(cudaMemsetAsync(p->xhot, 0, size_t(nhot + 1) * kPanelBytes, st));
-	SCUDA_TRY(cudaStreamSynchronize(st));
 	out = p;
 	return FMX_OK;
 }
