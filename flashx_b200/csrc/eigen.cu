@@ -105,18 +105,6 @@ __global__ void copy_cols_kernel(const float *in, int64_t ldi, float *out, int64
 	}
 }
 
-// One Chebyshev step on flat n x b blocks:  O = alpha (W - c0 Y) - beta P
-template <class YT, class PT, class OT>
-__global__ void cheb_kernel(const float *__restrict__ W, const YT *__restrict__ Y, const PT *__restrict__ P,
-		OT *__restrict__ O, int64_t count, float alpha, float c0, float beta)
-{
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
-		float v = alpha * (W[i] - c0 * ldf(Y + i));
-		if (P) v -= beta * ldf(P + i);
-		stf(O + i, v);
-	}
-}
-
 // One step of the filter in correction form, on flat n x b blocks:
 //   O = alpha W - ac0 E - beta P + cr[col] R + cx[col] X
 // (each of W, E, P, R, X may be absent); R FP32 or BF16.  With Rb, the step
@@ -175,11 +163,75 @@ __device__ __forceinline__ void st8(__nv_bfloat16 *p, const float (&v)[8])
 	*reinterpret_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Where a filter step leaves the hot rows of its block for the SpMM that reads
+// it (hot_pack_target): row r times s[r], rounded as that pack rounds it, at
+// xhot + slot[r] * b; slot null: nothing to leave.  The step has the rows at
+// hand, where the pack kernel gathers them again (4.3 us per SpMM at n = 50k,
+// 50 us at n = 4.2M).
+template <class T>
+struct pack_out {
+	const uint32_t *slot = nullptr;
+	T *xhot = nullptr;
+	const float *s = nullptr;
+	int b = 0, shift = -1;               // b = 2^shift, or -1
+
+	__device__ __forceinline__ void zero_row() const
+	{
+		if (slot && blockIdx.x == 0 && threadIdx.x < unsigned(b)) stf(xhot + threadIdx.x, 0.f);
+	}
+	template <int N>
+	__device__ __forceinline__ void put(int64_t i, const float (&v)[N]) const
+	{
+		if (!slot) return;
+		const uint32_t r = shift >= 0 ? uint32_t(i >> shift) : uint32_t(i / b);
+		const uint32_t q = __ldg(slot + r);
+		if (!q) return;
+		const float sc = s ? __ldg(s + r) : 1.f;
+		T *o = xhot + int64_t(q) * b + (i - int64_t(r) * b);
+#pragma unroll
+		for (int k = 0; k < N; k++) {
+			T t;
+			stf(&t, v[k]);                       // the block's own rounding first
+			stf(o + k, __fmul_rn(ldf(&t), sc));
+		}
+	}
+};
+
+// One Chebyshev step on flat n x b blocks:  O = alpha (W - c0 Y) - beta P, four
+// elements per thread where the rows are whole groups of four
+__global__ void cheb_kernel(const float *__restrict__ W, const float *__restrict__ Y, const float *__restrict__ P,
+		float *__restrict__ O, int64_t count, int b, float alpha, float c0, float beta, pack_out<float> hot)
+{
+	hot.zero_row();
+	// the roundings written out, so that every form gives the same bits
+	auto step = [&](float w, float y, float p) {
+		const float t = __fmaf_rn(-c0, y, w);
+		return P ? __fmaf_rn(alpha, t, -__fmul_rn(beta, p)) : __fmul_rn(alpha, t);
+	};
+	const int64_t t0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
+	if ((b & 3) == 0) {
+		for (int64_t i = 4 * t0; i < count; i += 4 * stride) {
+			const float4 w = ld4(W + i), y = ld4(Y + i);
+			const float4 p = P ? ld4(P + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+			const float v[4] = {step(w.x, y.x, p.x), step(w.y, y.y, p.y), step(w.z, y.z, p.z), step(w.w, y.w, p.w)};
+			st4(O + i, make_float4(v[0], v[1], v[2], v[3]));
+			hot.put(i, v);
+		}
+		return;
+	}
+	for (int64_t i = t0; i < count; i += stride) {
+		const float v[1] = {step(W[i], Y[i], P ? P[i] : 0.f)};
+		O[i] = v[0];
+		hot.put(i, v);
+	}
+}
+
 template <class WT, class ET, class PT, class RT, class OT>
 __global__ void corr_kernel(const WT *__restrict__ W, const ET *__restrict__ E, const PT *__restrict__ P,
 		const RT *__restrict__ R, const float *__restrict__ X, OT *__restrict__ O, int64_t count, int b,
-		float alpha, float ac0, float beta, col_coefs cf, __nv_bfloat16 *__restrict__ Rb)
+		float alpha, float ac0, float beta, col_coefs cf, __nv_bfloat16 *__restrict__ Rb, pack_out<OT> hot)
 {
+	hot.zero_row();
 	const bool pow2 = (b & (b - 1)) == 0;
 	const int64_t tstride = int64_t(gridDim.x) * blockDim.x;
 	if ((b & 7) == 0) {
@@ -218,6 +270,7 @@ __global__ void corr_kernel(const WT *__restrict__ W, const ET *__restrict__ E, 
 				for (int q = 0; q < 8; q++) v[q] += cf.x[col + q] * t[q];
 			}
 			st8(O + i, v);
+			hot.put(i, v);
 		}
 		return;
 	}
@@ -249,6 +302,8 @@ __global__ void corr_kernel(const WT *__restrict__ W, const ET *__restrict__ E, 
 				v.x += cf.x[col] * t.x; v.y += cf.x[col + 1] * t.y; v.z += cf.x[col + 2] * t.z; v.w += cf.x[col + 3] * t.w;
 			}
 			st4(O + i, v);
+			const float o[4] = {v.x, v.y, v.z, v.w};
+			hot.put(i, o);
 		}
 		return;
 	}
@@ -265,6 +320,8 @@ __global__ void corr_kernel(const WT *__restrict__ W, const ET *__restrict__ E, 
 		}
 		if (X) v += cf.x[col] * X[i];
 		stf(O + i, v);
+		const float o[1] = {v};
+		hot.put(i, o);
 	}
 }
 
@@ -703,7 +760,8 @@ struct solver {
 	// One application of the operator to k columns: diag(s) A diag(s) X, or
 	// A^T (A X) for the Gram operator (the intermediate in the output's type
 	// when the input is BF16, as the SpMM's type pairs require).
-	int spmm(int xt, const void *Xin, int k, void *Out, int yt = FMX_F32)
+	// `packed`: the step that wrote Xin left its hot rows (pack_for).
+	int spmm(int xt, const void *Xin, int k, void *Out, int yt = FMX_F32, bool packed = false)
 	{
 		if (o.op == FMX_EIGEN_OP_GRAM) {
 			const int tt = xt == FMX_BF16 ? yt : FMX_F32;
@@ -713,7 +771,8 @@ struct solver {
 			num_ops += 2 * k;
 			return FMX_OK;
 		}
-		E_TRY(fmx_spmm(m, xt, Xin, b, yt, Out, b, k, s, s, st));
+		if (packed) E_TRY(spmm_packed(m, xt, Xin, b, yt, Out, b, k, s, s, st));
+		else E_TRY(fmx_spmm(m, xt, Xin, b, yt, Out, b, k, s, s, st));
 		spmm_calls++;
 		num_ops += k;
 		return FMX_OK;
@@ -866,11 +925,33 @@ struct solver {
 		return finish_small();
 	}
 
-	template <class YT, class PT, class OT>
-	int cheb(const float *Wm, const YT *Y, const PT *P, OT *Out, float alpha, float c0, float beta)
+	// Whether a filter step writes the hot pack of the product that follows it
+	// (blocks that the SpMM takes as one panel: odd widths in at most 32
+	// one-element lanes), and its place.
+	template <class T>
+	bool packs() const
+	{
+		return o.op == FMX_EIGEN_OP_SCALED && b * int(sizeof(T)) <= pack_target(m).panel_bytes && (b % 2 == 0 || b <= 32);
+	}
+	template <class T>
+	pack_out<T> pack_for(bool want) const
+	{
+		pack_out<T> h;
+		if (!want || !packs<T>()) return h;
+		const hot_pack_target t = pack_target(m);
+		h.slot = t.slot;
+		h.xhot = static_cast<T *>(t.xhot);
+		h.s = s;
+		h.b = b;
+		h.shift = (b & (b - 1)) ? -1 : __builtin_ctz(unsigned(b));
+		return h;
+	}
+
+	int cheb(const float *Wm, const float *Y, const float *P, float *Out, float alpha, float c0, float beta, bool feeds)
 	{
 		const int64_t cnt = n * b;
-		cheb_kernel<YT, PT, OT><<<flat_grid(cnt), kThreads, 0, st>>>(Wm, Y, P, Out, cnt, alpha, c0, beta);
+		cheb_kernel<<<flat_grid(b & 3 ? cnt : cnt / 4), kThreads, 0, st>>>(Wm, Y, P, Out, cnt, b, alpha, c0, beta,
+				pack_for<float>(feeds));
 		ECUDA_TRY(cudaGetLastError());
 		return FMX_OK;
 	}
@@ -884,14 +965,14 @@ struct solver {
 		const double c0 = (cut + lo) / 2;
 		const double s1 = e / (up - c0);
 		double sj = s1;
-		E_TRY(cheb(NX, X, (const float *)nullptr, B[0], float(s1 / e), float(c0), 0.f));
+		E_TRY(cheb(NX, X, nullptr, B[0], float(s1 / e), float(c0), 0.f, mdeg > 1));
 		int cur = 0, prev = -1;                           // prev -1 = X
 		for (int j = 2; j <= mdeg; j++) {
 			const double sn = 1.0 / (2.0 / s1 - sj);
-			E_TRY(spmm(FMX_F32, B[cur], b, W));
+			E_TRY(spmm(FMX_F32, B[cur], b, W, FMX_F32, packs<float>()));
 			const int nxt = (cur + 1) % 3 == prev ? (cur + 2) % 3 : (cur + 1) % 3;
 			const float *P = prev < 0 ? X : B[prev];
-			E_TRY(cheb(W, (const float *)B[cur], P, B[nxt], float(2 * sn / e), float(c0), float(sj * sn)));
+			E_TRY(cheb(W, B[cur], P, B[nxt], float(2 * sn / e), float(c0), float(sj * sn), j < mdeg));
 			prev = cur;
 			cur = nxt;
 			sj = sn;
@@ -902,11 +983,11 @@ struct solver {
 
 	template <class WT, class ET, class PT, class RT, class OT>
 	int corr_step(const WT *Wm, const ET *E, const PT *P, const RT *R, const float *Xs, OT *Out, float alpha,
-			float ac0, float beta, const col_coefs &cf, __nv_bfloat16 *Rb = nullptr)
+			float ac0, float beta, const col_coefs &cf, __nv_bfloat16 *Rb = nullptr, bool feeds = false)
 	{
 		const int64_t cnt = n * b;
 		corr_kernel<WT, ET, PT, RT, OT><<<flat_grid(cnt), kThreads, 0, st>>>(Wm, E, P, R, Xs, Out, cnt, b, alpha, ac0,
-				beta, cf, Rb);
+				beta, cf, Rb, pack_for<OT>(feeds));
 		ECUDA_TRY(cudaGetLastError());
 		return FMX_OK;
 	}
@@ -944,7 +1025,7 @@ struct solver {
 		// E_1, and R in BF16 for the middle steps (their BF16 operands carry
 		// the same relative rounding)
 		E_TRY(corr_step((const float *)nullptr, (const float *)nullptr, (const float *)nullptr, R,
-				(const float *)nullptr, (bf *)B[0], 0.f, 0.f, 0.f, cf, Rb));
+				(const float *)nullptr, (bf *)B[0], 0.f, 0.f, 0.f, cf, Rb, true));
 		int cur = 0, prev = -1;
 		double sj = s1;
 		for (int jdeg = 2; jdeg <= mdeg; jdeg++) {
@@ -952,7 +1033,7 @@ struct solver {
 			const double alpha = 2 * sn / e, beta = sj * sn;
 			const bool last = jdeg == mdeg;
 			// W = A_s E in BF16 too: its rounding is relative to the correction
-			E_TRY(spmm(FMX_BF16, B[cur], b, W, FMX_BF16));
+			E_TRY(spmm(FMX_BF16, B[cur], b, W, FMX_BF16, packs<bf>()));
 			for (int j = 0; j < b; j++) {
 				Dn[j] = alpha * (hsmall->theta[j] - c0) * Dc[j] - beta * Dp[j];
 				cf.r[j] = float(alpha * Dc[j]);
@@ -964,7 +1045,7 @@ struct solver {
 			const float a = float(alpha), ac = float(alpha * c0), bt = float(beta);
 			const bf *Wb = (const bf *)W;
 			if (last) E_TRY(corr_step(Wb, E, P, R, X, B[nxt], a, ac, bt, cf));
-			else E_TRY(corr_step(Wb, E, P, (const bf *)Rb, (const float *)nullptr, (bf *)B[nxt], a, ac, bt, cf));
+			else E_TRY(corr_step(Wb, E, P, (const bf *)Rb, (const float *)nullptr, (bf *)B[nxt], a, ac, bt, cf, nullptr, true));
 			prev = cur;
 			cur = nxt;
 			sj = sn;

@@ -139,6 +139,21 @@ struct device_guard {
 // A matrix from host CSR (and its transpose, or null for a symmetric one).
 int matrix_from_csr(const host_csr &a, const host_csr *at, int device, fmx_matrix **out);
 
+// ---- products whose producer fills the hot pack -----------------------------
+// The kernel that writes X can write X's hot rows to the matrix's hot pack as
+// it goes, which saves the product its pack kernel: the row of column c,
+// scaled by s_in and rounded as the pack rounds it, at xhot + slot[c] * k
+// elements when slot[c] != 0, and zeros at xhot[0 .. k).  For panels of at most
+// panel_bytes per row; spmm_packed then runs the product.
+struct hot_pack_target {
+	const uint32_t *slot;
+	void *xhot;
+	int panel_bytes;
+};
+hot_pack_target pack_target(const fmx_matrix *m);
+int spmm_packed(const fmx_matrix *m, int xt, const void *X, int64_t ldx, int yt, void *Y, int64_t ldy, int64_t k,
+		const void *sin, const void *sout, cudaStream_t st);
+
 // ---- fused PageRank iteration ----------------------------------------------
 // The update of fm::alg::PageRank (PageRank.cpp:110-123) applied where the
 // SpMV on A^T closes a row: p2 = out * d + teleport; converged += |pr1 - p2|
@@ -173,10 +188,9 @@ bool pagerank_needs_out(const fmx_matrix *mt);
 // Hot columns of mt's part (a pack holds one value more: slot 0 is zero), its
 // chunked rows and their chunks.
 void pagerank_sizes(const fmx_matrix *mt, uint64_t *hot, uint64_t *heavy, uint64_t *chunks);
-// Set heavy_mask (ceil(nrows / 32) words) and chunk_heavy from mt's chunked
-// rows, whose list is *heavy, and slot (nrows words) from its hot columns;
-// mask and slot zeroed by the caller.
-int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, uint32_t *chunk_heavy, const void **heavy,
+// Set heavy_mask (ceil(nrows / 32) words, zeroed by the caller) and chunk_heavy
+// from mt's chunked rows, whose list is *heavy; *slot: its columns' hot slots.
+int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *chunk_heavy, const uint32_t **slot, const void **heavy,
 		cudaStream_t st);
 
 } // namespace fmx

@@ -111,7 +111,7 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	cudaStream_t st = g.st;
 	const int64_t n = int64_t(nr);
 	float *deg, *in0, *in1, *pr1, *xh0, *xh1, *out = nullptr;
-	uint32_t *mask, *slot, *arrived, *chunk_heavy;
+	uint32_t *mask, *arrived, *chunk_heavy;
 	unsigned long long *state;
 	auto alloc = [&](void **q, size_t bytes) -> int {
 		cudaError_t e = work_alloc(q, std::max<size_t>(bytes, 16), st);
@@ -122,18 +122,17 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	const size_t mask_words = size_t((n + 31) / 32);
 	for (float **b : {&deg, &in0, &in1, &pr1}) P_TRY(alloc(reinterpret_cast<void **>(b), size_t(n) * sizeof(float)));
 	// one block of zeroed words: the loop state, the two hot packs (their slot
-	// 0 stays zero), the mask, the slots and the arrival counts
+	// 0 stays zero), the mask and the arrival counts
 	uint64_t n_hot = 0, n_heavy = 0, n_chunks = 0;
 	pagerank_sizes(mt, &n_hot, &n_heavy, &n_chunks);
 	const size_t pack = size_t(n_hot) + 1;
-	const size_t zbytes = 8 * sizeof(unsigned long long) + (2 * pack + mask_words + size_t(n) + n_heavy) * sizeof(uint32_t);
+	const size_t zbytes = 8 * sizeof(unsigned long long) + (2 * pack + mask_words + n_heavy) * sizeof(uint32_t);
 	P_TRY(alloc(reinterpret_cast<void **>(&state), zbytes));
 	P_TRY(alloc(reinterpret_cast<void **>(&chunk_heavy), n_chunks * sizeof(uint32_t)));
 	xh0 = reinterpret_cast<float *>(state + 8);
 	xh1 = xh0 + pack;
 	mask = reinterpret_cast<uint32_t *>(xh1 + pack);
-	slot = mask + mask_words;
-	arrived = slot + n;
+	arrived = mask + mask_words;
 	if (pagerank_needs_out(mt)) P_TRY(alloc(reinterpret_cast<void **>(&out), size_t(n) * sizeof(float)));
 	// the loop state comes back through pinned words per host thread, one set
 	// per batch in flight
@@ -147,7 +146,6 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	pr_epi e{};
 	e.deg = deg;
 	e.heavy_mask = mask;
-	e.slot = slot;
 	e.chunk_heavy = chunk_heavy;
 	e.arrived = arrived;
 	e.pr = pr;
@@ -159,8 +157,8 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	e.n = uint64_t(n);
 	e.max_iters = max_iters;
 	PCUDA_TRY(cudaMemsetAsync(state, 0, zbytes, st));
-	P_TRY(pagerank_maps(mt, mask, slot, chunk_heavy, &e.heavy, st));
-	init_kernel<<<gb, kThreads, 0, st>>>(deg, pr, in0, pr1, slot, xh0, n, p0);
+	P_TRY(pagerank_maps(mt, mask, chunk_heavy, &e.slot, &e.heavy, st));
+	init_kernel<<<gb, kThreads, 0, st>>>(deg, pr, in0, pr1, e.slot, xh0, n, p0);
 	PCUDA_TRY(cudaGetLastError());
 	struct events {
 		cudaEvent_t e[2] = {nullptr, nullptr};

@@ -81,6 +81,7 @@ struct gpu_part {
 	uint32_t *col = nullptr;
 	void *val = nullptr;
 	int32_t *hot_col = nullptr;
+	uint32_t *slot = nullptr;            // a column's hot slot (ncols; 0: none)
 	uint32_t n_hot = 0;
 	void *xhot = nullptr;                // (n_hot + 1) * kPanelBytes
 	uint32_t n_exact = 0;                // rows summed in the reference's order
@@ -130,7 +131,7 @@ struct gpu_part {
 		int cur = 0;
 		cudaGetDevice(&cur);
 		cudaSetDevice(device);
-		void *ps[] = {col, val, hot_col, xhot, ranges, fine, heavy, partial, stage_x, stage_y, slot_col[0], slot_col[1],
+		void *ps[] = {col, val, hot_col, slot, xhot, ranges, fine, heavy, partial, stage_x, stage_y, slot_col[0], slot_col[1],
 				slot_val[0], slot_val[1]};
 		for (void *p : ps)
 			if (p) cudaFree(p);

@@ -6,7 +6,7 @@
 //
 //   1. in-degrees (atomic counts), hot columns = the stable radix sort of
 //      the columns of in-degree >= 2 by min(indeg, 2^16) descending, ties in
-//      column order; slot_of[c] = 1 + its rank below kHotMax, else -1
+//      column order; slot_of[c] = 1 + its rank below kHotMax, else 0
 //   2. per row: len = seg_row_len(d), chunk count, heavy flag; exclusive
 //      scans give the lens before each row (L), the first chunk of each
 //      heavy row and its heavy index
@@ -77,9 +77,9 @@ __global__ void hot_keys_kernel(const uint32_t *indeg, uint64_t ncols, uint32_t 
 	if ((threadIdx.x & 31) == 0 && c_local) atomicAdd(ncand, c_local);
 }
 
-__global__ void slot_kernel(const uint32_t *hot, uint32_t nhot, int32_t *slot_of)
+__global__ void slot_kernel(const uint32_t *hot, uint32_t nhot, uint32_t *slot_of)
 {
-	GRID_STRIDE(s, nhot) slot_of[hot[s]] = int32_t(s + 1);
+	GRID_STRIDE(s, nhot) slot_of[hot[s]] = uint32_t(s + 1);
 }
 
 // rows [0, n): len, chunk count, heavy flag; index n holds zeros (the scans
@@ -221,18 +221,18 @@ __device__ __forceinline__ void copy_val(char *dst, const char *src, size_t es)
 // entries [b, e) of row r at stream offset `at`: hot slot or column id, the
 // row-end bit on the row's last entry when `close`; returns the hot count
 __device__ __forceinline__ uint32_t put_entries(const int32_t *col, const char *val, size_t es, uint32_t rb,
-		uint32_t b, uint32_t e, uint64_t at, bool close, const int32_t *slot_of, uint32_t *out, char *oval,
+		uint32_t b, uint32_t e, uint64_t at, bool close, const uint32_t *slot_of, uint32_t *out, char *oval,
 		int lane)
 {
 	uint32_t h = 0;
 	for (uint32_t i = b + lane; i < e; i += 32) {
 		const uint32_t c = uint32_t(col[rb + i]);
-		const int32_t sl = slot_of[c];
-		uint32_t v = sl >= 0 ? (uint32_t(sl) | kHot) : c;
+		const uint32_t sl = slot_of[c];
+		uint32_t v = sl ? (sl | kHot) : c;
 		if (close && i + 1 == e) v |= kEnd;
 		out[at + (i - b)] = v;
 		if (es) copy_val(oval + (at + (i - b)) * es, val + size_t(rb + i) * es, es);
-		h += sl >= 0;
+		h += sl != 0;
 	}
 	return h;
 }
@@ -240,7 +240,7 @@ __device__ __forceinline__ uint32_t put_entries(const int32_t *col, const char *
 // a warp per row: the row's place in its run, then its chunks
 __global__ void scatter_kernel(const uint32_t *row_ptr, const int32_t *col, const char *val, size_t es, uint64_t n,
 		const uint64_t *L, const uint32_t *start, const uint32_t *sidx, const uint64_t *seg_L0, const uint64_t *at,
-		const uint32_t *chunks, const uint32_t *cfirst, uint32_t s_run, const int32_t *slot_of, uint32_t *out,
+		const uint32_t *chunks, const uint32_t *cfirst, uint32_t s_run, const uint32_t *slot_of, uint32_t *out,
 		char *oval, unsigned long long *hot_entries)
 {
 	const int lane = threadIdx.x & 31;
@@ -381,11 +381,11 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 
 	// 1. hot columns
 	uint32_t *indeg, *hk0, *hk1, *hv0, *hv1;
-	int32_t *slot_of;
 	TRY(t.get(&indeg, nc)); TRY(t.get(&hk0, nc)); TRY(t.get(&hk1, nc)); TRY(t.get(&hv0, nc)); TRY(t.get(&hv1, nc));
-	TRY(t.get(&slot_of, nc));
+	TRY(dalloc(&p->slot, nc, p->bytes));
+	uint32_t *slot_of = p->slot;
 	SCUDA_TRY(cudaMemsetAsync(indeg, 0, std::max<uint64_t>(nc, 1) * sizeof(uint32_t), st));
-	SCUDA_TRY(cudaMemsetAsync(slot_of, 0xFF, std::max<uint64_t>(nc, 1) * sizeof(int32_t), st));
+	if (nc) SCUDA_TRY(cudaMemsetAsync(slot_of, 0, nc * sizeof(uint32_t), st));
 	if (nnz) indeg_kernel<<<grid(nnz), kT, 0, st>>>(csr.col, nnz, indeg);
 	if (nc) hot_keys_kernel<<<grid(nc), kT, 0, st>>>(indeg, nc, hk0, hv0, cnt + 0);
 	SCUDA_TRY(cudaGetLastError());

@@ -1116,7 +1116,7 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 		for (uint64_t i = b; i < e; i++) indeg[csr.col[i]].fetch_add(1, std::memory_order_relaxed);
 	});
 	std::vector<int32_t> hot_col;
-	std::vector<int32_t> slot_of(csr.ncols, -1);
+	std::vector<uint32_t> slot_of(csr.ncols, 0);
 	{
 		// counting sort of the columns by in-degree, descending, capped
 		const uint32_t cap = 1u << 16;
@@ -1134,7 +1134,7 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 		}
 		hot_col.assign(order.begin(), order.begin() + nhot);
 		// slot 0 is the zero row; hot columns take slots 1..nhot
-		for (uint64_t s = 0; s < nhot; s++) slot_of[hot_col[s]] = int32_t(s + 1);
+		for (uint64_t s = 0; s < nhot; s++) slot_of[hot_col[s]] = uint32_t(s + 1);
 	}
 
 	// Work segments: runs of consecutive rows (every row in order; an exact
@@ -1239,9 +1239,9 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 		uint64_t h = 0;
 		for (uint32_t i = b; i < e; i++) {
 			const uint32_t c = uint32_t(csr.col[rb + i]);
-			const int32_t sl = slot_of[c];
-			col[at + (i - b)] = sl >= 0 ? (uint32_t(sl) | kHot) : c;
-			h += sl >= 0;
+			const uint32_t sl = slot_of[c];
+			col[at + (i - b)] = sl ? (sl | kHot) : c;
+			h += sl != 0;
 		}
 		if (es) memcpy(&val[at * es], &csr.val[size_t(rb + b) * es], size_t(e - b) * es);
 		return h;
@@ -1283,6 +1283,7 @@ static int make_part(const host_csr &csr, int device, std::shared_ptr<gpu_part> 
 		}
 	}
 	if (!rc) rc = upload(&p->hot_col, hot_col.data(), hot_col.size(), bytes);
+	if (!rc) rc = upload(&p->slot, slot_of.data(), slot_of.size(), bytes);
 	if (!rc) rc = upload(&p->ranges, ranges.data(), ranges.size(), bytes);
 	if (!rc) rc = upload(&p->fine, fine.data(), fine.size(), bytes);
 	// longest first (the fixup gives each long row a warp and packs the short
@@ -1495,7 +1496,8 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 
 template <class XT, class YT, class A, class WT>
 static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int64_t ldy, int64_t k,
-		const void *sin, const void *sout, cudaStream_t st, void *xhot = nullptr, void *partial = nullptr)
+		const void *sin, const void *sout, cudaStream_t st, void *xhot = nullptr, void *partial = nullptr,
+		bool packed = false)
 {
 	if (!xhot) xhot = p.xhot;
 	if (!partial) partial = p.partial;
@@ -1521,9 +1523,10 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 		a.n_ranges = p.fine ? p.n_fine : p.n_ranges;
 		a.G = kp / vn;
 		a.R = 32 / a.G;
-		if (int rc = launch_pack<XT, A>(p, static_cast<const XT *>(a.X), ldx, kp, static_cast<XT *>(xhot), kp,
-				static_cast<const A *>(sin), st))
-			return rc;
+		if (!packed)
+			if (int rc = launch_pack<XT, A>(p, static_cast<const XT *>(a.X), ldx, kp, static_cast<XT *>(xhot), kp,
+					static_cast<const A *>(sin), st))
+				return rc;
 		if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
 				switch (vn) {
 				case 1: return launch_lanes_scaled<XT, YT, A, WT, 1>(p, sa, st);
@@ -1544,21 +1547,21 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 
 template <class XT, class YT, class A>
 static int run_w(const gpu_part &p, const void *X, int64_t ldx, void *Y, int64_t ldy, int64_t k,
-		const void *sin, const void *sout, cudaStream_t st)
+		const void *sin, const void *sout, cudaStream_t st, bool packed)
 {
 	switch (p.prim) {
-	case FMX_P_BOOL: return run_typed<XT, YT, A, void>(p, X, ldx, Y, ldy, k, sin, sout, st);
+	case FMX_P_BOOL: return run_typed<XT, YT, A, void>(p, X, ldx, Y, ldy, k, sin, sout, st, nullptr, nullptr, packed);
 	case FMX_P_FLOAT:
-		if constexpr (std::is_floating_point<A>::value) return run_typed<XT, YT, A, float>(p, X, ldx, Y, ldy, k, sin, sout, st);
+		if constexpr (std::is_floating_point<A>::value) return run_typed<XT, YT, A, float>(p, X, ldx, Y, ldy, k, sin, sout, st, nullptr, nullptr, packed);
 		break;
 	case FMX_P_DOUBLE:
-		if constexpr (std::is_same<A, double>::value) return run_typed<XT, YT, A, double>(p, X, ldx, Y, ldy, k, sin, sout, st);
+		if constexpr (std::is_same<A, double>::value) return run_typed<XT, YT, A, double>(p, X, ldx, Y, ldy, k, sin, sout, st, nullptr, nullptr, packed);
 		break;
 	case FMX_P_INTEGER:
-		if constexpr (std::is_integral<A>::value) return run_typed<XT, YT, A, int32_t>(p, X, ldx, Y, ldy, k, sin, sout, st);
+		if constexpr (std::is_integral<A>::value) return run_typed<XT, YT, A, int32_t>(p, X, ldx, Y, ldy, k, sin, sout, st, nullptr, nullptr, packed);
 		break;
 	case FMX_P_LONG:
-		if constexpr (std::is_same<A, int64_t>::value) return run_typed<XT, YT, A, int64_t>(p, X, ldx, Y, ldy, k, sin, sout, st);
+		if constexpr (std::is_same<A, int64_t>::value) return run_typed<XT, YT, A, int64_t>(p, X, ldx, Y, ldy, k, sin, sout, st, nullptr, nullptr, packed);
 		break;
 	}
 	return set_error(FMX_ERR_TYPE, "matrix entry type %d does not match the dense type "
@@ -1567,7 +1570,7 @@ static int run_w(const gpu_part &p, const void *X, int64_t ldx, void *Y, int64_t
 }
 
 int spmm_part(const gpu_part &p, int xt, const void *X, int64_t ldx, int yt, void *Y, int64_t ldy,
-		int64_t k, const void *sin, const void *sout, cudaStream_t st)
+		int64_t k, const void *sin, const void *sout, cudaStream_t st, bool packed = false)
 {
 	if (k <= 0) return set_error(FMX_ERR_DIM, "k must be positive (got %lld)", (long long)k);
 	if (!X || !Y) return set_error(FMX_ERR_INVAL, "null X or Y");
@@ -1577,20 +1580,31 @@ int spmm_part(const gpu_part &p, int xt, const void *X, int64_t ldx, int yt, voi
 	cudaGetDevice(&cur);
 	if (cur != p.device) CUDA_TRY(cudaSetDevice(p.device));
 	int rc;
-	if (xt == FMX_F32 && yt == FMX_F32) rc = run_w<float, float, float>(p, X, ldx, Y, ldy, k, sin, sout, st);
-	else if (xt == FMX_F64 && yt == FMX_F64) rc = run_w<double, double, double>(p, X, ldx, Y, ldy, k, sin, sout, st);
-	else if (xt == FMX_BF16 && yt == FMX_F32) rc = run_w<__nv_bfloat16, float, float>(p, X, ldx, Y, ldy, k, sin, sout, st);
-	else if (xt == FMX_BF16 && yt == FMX_BF16) rc = run_w<__nv_bfloat16, __nv_bfloat16, float>(p, X, ldx, Y, ldy, k, sin, sout, st);
+	if (xt == FMX_F32 && yt == FMX_F32) rc = run_w<float, float, float>(p, X, ldx, Y, ldy, k, sin, sout, st, packed);
+	else if (xt == FMX_F64 && yt == FMX_F64) rc = run_w<double, double, double>(p, X, ldx, Y, ldy, k, sin, sout, st, packed);
+	else if (xt == FMX_BF16 && yt == FMX_F32) rc = run_w<__nv_bfloat16, float, float>(p, X, ldx, Y, ldy, k, sin, sout, st, packed);
+	else if (xt == FMX_BF16 && yt == FMX_BF16) rc = run_w<__nv_bfloat16, __nv_bfloat16, float>(p, X, ldx, Y, ldy, k, sin, sout, st, packed);
 	else if (xt == FMX_I32 && yt == FMX_I32) {
 		rc = (sin || sout) ? set_error(FMX_ERR_UNSUPPORTED, "row scales need a floating-point type")
-				: run_w<int32_t, int32_t, int32_t>(p, X, ldx, Y, ldy, k, nullptr, nullptr, st);
+				: run_w<int32_t, int32_t, int32_t>(p, X, ldx, Y, ldy, k, nullptr, nullptr, st, packed);
 	} else if (xt == FMX_I64 && yt == FMX_I64) {
 		rc = (sin || sout) ? set_error(FMX_ERR_UNSUPPORTED, "row scales need a floating-point type")
-				: run_w<int64_t, int64_t, int64_t>(p, X, ldx, Y, ldy, k, nullptr, nullptr, st);
+				: run_w<int64_t, int64_t, int64_t>(p, X, ldx, Y, ldy, k, nullptr, nullptr, st, packed);
 	} else rc = set_error(FMX_ERR_TYPE, "unsupported type pair x=%d y=%d "
 			"(input and output matrices need the same type, sparse_matrix.cpp:754-758)", xt, yt);
 	if (cur != p.device) cudaSetDevice(cur);
 	return rc;
+}
+
+hot_pack_target pack_target(const fmx_matrix *m)
+{
+	return {m->a->slot, m->a->xhot, kPanelBytes};
+}
+
+int spmm_packed(const fmx_matrix *m, int xt, const void *X, int64_t ldx, int yt, void *Y, int64_t ldy, int64_t k,
+		const void *sin, const void *sout, cudaStream_t st)
+{
+	return spmm_part(*m->a, xt, X, ldx, yt, Y, ldy, k, sin, sout, st, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -1613,11 +1627,6 @@ __global__ void chunk_heavy_kernel(const heavy_row *heavy, uint32_t n_heavy, uin
 		for (uint32_t c = 0; c < heavy[i].count; c++) chunk_heavy[heavy[i].first + c] = i;
 }
 
-__global__ void hot_slot_kernel(const int32_t *hot_col, uint32_t n_hot, uint32_t *slot)
-{
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_hot; i += gridDim.x * blockDim.x) slot[hot_col[i]] = i + 1;
-}
-
 __global__ void heavy_mask_kernel(const heavy_row *heavy, uint32_t n_heavy, uint32_t *mask)
 {
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_heavy; i += gridDim.x * blockDim.x) {
@@ -1626,17 +1635,16 @@ __global__ void heavy_mask_kernel(const heavy_row *heavy, uint32_t n_heavy, uint
 	}
 }
 
-int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *slot, uint32_t *chunk_heavy, const void **heavy,
+int pagerank_maps(const fmx_matrix *mt, uint32_t *mask, uint32_t *chunk_heavy, const uint32_t **slot, const void **heavy,
 		cudaStream_t st)
 {
 	const gpu_part &p = *mt->a;
 	*heavy = p.heavy;
+	*slot = p.slot;
 	auto grid = [](uint32_t n) { return unsigned(std::min<uint32_t>((n + 255) / 256, 1024)); };
 	if (p.n_heavy) heavy_mask_kernel<<<grid(p.n_heavy), 256, 0, st>>>(p.heavy, p.n_heavy, mask);
 	CUDA_TRY(cudaGetLastError());
 	if (p.n_heavy) chunk_heavy_kernel<<<grid(p.n_heavy), 256, 0, st>>>(p.heavy, p.n_heavy, chunk_heavy);
-	CUDA_TRY(cudaGetLastError());
-	if (p.n_hot) hot_slot_kernel<<<grid(p.n_hot), 256, 0, st>>>(p.hot_col, p.n_hot, slot);
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
 }

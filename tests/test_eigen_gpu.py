@@ -53,6 +53,27 @@ def _sin_angle(X, U):
 
 
 @pytest.mark.parametrize("precision", ["plain", "mixed"])
+@pytest.mark.parametrize("block", [3, 16, 17, 20, 31, 32, 33, 48, 63, 64])
+def test_block_widths(torch_cuda, precision, block):
+    """Blocks of one and of several SpMM panels, whole and odd: the filter
+    steps leave the next product's hot rows in the former only."""
+    n = 4000
+    src, dst, _ = sbm_edges(n, 2, 20.0, 20.0, seed=block)
+    N, _, _ = _na(n, src, dst)
+    opts = eigen_options()
+    opts.init(2)
+    opts.block_size = block
+    opts.which = "LA"
+    opts.tol = TOL
+    opts.precision = precision
+    res = compute_eigen(NA_operator(_matrix(n, src, dst)), True, opts)
+    assert res.status.converged == 2
+    assert _residuals(N, res.vals, res.vecs.double().cpu().numpy()).max() <= 2 * TOL
+    ref = eigsh(N, k=2, which="LA", return_eigenvectors=False)
+    np.testing.assert_allclose(np.sort(res.vals), np.sort(ref), atol=1e-6)
+
+
+@pytest.mark.parametrize("precision", ["plain", "mixed"])
 @pytest.mark.parametrize("n,B,ratio", [(6000, 4, 20.0), (12000, 8, 30.0)])
 def test_sbm_top_blocks(torch_cuda, precision, n, B, ratio):
     src, dst, _ = sbm_edges(n, B, 20.0, ratio, seed=n + B)
