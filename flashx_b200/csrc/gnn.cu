@@ -276,22 +276,46 @@ __global__ void __launch_bounds__(kThreads) loss_kernel(const double *__restrict
 	}
 }
 
-// dY = U P1 + Y P2 (FP32): a thread per (row, output column)
+// dY = U P1 + Y P2 (FP32): a thread per row, four output columns at a time;
+// each output adds U's terms, then Y's, in column order.  (A thread per row and
+// column read every operand with 4-byte loads: 12.6 us at n = 100k.)
 __global__ void __launch_bounds__(kThreads) dy_kernel(const float *__restrict__ U, int64_t ldu, int nev,
 		const float *__restrict__ Y, const float *__restrict__ P1, const float *__restrict__ P2, int64_t n,
 		float *__restrict__ dY)
 {
-	__shared__ float s1[kMaxNev * kOut], s2[kOut * kOut];
-	for (int i = threadIdx.x; i < nev * kOut; i += kThreads) s1[i] = P1[i];
-	for (int i = threadIdx.x; i < kOut * kOut; i += kThreads) s2[i] = P2[i];
+	__shared__ float4 s1[kMaxNev][kOut / 4], s2[kOut][kOut / 4];
+	for (int i = threadIdx.x; i < nev * (kOut / 4); i += kThreads) s1[i / (kOut / 4)][i % (kOut / 4)] = reinterpret_cast<const float4 *>(P1)[i];
+	for (int i = threadIdx.x; i < kOut * (kOut / 4); i += kThreads) s2[i / (kOut / 4)][i % (kOut / 4)] = reinterpret_cast<const float4 *>(P2)[i];
 	__syncthreads();
-	const int j = threadIdx.x % kOut;
-	for (int64_t row = int64_t(blockIdx.x) * (kThreads / kOut) + threadIdx.x / kOut; row < n;
-			row += int64_t(gridDim.x) * (kThreads / kOut)) {
-		float s = 0.f;
-		for (int k = 0; k < nev; k++) s = fmaf(U[row * ldu + k], s1[k * kOut + j], s);
-		for (int k = 0; k < kOut; k++) s = fmaf(Y[row * kOut + k], s2[k * kOut + j], s);
-		dY[row * kOut + j] = s;
+	for (int64_t row = int64_t(blockIdx.x) * kThreads + threadIdx.x; row < n; row += int64_t(gridDim.x) * kThreads) {
+		float y[kOut];
+#pragma unroll
+		for (int v = 0; v < kOut / 4; v++) {
+			const float4 t = reinterpret_cast<const float4 *>(Y + row * kOut)[v];
+			y[4 * v] = t.x; y[4 * v + 1] = t.y; y[4 * v + 2] = t.z; y[4 * v + 3] = t.w;
+		}
+		float4 o[kOut / 4];
+#pragma unroll
+		for (int v = 0; v < kOut / 4; v++) o[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+		auto term = [&](float x, const float4 (&p)[kOut / 4]) {
+#pragma unroll
+			for (int v = 0; v < kOut / 4; v++) {
+				o[v].x = fmaf(x, p[v].x, o[v].x); o[v].y = fmaf(x, p[v].y, o[v].y);
+				o[v].z = fmaf(x, p[v].z, o[v].z); o[v].w = fmaf(x, p[v].w, o[v].w);
+			}
+		};
+		const float *u = U + row * ldu;
+		int k = 0;
+		for (; k + 4 <= nev; k += 4) {
+			const float t[4] = {u[k], u[k + 1], u[k + 2], u[k + 3]};
+#pragma unroll
+			for (int z = 0; z < 4; z++) term(t[z], s1[k + z]);
+		}
+		for (; k < nev; k++) term(u[k], s1[k]);
+#pragma unroll
+		for (int q = 0; q < kOut; q++) term(y[q], s2[q]);
+#pragma unroll
+		for (int v = 0; v < kOut / 4; v++) reinterpret_cast<float4 *>(dY + row * kOut)[v] = o[v];
 	}
 }
 
@@ -389,12 +413,29 @@ int forward(const fmx_gnn *g, const fmx_matrix *m, const float *scale, const flo
 	return FMX_OK;
 }
 
+// What a call brings back to the host: pinned, one per host thread, so that
+// its copies share one wait (each copy into pageable memory is a wait of its
+// own).
+struct host_out {
+	float grad[kParams];
+	double loss;
+	int err;
+};
+int host_results(host_out **out)
+{
+	static thread_local host_out *pinned = nullptr;
+	if (!pinned) GCUDA_TRY(cudaMallocHost(&pinned, sizeof(host_out)));
+	*out = pinned;
+	return FMX_OK;
+}
+
 int read_err(const fmx_gnn *g, cudaStream_t st)
 {
-	int e = 0;
-	GCUDA_TRY(cudaMemcpyAsync(&e, g->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+	host_out *h = nullptr;
+	G_TRY(host_results(&h));
+	GCUDA_TRY(cudaMemcpyAsync(&h->err, g->err, sizeof(int), cudaMemcpyDeviceToHost, st));
 	GCUDA_TRY(cudaStreamSynchronize(st));
-	if (e) return set_error(FMX_ERR_CUDA, "a tensor-core wait ran out of time");
+	if (h->err) return set_error(FMX_ERR_CUDA, "a tensor-core wait ran out of time");
 	return FMX_OK;
 }
 
@@ -548,7 +589,7 @@ int fmx_gnn_loss_grad(fmx_gnn *g, const fmx_matrix *m, const float *scale, const
 	G_TRY(fmx_dense_gram(FMX_DENSE_F64, U, ldu, nev, Y, kOut, kOut, n, dpart, M, nullptr, st));
 	loss_kernel<<<1, kThreads, 0, st>>>(G, M, nev, P1, P2, dloss);
 	GCUDA_TRY(cudaGetLastError());
-	dy_kernel<<<grid_for(n * kOut), kThreads, 0, st>>>(U, ldu, nev, Y, P1, P2, n, dY);
+	dy_kernel<<<grid_for(n), kThreads, 0, st>>>(U, ldu, nev, Y, P1, P2, n, dY);
 	GCUDA_TRY(cudaGetLastError());
 	// layer 2: Y = A_s Z2, Z2 = H W2
 	G_TRY(fmx_spmm(m, FMX_F32, dY, kOut, FMX_F32, dZ2, kOut, kOut, scale, scale, st));
@@ -562,9 +603,14 @@ int fmx_gnn_loss_grad(fmx_gnn *g, const fmx_matrix *m, const float *scale, const
 	sum_parts_kernel<<<(kH + 7) / 8, 1024, 0, st>>>(bpart, rparts, kH, g->g + kOffB1);
 	GCUDA_TRY(cudaGetLastError());
 	G_TRY(fmx_dense_gram(precision, Z, kZ, kZ, dH, kH, kH, n, gpart, g->g + kOffW1, g->err, st));
-	if (loss) GCUDA_TRY(cudaMemcpyAsync(loss, dloss, sizeof(double), cudaMemcpyDeviceToHost, st));
-	if (grad_host) GCUDA_TRY(cudaMemcpyAsync(grad_host, g->g, sizeof(float) * kParams, cudaMemcpyDeviceToHost, st));
-	return read_err(g, st);
+	host_out *h = nullptr;
+	G_TRY(host_results(&h));
+	if (loss) GCUDA_TRY(cudaMemcpyAsync(&h->loss, dloss, sizeof(double), cudaMemcpyDeviceToHost, st));
+	if (grad_host) GCUDA_TRY(cudaMemcpyAsync(h->grad, g->g, sizeof(float) * kParams, cudaMemcpyDeviceToHost, st));
+	G_TRY(read_err(g, st));
+	if (loss) *loss = h->loss;
+	if (grad_host) memcpy(grad_host, h->grad, sizeof(h->grad));
+	return FMX_OK;
 }
 
 int fmx_gnn_adam_step(fmx_gnn *g, float lr, void *stream)

@@ -303,18 +303,24 @@ struct accum {
 
 // The PageRank update at a row close (EPI): rows of the fixup's heavy list
 // are left to the fixup.
-__device__ __forceinline__ void pr_update(const pr_epi &e, int64_t row, float out, unsigned &cnt)
+struct pr_row {
+	float pr1, deg;
+	uint32_t slot;
+};
+__device__ __forceinline__ pr_row pr_load(const pr_epi &e, int64_t row)
+{
+	return {e.pr1[row], e.deg[row], __ldg(e.slot + row)};
+}
+__device__ __forceinline__ void pr_update(const pr_epi &e, int64_t row, const pr_row &o, float out, unsigned &cnt)
 {
 	const float p2 = __fadd_rn(__fmul_rn(out, e.damping), e.teleport);
-	const float diff = fabsf(__fsub_rn(e.pr1[row], p2));
+	const float diff = fabsf(__fsub_rn(o.pr1, p2));
 	cnt += diff < e.eps;
 	e.pr[row] = p2;
-	const float d = e.deg[row];
-	const float x = __fdiv_rn(p2, d);
+	const float x = __fdiv_rn(p2, o.deg);
 	e.in_next[row] = x;
-	const uint32_t s = __ldg(e.slot + row);
-	if (s) e.xhot_next[s] = x;
-	e.pr1[row] = __fmul_rn(x, d);
+	if (o.slot) e.xhot_next[o.slot] = x;
+	e.pr1[row] = __fmul_rn(x, o.deg);
 }
 
 // The loop test (PageRank.cpp:96,124-129) by the last block of an iteration's
@@ -667,7 +673,7 @@ __device__ __forceinline__ void pr_chunk(const pr_epi &e, float *partial, uint32
 	}
 	if (lane == 0) {
 		e.arrived[h] = 0;
-		pr_update(e, hr.row, v, cnt);
+		pr_update(e, hr.row, pr_load(e, hr.row), v, cnt);
 	}
 }
 
@@ -742,12 +748,27 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 		}
 		if (runs) {
 			for (int q = lane; q < nrow; q += 32) {
-				const int b0 = q ? int(send[wib][q - 1]) + 1 : 0, b1 = send[wib][q];
-				T acc = T(0);
-				for (int i = b0; i <= b1; i++) acc = acc_add(acc, sval[wib][i]);
+				const int b0 = q ? int(send[wib][q - 1]) + 1 : 0, b1 = send[wib][q] + 1;
 				const uint32_t row = rg.row0 + uint32_t(q);
+				// the row's old values load while it is summed
+				pr_row old{};
+				uint32_t heavy = 0;
 				if constexpr (EPI) {
-					if (!((__ldg(e.heavy_mask + (row >> 5)) >> (row & 31)) & 1u)) pr_update(e, int64_t(row), acc, cnt);
+					old = pr_load(e, int64_t(row));
+					heavy = (__ldg(e.heavy_mask + (row >> 5)) >> (row & 31)) & 1u;
+				}
+				T acc = T(0);
+				int i = b0;
+				for (; i + 8 <= b1; i += 8) {         // 8 shared-memory reads in flight
+					T v[8];
+#pragma unroll
+					for (int z = 0; z < 8; z++) v[z] = sval[wib][i + z];
+#pragma unroll
+					for (int z = 0; z < 8; z++) acc = acc_add(acc, v[z]);
+				}
+				for (; i < b1; i++) acc = acc_add(acc, sval[wib][i]);
+				if constexpr (EPI) {
+					if (!heavy) pr_update(e, int64_t(row), old, acc, cnt);
 				} else {
 					static_cast<T *>(a.Y)[int64_t(row) * a.ldy] = acc;
 				}
@@ -781,7 +802,7 @@ __global__ void __launch_bounds__(kThreads) pr_apply_kernel(const float *__restr
 	if (e.state[1]) return;
 	unsigned cnt = 0;
 	for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads)
-		pr_update(e, i, out[i], cnt);
+		pr_update(e, i, pr_load(e, i), out[i], cnt);
 	cnt = __reduce_add_sync(0xffffffffu, cnt);
 	if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(e.state, (unsigned long long)cnt);
 	pr_finish(e);

@@ -389,6 +389,31 @@ def test_repeated_calls_varying_k(torch_cuda):
             assert np.array_equal(_gpu_spmm(torch, m, X), oracle.spmm(idx, mat, X))
 
 
+@pytest.mark.parametrize("n,k,dtype", [(3000, 16, "float32"), (3000, 1, "float32"), (3000, 7, "float64"),
+                                       (200000, 16, "float32"), (200000, 1, "float32")])
+def test_graph_capture(torch_cuda, n, k, dtype):
+    """A product captured in a CUDA graph (its kernels are dependent launches
+    where they are short) replays on new operands with the eager results."""
+    torch = torch_cuda
+    src, dst = _graph(n, 12 * n, 51, ((7, 1500), (9, 600)))
+    m = sparse_matrix.create(matrix_image.build(src, dst, None, nrows=n, ncols=n, dedup=True), None)
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn((n, k), generator=g, device="cuda", dtype=getattr(torch, dtype))
+    y = torch.empty_like(x)
+    assert m.multiply(x, y)                       # the kernels' first use: outside the capture
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert m.multiply(x, y)
+        assert m.multiply(y, x)
+    for seed in (1, 2):
+        x0 = torch.randn(x.shape, generator=g, device="cuda", dtype=x.dtype)
+        x.copy_(x0)
+        graph.replay()
+        torch.cuda.synchronize()
+        y1 = m.multiply(x0)
+        assert torch.equal(y, y1) and torch.equal(x, m.multiply(y1))
+
+
 def test_empty_matrix(torch_cuda):
     """A matrix without edges (every block row stored as one empty tile) gives
     Y = 0, overwriting whatever Y held."""
