@@ -110,19 +110,13 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
 	return r;
 }
 
-// Streaming (read-once) loads and stores: evict-first in L1 and L2 so that
-// the gathered X rows keep the caches.
-__device__ __forceinline__ float ld_stream(const float *p) { return __ldcs(p); }
-__device__ __forceinline__ double ld_stream(const double *p) { return __ldcs(p); }
-__device__ __forceinline__ int32_t ld_stream(const int32_t *p) { return __ldcs(p); }
-__device__ __forceinline__ int64_t ld_stream(const int64_t *p) { return (int64_t)__ldcs((const long long *)p); }
-
 // VEC elements of T: one 16-byte vector, or a scalar (VEC == 1).
 template <class T, int VEC>
 struct xvec {
 	T v[VEC];
 };
 
+// Streaming stores (evict-first), so that the gathered rows keep the caches.
 template <class T, int VEC>
 __device__ __forceinline__ void st_y(T *p, const T (&v)[VEC])
 {
@@ -145,58 +139,16 @@ __device__ __forceinline__ void st_y(T *p, const T (&v)[VEC])
 	}
 }
 
-// L2 eviction priorities for the gathers (createpolicy, PTX ISA 7.4+).
-__device__ __forceinline__ uint64_t policy_evict_last()
-{
-	uint64_t p;
-	asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-	return p;
-}
-__device__ __forceinline__ uint64_t policy_evict_first()
-{
-	uint64_t p;
-	asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-	return p;
-}
-
-// Read-only gather of VEC elements of T (16 bytes, or one scalar) with an L2
-// eviction-priority hint.
-template <class T, int VEC>
-__device__ __forceinline__ xvec<T, VEC> ld_x_hint(const T *p, uint64_t pol)
-{
-	xvec<T, VEC> r;
-	if constexpr (VEC * sizeof(T) == 16) {
-		uint32_t a, b, c, d;
-		asm volatile("ld.global.nc.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
-				: "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "l"(p), "l"(pol));
-		uint4 u = make_uint4(a, b, c, d);
-		memcpy(&r, &u, 16);
-	} else if constexpr (sizeof(T) == 8) {
-		static_assert(VEC == 1, "scalar path");
-		uint64_t a;
-		asm volatile("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(a) : "l"(p), "l"(pol));
-		memcpy(&r, &a, 8);
-	} else if constexpr (sizeof(T) == 4) {
-		static_assert(VEC == 1, "scalar path");
-		uint32_t a;
-		asm volatile("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(a) : "l"(p), "l"(pol));
-		memcpy(&r, &a, 4);
-	} else {
-		static_assert(VEC == 1 && sizeof(T) == 2, "scalar path");
-		unsigned short a;
-		asm volatile("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(a) : "l"(p), "l"(pol));
-		memcpy(&r, &a, 2);
-	}
-	return r;
-}
-
 // Programmatic dependent launch.  A call's kernels are launched with the
 // attribute, so that the next one's blocks come in while the last one's drain;
 // dep_wait() holds them until the kernel before has completed.  Every kernel of
 // such a chain waits, and lets its successor in only then: when one starts,
 // everything before its predecessor is complete, and the read-only loads see no
 // line from before it.  The first kernel of a call carries no attribute and
-// follows all earlier work of the stream as usual.
+// follows all earlier work of the stream as usual.  What a kernel of the chain
+// writes is read by plain loads only: ld.global.nc asks for data that nobody
+// writes while the kernel is resident, and the compiler may move an __ldg, or
+// a load through a const __restrict__ pointer, above the wait.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -369,31 +321,34 @@ __device__ __forceinline__ void ld32_nc(const void *p, uint32_t (&r)[8])
 }
 
 // VN elements of T in one load (2 to 32 bytes).  Volatile: a step's loads
-// stay where they are written, all before the adds.
+// stay where they are written, all before the adds.  Not .nc: the kernel
+// before may have written the rows while this one was already resident.
 template <class T, int VN>
 __device__ __forceinline__ xvec<T, VN> ld_n(const char *p)
 {
 	xvec<T, VN> r;
 	if constexpr (VN * sizeof(T) == 32) {
 		uint32_t v[8];
-		ld32_nc(p, v);
+		asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+				: "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+				: "l"(p));
 		memcpy(&r, v, 32);
 	} else if constexpr (VN * sizeof(T) == 16) {
 		uint32_t v[4];
-		asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
+		asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
 		memcpy(&r, v, 16);
 	} else if constexpr (VN * sizeof(T) == 8) {
 		uint32_t v[2];
-		asm volatile("ld.global.nc.v2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
+		asm volatile("ld.global.v2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
 		memcpy(&r, v, 8);
 	} else if constexpr (VN * sizeof(T) == 4) {
 		uint32_t v;
-		asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+		asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
 		memcpy(&r, &v, 4);
 	} else {
 		static_assert(VN == 1 && sizeof(T) == 2, "one 2-byte element");
 		unsigned short v;
-		asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+		asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
 		memcpy(&r, &v, 2);
 	}
 	return r;
@@ -690,7 +645,6 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 	const uint32_t nw = (gridDim.x * kThreads) >> 5;
 	const T *X = static_cast<const T *>(a.X);
 	const T *H = static_cast<const T *>(a.xhot);
-	const uint64_t pol_hot = policy_evict_last(), pol_cold = policy_evict_first();
 	unsigned cnt = 0;
 	// the matrix does not change: the first range's ids load while the kernel
 	// before this one still runs
@@ -720,8 +674,7 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			if (i < rg.len) {
 				const uint32_t c = raw[j] & kIdxMask;
 				const bool hot = raw[j] & kHot;
-				t[j] = ld_x_hint<T, 1>((hot ? H : X) + int64_t(c) * (hot ? int64_t(1) : a.ldx),
-						hot ? pol_hot : pol_cold).v[0];
+				t[j] = ld_n<T, 1>(reinterpret_cast<const char *>((hot ? H : X) + int64_t(c) * (hot ? int64_t(1) : a.ldx))).v[0];
 			}
 		}
 		if constexpr (!kBinary) {
@@ -795,7 +748,7 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 }
 
 // The update of one PageRank iteration over `out` = A^T in.
-__global__ void __launch_bounds__(kThreads) pr_apply_kernel(const float *__restrict__ out, int64_t n, const pr_epi e)
+__global__ void __launch_bounds__(kThreads) pr_apply_kernel(const float *out, int64_t n, const pr_epi e)
 {
 	dep_wait();
 	dep_launch();

@@ -123,3 +123,20 @@ def test_workspace_pool_release(torch_cuda):
     p2, i2 = PageRank(m, 30, 0.85)
     assert i1 == i2 and torch.equal(p1, p2)
     release_cached(0)
+
+
+@pytest.mark.parametrize("n,m", [(6000, 50000), (300000, 2000000)])
+def test_pagerank_repeats_bit_exact(torch_cuda, n, m):
+    """Iterations overlap their neighbours' launches; both forms (a warp per
+    range; the row kernel beyond 64 ranges per SM) must read only finished
+    vectors, every time."""
+    src, dst = _directed(n, m, 12)
+    mat, img, timg = create_2d_matrix(src, dst, None, block_size=(16384, 16384), is_sym=False, nrows=n, ncols=n,
+                                      return_images=True)
+    (idx, im), (tidx, tim) = img.bytes(), timg.bytes()
+    assert np.bincount(dst, minlength=n).max() <= _lib.EXACT_ROW_MAX
+    ref, rit = oracle.pagerank(idx, im, tidx, tim, 12, 0.85, nthreads=4)
+    for _ in range(20):
+        pr, it = PageRank(mat, 12, 0.85)
+        assert it == rit
+        assert np.array_equal(pr.cpu().numpy(), ref)
