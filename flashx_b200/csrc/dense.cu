@@ -16,7 +16,8 @@
 //     For 16-column blocks stored back to back the 3xTF32 forms copy X rows
 //     into place as the hi parts (tc_gemm_x3s, tc_gram_x3s), since the MMA
 //     reads FP32 as TF32 by dropping the low mantissa bits.
-//  gram_f64  G = X^T W in FP64 on the CUDA cores (Cholesky-QR, residuals)
+//  gram_dmma G = X^T W in FP64 on the FP64 MMA path (Cholesky-QR, Rayleigh
+//     quotient)
 //  small FP64 kernels on one CTA: Cholesky factor inverse, Jacobi
 //  eigendecomposition (the projected Rayleigh-Ritz problem).
 //

@@ -24,8 +24,8 @@
 // stall the iteration).
 //
 // Precision modes:
-//   FMX_EIGEN_PLAIN  FP32 SpMM operands; every dense product on CUDA cores
-//                    with FP64 accumulation.
+//   FMX_EIGEN_PLAIN  FP32 SpMM operands; every dense product in FP64 (the FP64
+//                    MMA path; CUDA cores for the updates of b > 32).
 //   FMX_EIGEN_MIXED  the filter runs in correction form, Y = X p(Theta) + E,
 //                    with every filter SpMM on BF16 operands (FP32
 //                    accumulation): their rounding error is relative to the
@@ -873,12 +873,11 @@ struct solver {
 	int rayleigh_ritz(const float *Q)
 	{
 		E_TRY(spmm(FMX_F32, Q, b, W));
-		// The Rayleigh quotient Q^T W stays an FP64 Gram in both modes.  The
-		// 3xTF32 tensor-core Gram is faster at b = 16 (165 against 263 us at
-		// n = 4.2M), but its 7e-5 relative error reaches Theta and through it
-		// the correction form's R = A X - X Theta: at R-MAT scale 22 the mixed
-		// solve then took a fifth filter pass (51 SpMMs, 66 ms, against 42 and
-		// 55 ms).
+		// The Rayleigh quotient Q^T W is an FP64 Gram in both modes: 108 us at
+		// n = 4.2M, b = 16 against the 3xTF32 Gram's 165 us, whose 7e-5 relative
+		// error would also reach Theta and through it the correction form's
+		// R = A X - X Theta (at R-MAT scale 22 the mixed solve then took a fifth
+		// filter pass, 51 SpMMs instead of 42).
 		E_TRY(fmx_dense_gram(FMX_DENSE_F64, Q, b, b, W, b, b, n, gpart, H, nullptr, st));
 		E_TRY(fmx_dense_sym_eig(H, b, wv, V, st));
 		order_kernel<<<1, 1, 0, st>>>(wv, b, o.which == FMX_EIGEN_LM, perm, dsmall->theta);

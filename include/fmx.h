@@ -178,8 +178,9 @@ int fmx_matrix_free(fmx_matrix *m);
 
 /* The solvers (fmx_eigen_solve, fmx_pagerank, the GNN, the device builder)
  * take their device workspace from one memory pool per device that keeps
- * freed memory reserved for the next call.  Hand it back to the driver (as
- * torch.cuda.empty_cache does for torch's cache). */
+ * freed memory reserved for the next call, and fmx_spmm_host copies pageable
+ * buffers through 8 MB of pinned slots per device.  Hand both back to the
+ * driver (as torch.cuda.empty_cache does for torch's cache). */
 int fmx_release_cached(int device);
 
 /* ---- SpMM -----------------------------------------------------------------
@@ -227,7 +228,9 @@ int fmx_spmm_noalloc(const fmx_matrix *m, const float *X, int64_t ldx, float *Y,
                      int64_t ldy, int64_t k, void *stream);
 
 /* Host-buffer SpMM: copies X in and Y out through the device (pinned or
- * pageable host memory), synchronous.  The e2e path a CPU caller uses. */
+ * pageable host memory), synchronous.  The e2e path a CPU caller uses.
+ * Pageable buffers of 1 MB or more are copied by up to 8 host threads of the
+ * call through pinned slots, which one call at a time holds. */
 int fmx_spmm_host(const fmx_matrix *m, int x_type, const void *X_host, int64_t ldx,
                   int y_type, void *Y_host, int64_t ldy, int64_t k);
 
@@ -278,7 +281,7 @@ int fmx_matrix_layout_digest(const fmx_matrix *m, int transpose, uint64_t *diges
  *   FMX_DENSE_BF16    tensor cores (tcgen05), BF16 operands, FP32 accumulate
  *   FMX_DENSE_TF32X3  tensor cores, each operand split x = hi + lo in TF32 and
  *                     hi*hi + hi*lo + lo*hi accumulated in FP32 (FP32 accuracy)
- *   FMX_DENSE_F64     CUDA cores, FP64 accumulate (Gram only)
+ *   FMX_DENSE_F64     FP64 MMA path, FP64 accumulate (Gram only)
  * `err` (device int) is set to 1 if a tensor-core wait ran out of time. */
 #define FMX_DENSE_BF16 0
 #define FMX_DENSE_TF32X3 1
@@ -313,7 +316,7 @@ int fmx_dense_sym_eig(const double *H, int b, double *w, double *V, void *stream
 #define FMX_EIGEN_LM 1      /* largest magnitude ("LM", the reference's default) */
 #define FMX_EIGEN_OP_SCALED 0
 #define FMX_EIGEN_OP_GRAM 1
-#define FMX_EIGEN_PLAIN 0   /* FP32 SpMM operands; dense products in FP64 on CUDA cores */
+#define FMX_EIGEN_PLAIN 0   /* FP32 SpMM operands; dense products in FP64 */
 #define FMX_EIGEN_MIXED 1   /* filter in correction form with BF16 SpMM operands (FP32
                                accumulation), Rayleigh-Ritz SpMM in FP32; CholQR basis
                                update on tensor cores (3xTF32) until tensor_until, FP64
