@@ -815,11 +815,8 @@ struct solver {
 		ECUDA_TRY(cudaMemcpyAsync(eye, I.data(), I.size() * sizeof(double), cudaMemcpyHostToDevice, st));
 		ECUDA_TRY(cudaMemsetAsync(tc_err, 0, sizeof(int), st));
 		ECUDA_TRY(cudaMemsetAsync(info, 0, 4 * sizeof(int), st));
-		// pinned, once per host thread (a page-locked allocation per solve can
-		// stall for a long time in a process that holds much pinned memory)
-		static thread_local small_out *pinned = nullptr;
-		if (!pinned) ECUDA_TRY(cudaMallocHost(&pinned, sizeof(small_out)));
-		hsmall = pinned;
+		static thread_local thread_pinned<small_out> pinned;
+		ECUDA_TRY(pinned.get(&hsmall));
 		return FMX_OK;
 	}
 

@@ -21,6 +21,24 @@ namespace fmx {
 // Sets the thread-local message returned by fmx_last_error() and returns code.
 int set_error(int code, const char *fmt, ...);
 
+// Pinned host memory of one host thread, allocated by its first use and freed
+// when the thread ends (a page-locked allocation per call can stall for a long
+// time in a process that holds much pinned memory).  Declare it thread_local.
+template <class T>
+struct thread_pinned {
+	T *p = nullptr;
+	cudaError_t get(T **out)
+	{
+		const cudaError_t e = p ? cudaSuccess : cudaMallocHost(reinterpret_cast<void **>(&p), sizeof(T));
+		*out = p;
+		return e;
+	}
+	~thread_pinned()
+	{
+		if (p) cudaFreeHost(p);
+	}
+};
+
 // ---- the reference's on-disk 2D format -------------------------------------
 // matrix_header::info (matrix/matrix_header.h:102-121), x86-64 layout,
 // padded to one 4096-byte page.

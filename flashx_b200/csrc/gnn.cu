@@ -423,9 +423,8 @@ struct host_out {
 };
 int host_results(host_out **out)
 {
-	static thread_local host_out *pinned = nullptr;
-	if (!pinned) GCUDA_TRY(cudaMallocHost(&pinned, sizeof(host_out)));
-	*out = pinned;
+	static thread_local thread_pinned<host_out> pinned;
+	GCUDA_TRY(pinned.get(out));
 	return FMX_OK;
 }
 

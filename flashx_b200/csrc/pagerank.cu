@@ -136,8 +136,11 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 	if (pagerank_needs_out(mt)) P_TRY(alloc(reinterpret_cast<void **>(&out), size_t(n) * sizeof(float)));
 	// the loop state comes back through pinned words per host thread, one set
 	// per batch in flight
-	static thread_local unsigned long long *hstate = nullptr;
-	if (!hstate) PCUDA_TRY(cudaMallocHost(&hstate, 2 * 4 * sizeof(unsigned long long)));
+	struct host_state { unsigned long long w[2 * 4]; };
+	static thread_local thread_pinned<host_state> pinned;
+	host_state *hs = nullptr;
+	PCUDA_TRY(pinned.get(&hs));
+	unsigned long long *hstate = hs->w;
 	const unsigned gb = grid_for(n);
 	fill_kernel<<<gb, kThreads, 0, st>>>(in1, n, 1.0f);
 	PCUDA_TRY(cudaGetLastError());

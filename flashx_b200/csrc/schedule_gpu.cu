@@ -322,9 +322,11 @@ struct counts_back {
 	explicit counts_back(cudaStream_t s) : st(s) {}
 	int init()
 	{
-		static thread_local unsigned long long *pinned = nullptr;
-		if (!pinned) SCUDA_TRY(cudaMallocHost(&pinned, 16 * sizeof(unsigned long long)));
-		w = pinned;
+		struct words { unsigned long long w[16]; };
+		static thread_local thread_pinned<words> pinned;
+		words *p = nullptr;
+		SCUDA_TRY(pinned.get(&p));
+		w = p->w;
 		return FMX_OK;
 	}
 	template <class T>

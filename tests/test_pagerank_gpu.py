@@ -140,3 +140,25 @@ def test_pagerank_repeats_bit_exact(torch_cuda, n, m):
         pr, it = PageRank(mat, 12, 0.85)
         assert it == rit
         assert np.array_equal(pr.cpu().numpy(), ref)
+
+
+def test_pagerank_from_ending_threads(torch_cuda):
+    """The loop state's pinned words belong to a thread and go with it."""
+    import threading
+    src, dst = _directed(3000, 20000, 13)
+    m = create_2d_matrix(src, dst, None, block_size=(1024, 1024), is_sym=False, nrows=3000, ncols=3000)
+    ref, rit = PageRank(m, 20, 0.85)
+    ref = ref.cpu().numpy()
+    got = []
+
+    def run():
+        pr, it = PageRank(m, 20, 0.85)
+        got.append((pr.cpu().numpy(), it))
+
+    for _ in range(4):
+        t = threading.Thread(target=run)
+        t.start()
+        t.join()
+    assert len(got) == 4
+    for pr, it in got:
+        assert it == rit and np.array_equal(pr, ref)
