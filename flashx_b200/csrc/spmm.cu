@@ -306,7 +306,7 @@ __device__ __forceinline__ void pr_finish(const pr_epi &e)
 // row close is a branch: predicated stores cost every entry the conversion.
 // Times of the former kernels -> this one (whole fmx_spmm, B200):
 //   FP32 k = 16, R-MAT scale 16 / 20 / 22 / 24   41 / 177 / 512 / 1855 ->
-//                                               27 / 130 / 411 / 1785 us
+//                                               21 / 119 / 411 / 1785 us
 //   FP64 k = 8, scale 22                         593 -> 430 us
 //   FP32 k = 10 / 33, scale 20                   427 / 1111 -> 156 / 684 us
 //   int64 k = 4 weighted, scale 20               177 -> 149 us
@@ -534,17 +534,17 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 // in flight need the registers (spills cost more than the warps: BF16 with
 // 24 warps 801 us against 446 us with 20).
 constexpr int kLaneThreads = 128;
-constexpr int lane_blocks(int bytes, bool scaled, int esize)
+constexpr int lane_blocks(int bytes, bool scaled, int esize, int step)
 {
-	return bytes == 32 ? (scaled ? 4 : 3) : (scaled && esize == 8) ? 4 : (scaled || esize == 2) ? 5 : 6;
+	return step == 32 ? 2 : bytes == 16 && step == 16 ? 3 : bytes == 32 ? (scaled ? 4 : 3) : (scaled && esize == 8) ? 4 : (scaled || esize == 2) ? 5 : 6;
 }
-// Entries per step: 16 in lanes of at most 8 bytes of an unweighted, unscaled
+// Entries per step (launch_lanes takes more for small matrices): 16 in lanes of at most 8 bytes of an unweighted, unscaled
 // product (small or odd panels: R-MAT scale 18, k = 5, 39 against 43 us with
 // 8), else 8.
 constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 && esize >= 4 && plain ? 16 : 8; }
 
 template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
-__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT))))
+__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U))
 spmm_lane_kernel(const spmm_args a)
 {
 	dep_wait();
@@ -1357,23 +1357,43 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 	return FMX_OK;
 }
 
-template <class XT, class YT, class A, class WT, int VN, bool SI, bool SO>
-static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
+static int launch_step(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
-	constexpr int U = lane_step(VN * int(sizeof(XT)), int(sizeof(XT)), std::is_void<WT>::value && !SI && !SO);
 	auto kern = spmm_lane_kernel<XT, YT, A, WT, VN, U, SI, SO>;
 	static std::atomic<unsigned> blocks[64];
 	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kLaneThreads);
 	// A dependent launch hides the launch of a short kernel (R-MAT scale 16,
 	// k = 16: 26.8 -> 23.3 us with the fixup's).  Its blocks land where the pack's
 	// drain first instead of in SM order, which cost the BF16 operator at scale
-	// 21 2.6 %, so kernels of more than two rounds launch plainly; so do those
-	// of a streamed part, which follow their slice's copy.
+	// 21 2.6 %, so kernels of more than two rounds launch plainly (launch_lanes
+	// takes longer steps only for fewer); so do those of a streamed part,
+	// which follow their slice's copy.
 	const uint64_t groups = uint64_t(b) * (kLaneThreads / 32) * unsigned(a.R);
-	if (p.streamed || a.n_ranges > 2 * groups) kern<<<b, kLaneThreads, 0, st>>>(a);
+	constexpr bool kFew = U > lane_step(VN * int(sizeof(XT)), int(sizeof(XT)), std::is_void<WT>::value && !SI && !SO);
+	if (p.streamed || (!kFew && a.n_ranges > 2 * groups)) kern<<<b, kLaneThreads, 0, st>>>(a);
 	else CUDA_TRY(launch_dep(kern, b, kLaneThreads, st, a));
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
+}
+
+template <class XT, class YT, class A, class WT, int VN, bool SI, bool SO>
+static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
+{
+	constexpr int U = lane_step(VN * int(sizeof(XT)), int(sizeof(XT)), std::is_void<WT>::value && !SI && !SO);
+	// A small matrix leaves the machine to its longest ranges, rows of up to 256
+	// entries whose steps each wait for their gathers: more entries a step then
+	// beat more warps.  Lines in entries per group at 24 warps per SM.  Steps of
+	// 8, 16, 32 at 2 / 8 / 17 entries (FP32 k = 16, R-MAT scale 12 / 14 / 15):
+	// 20.6, 17.6, 17.2 / 22.6, 20.0, 16.6 / 22.7, 20.6, 17.8 us; at 33 (k = 8 at
+	// scale 17; int64 weighted k = 4) 24.8, 22.7, 24.7 and 30.8, 28.8, 32.4; at 45
+	// (int64, n = 300k) 36.2, 37.1, 41.1 us.
+	if constexpr (VN > 1 && (VN * sizeof(XT) == 16 || VN * sizeof(XT) == 8) && sizeof(XT) >= 4 && !SI && !SO) {
+		const uint64_t groups = 148ull * 24 * unsigned(a.R);
+		if (p.nnz <= 24 * groups) return launch_step<XT, YT, A, WT, VN, 32, SI, SO>(p, a, st);
+		if (U < 16 && p.nnz <= 40 * groups) return launch_step<XT, YT, A, WT, VN, 16, SI, SO>(p, a, st);
+	}
+	return launch_step<XT, YT, A, WT, VN, U, SI, SO>(p, a, st);
 }
 
 template <class XT, class YT, class A, class WT, int VN>

@@ -288,6 +288,26 @@ def test_lane_widths(torch_cuda, dtype, k):
             assert (got[:, :off] == 77).all() and (got[:, off + k:] == 77).all()
 
 
+@pytest.mark.parametrize("k,dtype,wdt", [(16, np.float32, None), (16, np.float32, np.float32), (12, np.float32, None),
+                                         (8, np.float64, None), (10, np.float32, None), (4, np.int64, np.int64)])
+@pytest.mark.parametrize("per_group", [20, 30, 50])
+def test_lane_steps(torch_cuda, per_group, k, dtype, wdt):
+    """The row kernel takes 32, 16 or 8 entries a step by the entries per lane
+    group of the machine (lines at 24 and 40); integer values keep every sum
+    exact, so all elements equal the oracle's, in rows of 0 to 256 entries and
+    in one longer row."""
+    torch = torch_cuda
+    lanes = k * np.dtype(dtype).itemsize // (8 if k == 10 else 16)
+    mm = per_group * 148 * 24 * (32 // lanes)
+    n = 20000
+    src, dst = _graph(n, mm, per_group + k, ((5, 256), (19999, 255), (77, 9000)))
+    vals = None if wdt is None else np.random.default_rng(k).integers(1, 5, len(src)).astype(wdt)
+    idx, mat = oracle.build_image(src, dst, vals, block=(16384, 16384), dedup=True)
+    m = sparse_matrix.create(matrix_image.from_bytes(idx, mat), None)
+    X = _dense(np.random.default_rng(k), (n, k), dtype, integer=True)
+    assert np.array_equal(_gpu_spmm(torch, m, X), oracle.spmm(idx, mat, X))
+
+
 def test_host_buffers_e2e(torch_cuda):
     src, dst = _graph(5000, 40000, 21)
     idx, mat = oracle.build_image(src, dst, None, block=(1024, 1024), dedup=True)
