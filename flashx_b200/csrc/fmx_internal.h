@@ -178,7 +178,7 @@ int spmm_packed(const fmx_matrix *m, int xt, const void *X, int64_t ldx, int yt,
 // < eps; pr = p2; in_next = p2 / deg; pr1 = in_next * deg.  A hot column's next
 // input also goes to its slot of the next hot pack (slot[row], 0: none).
 // state[0] counts this iteration's converged vertices, state[1] is the done
-// flag (set once every vertex converged or the iteration cap is reached; the
+// flag (set once every vertex converged or the iteration cap is reached; all
 // kernels of later iterations then return at once), state[2] the iterations
 // run, state[3] the blocks of the iteration's last kernel that are through:
 // the last of them applies the loop test (when `finish` is set).  A chunked row
@@ -203,6 +203,9 @@ struct pr_epi {
 int pagerank_iteration(const fmx_matrix *mt, const float *in, float *xhot, float *out, const pr_epi &e, cudaStream_t st);
 // Whether pagerank_iteration needs `out`.
 bool pagerank_needs_out(const fmx_matrix *mt);
+// Whether an iteration copies the matrix's entries to the device, also one
+// that is queued after the loop ended.
+bool pagerank_streamed(const fmx_matrix *mt);
 // Hot columns of mt's part (a pack holds one value more: slot 0 is zero), its
 // chunked rows and their chunks.
 void pagerank_sizes(const fmx_matrix *mt, uint64_t *hot, uint64_t *heavy, uint64_t *chunks);

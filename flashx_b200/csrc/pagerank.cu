@@ -15,14 +15,17 @@
 // One iteration of a small matrix is one pass: the SpMV on the transpose
 // (k = 1) applies the damping, counts the converged vertices and writes the
 // next input, and its hot pack, where it closes each row (rows summed in chunks
-// by the warp whose chunk arrives last); the last block applies the loop test.  Larger ones run the row kernel and the update as a
-// pass over the rows.  Input and pack are double-buffered (other rows still
-// gather this iteration's while the next ones are written).  What bounds a
-// small iteration is its kernels' latency: as four launches (pack, SpMV,
-// fixup, loop test) R-MAT scale 16 took 27 us per iteration.  Iterations are
-// queued in batches, one batch ahead of the host's read of the loop state; an
-// iteration queued after the loop ended returns at once, so the result and
-// the count match a loop that tests on the host after every iteration.
+// by the warp whose chunk arrives last); the last block applies the loop test.
+// Larger ones run the row kernel, its fixup and the update as a pass over the
+// rows.  Input and pack are double-buffered (other rows still gather this
+// iteration's while the next ones are written).  What bounds a small iteration
+// is its kernels' latency: as four launches (pack, SpMV, fixup, loop test)
+// R-MAT scale 16 took 27 us per iteration.  Iterations are queued in batches,
+// one batch ahead of the host's read of the loop state; every kernel of an
+// iteration queued after the loop ended returns at once, so the result and the
+// count match a loop that tests on the host after every iteration.  A streamed
+// matrix copies its entries for every queued iteration, so its batches are
+// queued one at a time.
 #include "fmx_internal.h"
 
 #include <cuda_runtime.h>
@@ -168,10 +171,11 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 		~events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
 	} ev;
 	for (cudaEvent_t &x : ev.e) PCUDA_TRY(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+	const uint64_t ahead = pagerank_streamed(mt) ? 1 : 2;
 	uint64_t it = 0, queued = 0, batches = 0, read = 0;
 	bool done = n == 0 || max_iters == 0;
 	while (!done) {
-		// queue a batch, then read the state of the one before
+		// queue a batch, then read the state of the one before (of itself when streamed)
 		if (queued < max_iters) {
 			const uint64_t batch = std::min<uint64_t>(kBatch, max_iters - queued);
 			for (uint64_t b = 0; b < batch; b++, queued++) {
@@ -183,7 +187,7 @@ int fmx_pagerank(const fmx_matrix *m, uint64_t max_iters, float damping, float *
 			PCUDA_TRY(cudaMemcpyAsync(hstate + 4 * (batches & 1), state, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
 			PCUDA_TRY(cudaEventRecord(ev.e[batches & 1], st));
 			batches++;
-			if (batches - read < 2 && queued < max_iters) continue;
+			if (batches - read < ahead && queued < max_iters) continue;
 		}
 		PCUDA_TRY(cudaEventSynchronize(ev.e[read & 1]));
 		it = hstate[4 * (read & 1) + 2];

@@ -183,6 +183,7 @@ struct spmm_args {
 	int G;           // lanes per row group
 	int R;           // row groups per warp
 	uint32_t n_ranges;
+	const unsigned long long *state;     // PageRank's loop state (pr_epi), read by the STOP forms of the kernels
 };
 
 // The running sums of one lane: NV vectors of VEC elements.  FP32 with
@@ -543,12 +544,17 @@ constexpr int lane_blocks(int bytes, bool scaled, int esize, int step)
 // 8), else 8.
 constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 && esize >= 4 && plain ? 16 : 8; }
 
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
+// STOP: a product of a PageRank loop, which returns at once when the loop has
+// ended (fmx_spmm's instances do not look).
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool STOP = false>
 __global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U))
 spmm_lane_kernel(const spmm_args a)
 {
 	dep_wait();
 	dep_launch();
+	if constexpr (STOP) {
+		if (a.state[1]) return;
+	}
 	const int lane = threadIdx.x & 31;
 	const int G = a.G, R = a.R;
 	const int grp = lane / G;
@@ -666,6 +672,9 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			raw[j] = i < rg.len ? __ldcs(a.col + rg.e0 + i) : 0u;
 		}
 		wait();
+		if constexpr (EPI) {
+			if (done) break;
+		}
 		T t[J];
 #pragma unroll
 		for (int j = 0; j < J; j++) {
@@ -696,9 +705,6 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			sval[wib][i] = t[j];
 		}
 		__syncwarp();
-		if constexpr (EPI) {
-			if (done) break;
-		}
 		if (runs) {
 			for (int q = lane; q < nrow; q += 32) {
 				const int b0 = q ? int(send[wib][q - 1]) + 1 : 0, b1 = send[wib][q] + 1;
@@ -921,13 +927,17 @@ __device__ __forceinline__ void fix_store(const heavy_row &h, const A (&v)[4], i
 	}
 }
 
-template <class YT, class A, bool SCALE_OUT>
+template <class YT, class A, bool SCALE_OUT, bool STOP>
 __global__ void __launch_bounds__(256) spmm_fixup_kernel(const heavy_row *heavy, uint32_t n_heavy, uint32_t n_block,
-		uint32_t n_long, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, int L)
+		uint32_t n_long, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, int L,
+		const unsigned long long *state)
 {
 	__shared__ A red[8][32][4];
 	dep_wait();
 	dep_launch();
+	if constexpr (STOP) {
+		if (state[1]) return;
+	}
 	constexpr bool kVec4 = std::is_same<A, float>::value;
 	const bool vec = kVec4 && (k % 4) == 0;
 	const int units = vec ? k / 4 : k, nv = vec ? 4 : 1;
@@ -978,8 +988,9 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const heavy_row *heavy,
 	}
 }
 
-template <class YT, class A, bool SCALE_OUT>
-static int launch_fixup(const gpu_part &p, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, cudaStream_t st)
+template <class YT, class A, bool SCALE_OUT, bool STOP = false>
+static int launch_fixup(const gpu_part &p, const A *partial, YT *Y, int64_t ldy, int k, const A *s_out, cudaStream_t st,
+		const unsigned long long *state = nullptr)
 {
 	if (!p.n_heavy) return FMX_OK;
 	const bool vec = std::is_same<A, float>::value && (k % 4) == 0;
@@ -992,11 +1003,11 @@ static int launch_fixup(const gpu_part &p, const A *partial, YT *Y, int64_t ldy,
 	const uint64_t per_warp = uint64_t(32 / (L * (L < 32 ? 2 : 1)));    // short rows per warp
 	const uint64_t warps = n_long + (n_short + per_warp - 1) / per_warp;
 	const unsigned grid = nb + unsigned((warps + 7) / 8);
-	auto kern = spmm_fixup_kernel<YT, A, SCALE_OUT>;
+	auto kern = spmm_fixup_kernel<YT, A, SCALE_OUT, STOP>;
 	if (p.streamed)
-		kern<<<grid, 256, 0, st>>>(p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L);
+		kern<<<grid, 256, 0, st>>>(p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L, state);
 	else
-		CUDA_TRY(launch_dep(kern, grid, 256, st, p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L));
+		CUDA_TRY(launch_dep(kern, grid, 256, st, p.heavy, p.n_heavy, nb, uint32_t(n_long), partial, Y, ldy, k, s_out, L, state));
 	CUDA_TRY(cudaGetLastError());
 	return FMX_OK;
 }
@@ -1357,10 +1368,10 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 	return FMX_OK;
 }
 
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool STOP = false>
 static int launch_step(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
-	auto kern = spmm_lane_kernel<XT, YT, A, WT, VN, U, SI, SO>;
+	auto kern = spmm_lane_kernel<XT, YT, A, WT, VN, U, SI, SO, STOP>;
 	static std::atomic<unsigned> blocks[64];
 	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kLaneThreads);
 	// A dependent launch hides the launch of a short kernel (R-MAT scale 16,
@@ -1649,6 +1660,7 @@ void pagerank_sizes(const fmx_matrix *mt, uint64_t *hot, uint64_t *heavy, uint64
 	*heavy = mt->a->n_heavy;
 	*chunks = mt->a->n_partials;
 }
+bool pagerank_streamed(const fmx_matrix *mt) { return mt->a->streamed; }
 bool pagerank_needs_out(const fmx_matrix *mt) { return !spmv_by_warps(*mt->a); }
 
 template <class WT>
@@ -1672,11 +1684,14 @@ static int pr_iteration_typed(const gpu_part &p, const float *in, float *xhot, f
 	a.Y = out; a.partial = p.partial;
 	a.ldx = a.ldy = 1; a.k = 1; a.G = 1; a.R = 32;
 	a.n_ranges = p.fine ? p.n_fine : p.n_ranges;
+	a.state = e.state;
+	constexpr int U = lane_step(int(sizeof(float)), int(sizeof(float)), std::is_void<WT>::value);
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
-			return launch_lanes<float, float, float, WT, 1, false, false>(p, sa, st);
+			return launch_step<float, float, float, WT, 1, U, false, false, true>(p, sa, st);
 		}))
 		return rc;
-	if (int rc = launch_fixup<float, float, false>(p, static_cast<const float *>(p.partial), out, 1, 1, nullptr, st)) return rc;
+	if (int rc = launch_fixup<float, float, false, true>(p, static_cast<const float *>(p.partial), out, 1, 1, nullptr, st, e.state))
+		return rc;
 	const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((p.nrows + kThreads - 1) / kThreads, 148ull * 8)));
 	CUDA_TRY(launch_dep(pr_apply_kernel, g, kThreads, st, out, int64_t(p.nrows), e));
 	return FMX_OK;

@@ -162,3 +162,84 @@ def test_pagerank_from_ending_threads(torch_cuda):
     assert len(got) == 4
     for pr, it in got:
         assert it == rit and np.array_equal(pr, ref)
+
+
+def _stepwise(torch, m, n, most):
+    """The ranks after each iteration of a host-driven loop of plain SpMVs
+    with the update in float32 numpy, until it converges (or `most`)."""
+    mt = m.transpose()
+    d = np.float32(0.85)
+    deg = np.maximum(m.multiply(torch.ones((n, 1), device="cuda")).cpu().numpy()[:, 0], np.float32(1))
+    tele, eps = np.float32((1.0 - float(d)) / n), np.float32(0.001 / n)
+    x = np.full(n, np.float32(1.0 / n), dtype=np.float32) / deg
+    pr1 = x * deg
+    ref, conv = [], 0
+    while conv < n and len(ref) < most:
+        p2 = mt.multiply(torch.from_numpy(x).cuda().reshape(n, 1)).cpu().numpy()[:, 0] * d + tele
+        conv = int(np.count_nonzero(np.abs(pr1 - p2) < eps))
+        x = p2 / deg
+        pr1 = x * deg
+        ref.append(p2)
+    return ref, conv == n
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("streamed", [False, True])
+def test_pagerank_row_kernel_form(torch_cuda, weighted, streamed):
+    """Beyond 64 ranges per SM an iteration is the row kernel, the fixup of
+    chunked rows and a pass of updates, the latter two dependent launches: the
+    stepwise loop's bits and counts for caps below, at and far above the point
+    of convergence (iterations queued after it must change nothing), several
+    times over."""
+    torch = torch_cuda
+    from flashx_b200 import matrix_image, sparse_matrix
+    n = 1 << 18
+    src, dst = rmat_edges(18, seed=5)
+    w = np.random.default_rng(3).uniform(0.5, 1, len(src)).astype(np.float32) if weighted else None
+    img = matrix_image.build(src, dst, w, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+    timg = matrix_image.build(dst, src, w, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+    m = sparse_matrix.create(img, timg)
+    assert m.transpose().schedule()[2] > 0        # rows summed in chunks
+    ref, ended = _stepwise(torch, m, n, 100)
+    assert ended
+    if streamed:
+        m = sparse_matrix.create_streamed(img, timg, slice_entries=1 << 20)
+    for cap in (3, len(ref), 200, 200, 17, 200):
+        got, git = PageRank(m, cap, 0.85)
+        assert git == min(cap, len(ref))
+        assert np.array_equal(got.cpu().numpy(), ref[git - 1])
+
+
+@pytest.mark.parametrize("n,m,streamed", [(100_000, 1_600_000, False), (1 << 20, 16 << 20, False), (1 << 18, 4 << 20, True)])
+def test_pagerank_ends_with_convergence(torch_cuda, n, m, streamed):
+    """A uniform graph converges in a few iterations: a cap far above that
+    costs little more than a cap at it (the batch that is queued when the loop
+    ends runs empty; a streamed matrix copies its entries in it), in all forms
+    of the iteration.  Whole queued iterations would make the ratio 2 or more."""
+    import time
+    torch = torch_cuda
+    from flashx_b200 import matrix_image, sparse_matrix
+    src, dst = _directed(n, m, 14)
+    if streamed:
+        img = matrix_image.build(src, dst, None, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+        timg = matrix_image.build(dst, src, None, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+        a = sparse_matrix.create_streamed(img, timg, slice_entries=1 << 19)
+    else:
+        s, d = (torch.from_numpy(x.astype(np.int32)).cuda() for x in (src, dst))
+        a = sparse_matrix.from_device_edges(s, d, None, nrows=n, ncols=n, dedup=True, transpose=True)
+    p1, it = PageRank(a, 200, 0.85)
+    assert it <= 8                                # within the first batch
+    p2, it2 = PageRank(a, it, 0.85)
+    assert it2 == it and torch.equal(p1, p2)
+
+    def best(cap):
+        t = []
+        for _ in range(7):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            PageRank(a, cap, 0.85)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    best(it)
+    assert best(200) <= 1.5 * best(it)
