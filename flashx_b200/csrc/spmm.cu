@@ -183,7 +183,7 @@ struct spmm_args {
 	int G;           // lanes per row group
 	int R;           // row groups per warp
 	uint32_t n_ranges;
-	const unsigned long long *state;     // PageRank's loop state (pr_epi), read by the STOP forms of the kernels
+	const unsigned long long *state;     // PageRank's loop state (pr_epi), read by the forms of its loop
 };
 
 // The running sums of one lane: NV vectors of VEC elements.  FP32 with
@@ -385,10 +385,86 @@ __device__ __forceinline__ void ld_wn(const void *val, uint32_t e0, A (&w)[U])
 	}
 }
 
+// A chunk's sum in the kernels of k = 1 without row scales.  A chunk may be
+// added in any fixed order; this one is the same in the lane kernel, whatever
+// its step, and in the warp-per-range kernel, so that the choice between them
+// does not show in the results: binary trees over blocks of 16 places, block b
+// added to running sum b % 4, and a tree over those.  Its error is that of 32
+// strided sums and a tree over them (8000 chunks of 129 to 256 FP32 numbers,
+// RMS against FP64: 7.6e-8 of normal ones against 7.8e-8, 4.0e-8 of uniform
+// ones in both; a single running sum of the blocks has 8.9e-8 and 5.9e-8; a
+// whole binary tree 7.6e-8 and 4.3e-8, for more registers).
+static_assert(kChunk == 256, "chunk_sum and warp_chunk add 256 places");
+template <class A, int U>
+struct chunk_sum {
+	static_assert(U == 8 || U == 16, "half blocks or blocks");
+	A s0, s1, s2, s3, half;
+	bool odd;                                        // `half` waits for its right neighbour
+
+	__device__ __forceinline__ void zero()
+	{
+		s0 = s1 = s2 = s3 = half = A(0);
+		odd = false;
+	}
+	__device__ __forceinline__ void turn(A t)
+	{
+		s0 = s1; s1 = s2; s2 = s3; s3 = t;
+	}
+	// the sum of the next U entries
+	__device__ __forceinline__ void add(A t)
+	{
+		if (U == 16) {
+			turn(acc_add(s0, t));
+			return;
+		}
+		if (odd) turn(acc_add(s0, acc_add(half, t)));
+		else half = t;
+		odd = !odd;
+	}
+	// the sum of a chunk of `len` (padded) entries
+	__device__ __forceinline__ A sum(uint32_t len)
+	{
+		if (U == 8 && odd) turn(acc_add(s0, half));
+		for (uint32_t b = (len + 15) / 16; b & 3u; b++) turn(s0);      // running sum 0 first
+		return acc_add(acc_add(s0, s1), acc_add(s2, s3));
+	}
+};
+
+// The same sum by a warp whose lane l holds the terms 32 j + l in t[j], j < 8
+// (zeros beyond the chunk).
+template <class A>
+__device__ __forceinline__ A warp_chunk(const A *t, int lane)
+{
+	A v[8];
+#pragma unroll
+	for (int j = 0; j < 8; j++) v[j] = t[j];
+	// bits 0 to 2 of the place; each exchange halves the lane's values of j
+#pragma unroll
+	for (int b = 0; b < 3; b++) {
+		const bool hi = (lane >> b) & 1;
+#pragma unroll
+		for (int q = 0; q < (4 >> b); q++) {
+			const A give = hi ? v[2 * q] : v[2 * q + 1], keep = hi ? v[2 * q + 1] : v[2 * q];
+			v[q] = acc_add(keep, __shfl_xor_sync(0xffffffffu, give, 1 << b));
+		}
+	}
+	// bit 3: lane l has block 2 (l % 8) + l / 16
+	const A blk = acc_add(v[0], __shfl_xor_sync(0xffffffffu, v[0], 8));
+	A r = __shfl_sync(0xffffffffu, blk, lane & 25);
+#pragma unroll
+	for (int q = 1; q < 4; q++) r = acc_add(r, __shfl_sync(0xffffffffu, blk, (lane & 25) | (2 * q)));
+	r = acc_add(r, __shfl_xor_sync(0xffffffffu, r, 16));
+	return acc_add(r, __shfl_xor_sync(0xffffffffu, r, 1));
+}
+
 // One range, U entries per step: the gathers (and scales, weights and the
 // next step's column ids) of a step are all issued before its adds.  Entries
 // of chunks carry no end flag, so only row runs store.
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO>
+// K1: k = 1 without row scales (chunks by chunk_sum, in the loop that row runs
+// take: a warp's lanes differ, and a loop of its own took R-MAT scale 18 from
+// 23 to 27 us); else a chunk is one running sum, of whole steps in one-element
+// lanes.
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool K1>
 __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, int colbase)
 {
 	constexpr bool kBinary = std::is_void<WT>::value;
@@ -403,6 +479,8 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 	const A *sop = SO ? static_cast<const A *>(a.s_out) + rg.row0 : nullptr;
 	accum<A, VN, 1> acc;
 	acc.zero();
+	chunk_sum<A, U == 8 ? 8 : 16> chunk;
+	if constexpr (K1) chunk.zero();
 	uint32_t e = rg.e0;
 	const uint32_t e_end = e + rg.len;
 	auto ids = [&](uint32_t at, uint32_t (&r)[U]) {
@@ -493,8 +571,6 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 		bool done = false;
 		if constexpr (VN == 1) {
 			if (rg.slot != kNoSlot) {
-				// a chunk may be added in any fixed order: the step's terms
-				// by a tree (the error of one long running sum is larger)
 				A t[U];
 #pragma unroll
 				for (int u = 0; u < U; u++) {
@@ -506,7 +582,8 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 				for (int d = 1; d < U; d *= 2)
 #pragma unroll
 					for (int u = 0; u + d < U; u += 2 * d) t[u] = acc_add(t[u], t[u + d]);
-				acc.s[0][0] = acc_add(acc.s[0][0], t[0]);
+				if constexpr (K1) chunk.add(t[0]);
+				else acc.s[0][0] = acc_add(acc.s[0][0], t[0]);
 				done = true;
 			}
 		}
@@ -525,8 +602,12 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 	}
 	if (rg.slot != kNoSlot) {
 		A *p = static_cast<A *>(a.partial) + int64_t(rg.slot) * kPartialStride + colbase;
+		if constexpr (K1) {
+			p[0] = chunk.sum(rg.len);
+		} else {
 #pragma unroll
-		for (int i = 0; i < VN; i++) p[i] = acc.get(0, i);
+			for (int i = 0; i < VN; i++) p[i] = acc.get(0, i);
+		}
 	}
 }
 
@@ -535,26 +616,28 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 // in flight need the registers (spills cost more than the warps: BF16 with
 // 24 warps 801 us against 446 us with 20).
 constexpr int kLaneThreads = 128;
-constexpr int lane_blocks(int bytes, bool scaled, int esize, int step)
+constexpr int lane_blocks(int bytes, bool scaled, int esize, int step, bool k1)
 {
-	return step == 32 ? 2 : bytes == 16 && step == 16 ? 3 : bytes == 32 ? (scaled ? 4 : 3) : (scaled && esize == 8) ? 4 : (scaled || esize == 2) ? 5 : 6;
+	return k1 && esize == 8 && step == 16 ? 5 : step == 32 ? 2 : bytes == 16 && step == 16 ? 3 : bytes == 32 ? (scaled ? 4 : 3) : (scaled && esize == 8) ? 4 : (scaled || esize == 2) ? 5 : 6;
 }
 // Entries per step (launch_lanes takes more for small matrices): 16 in lanes of at most 8 bytes of an unweighted, unscaled
 // product (small or odd panels: R-MAT scale 18, k = 5, 39 against 43 us with
 // 8), else 8.
 constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 && esize >= 4 && plain ? 16 : 8; }
 
-// STOP: a product of a PageRank loop, which returns at once when the loop has
-// ended (fmx_spmm's instances do not look).
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool STOP = false>
-__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U))
+// FORM: kAny, kOne (k = 1 without row scales) or kLoop (the same in a PageRank
+// loop: it returns at once when the loop has ended).
+enum { kAny, kOne, kLoop };
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, int FORM>
+__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U, FORM != kAny))
 spmm_lane_kernel(const spmm_args a)
 {
 	dep_wait();
 	dep_launch();
-	if constexpr (STOP) {
+	if constexpr (FORM == kLoop) {
 		if (a.state[1]) return;
 	}
+	constexpr bool K1 = FORM != kAny;
 	const int lane = threadIdx.x & 31;
 	const int G = a.G, R = a.R;
 	const int grp = lane / G;
@@ -570,9 +653,9 @@ spmm_lane_kernel(const spmm_args a)
 	const uint32_t g1 = (wib * gridDim.x + blockIdx.x) * uint32_t(R) + uint32_t(grp);
 	uint32_t base = 0;
 	for (; base + ng <= a.n_ranges; base += ng)
-		run_range<XT, YT, A, WT, VN, U, SI, SO>(a, a.ranges[base + g0], colbase);
+		run_range<XT, YT, A, WT, VN, U, SI, SO, K1>(a, a.ranges[base + g0], colbase);
 	if (base + g1 < a.n_ranges)
-		run_range<XT, YT, A, WT, VN, U, SI, SO>(a, a.ranges[base + g1], colbase);
+		run_range<XT, YT, A, WT, VN, U, SI, SO, K1>(a, a.ranges[base + g1], colbase);
 }
 
 // k = 1 (SpMV): a warp per range.  The 32 lanes load the range's column ids
@@ -580,8 +663,8 @@ spmm_lane_kernel(const spmm_args a)
 // then each lane sums whole rows of the range from shared memory in entry
 // order, with one running sum per row and every add rounded, which is the
 // lane-group kernel's arithmetic: rows of up to 256 entries come out
-// identical.  A chunk of a longer row is added up by the whole warp (each
-// lane its own entries, then a fixed xor tree) into its partial slot.
+// identical.  A chunk of a longer row is added up by the whole warp
+// (warp_chunk) into its partial slot.
 // (spmv_by_warps says which matrices come here.)
 constexpr int kSpmvMax = 512;            // most entries of one range
 static_assert(((kRange - 1 + kExactMax + kStep - 1) / kStep) * kStep <= uint32_t(kSpmvMax) &&
@@ -734,11 +817,7 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			}
 		} else {
 			// a chunk: each lane adds its entries (j order), then a fixed xor tree
-			T acc = T(0);
-#pragma unroll
-			for (int j = 0; j < J; j++) acc = acc_add(acc, t[j]);
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1) acc = acc_add(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+			const T acc = warp_chunk(t, lane);
 			if constexpr (EPI) pr_chunk(e, static_cast<float *>(a.partial), rg.slot, acc, lane, cnt);
 			else if (lane == 0) static_cast<T *>(a.partial)[int64_t(rg.slot) * kPartialStride] = acc;
 		}
@@ -1368,10 +1447,10 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 	return FMX_OK;
 }
 
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool STOP = false>
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, int FORM = kAny>
 static int launch_step(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
-	auto kern = spmm_lane_kernel<XT, YT, A, WT, VN, U, SI, SO, STOP>;
+	auto kern = spmm_lane_kernel<XT, YT, A, WT, VN, U, SI, SO, FORM>;
 	static std::atomic<unsigned> blocks[64];
 	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kLaneThreads);
 	// A dependent launch hides the launch of a short kernel (R-MAT scale 16,
@@ -1533,6 +1612,10 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 					static_cast<const A *>(sin), st))
 				return rc;
 		if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
+				if constexpr (std::is_same<XT, A>::value && std::is_same<YT, A>::value && std::is_floating_point<A>::value)
+					if (k == 1 && !sin && !sout)
+						return launch_step<A, A, A, WT, 1, lane_step(int(sizeof(A)), int(sizeof(A)), std::is_void<WT>::value), false,
+								false, kOne>(p, sa, st);
 				switch (vn) {
 				case 1: return launch_lanes_scaled<XT, YT, A, WT, 1>(p, sa, st);
 				case 2: return launch_lanes_scaled<XT, YT, A, WT, 2>(p, sa, st);
@@ -1687,7 +1770,7 @@ static int pr_iteration_typed(const gpu_part &p, const float *in, float *xhot, f
 	a.state = e.state;
 	constexpr int U = lane_step(int(sizeof(float)), int(sizeof(float)), std::is_void<WT>::value);
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
-			return launch_step<float, float, float, WT, 1, U, false, false, true>(p, sa, st);
+			return launch_step<float, float, float, WT, 1, U, false, false, kLoop>(p, sa, st);
 		}))
 		return rc;
 	if (int rc = launch_fixup<float, float, false, true>(p, static_cast<const float *>(p.partial), out, 1, 1, nullptr, st, e.state))

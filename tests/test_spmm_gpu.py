@@ -520,3 +520,103 @@ def test_rmat_s24_weighted(torch_cuda, rmat_s24, k):
     light = rmat_s24["outdeg"][: 4 * 16384] <= _lib.EXACT_ROW_MAX
     assert np.array_equal(Y[light], R[light])
     np.testing.assert_allclose(Y, R, rtol=RTOL, atol=RTOL * np.abs(R).max())
+
+
+def _whole_runs(rows, n):
+    """Ranges of the warp-per-range kernel's list for binary rows of these
+    entry counts: runs of whole rows and chunks of longer ones (part.h)."""
+    d = np.bincount(rows, minlength=n)
+    L = np.cumsum(np.where((d >= 1) & (d <= _lib.EXACT_ROW_MAX), d, 1))
+    run = int(np.clip(int(L[-1]) // (148 * 32 * 16), 128, 256)) // 8 * 8
+    start = np.concatenate([[0], L[:-1]]) // run
+    heavy = d[d > _lib.EXACT_ROW_MAX]
+    return 1 + int(np.count_nonzero(np.diff(start))) + int(np.sum((heavy + 255) // 256))
+
+
+def _blocks256(t):
+    """Sums of rows of 256 terms: binary trees over blocks of 16, block b added
+    to running sum b % 4, a tree over those."""
+    t = t.reshape(len(t), 16, 16)
+    while t.shape[2] > 1:
+        t = t[:, :, 0::2] + t[:, :, 1::2]
+    a = np.zeros((len(t), 4), t.dtype)
+    for q in range(4):
+        a = a + t[:, 4 * q:4 * q + 4, 0]
+    return (a[:, 0] + a[:, 1]) + (a[:, 2] + a[:, 3])
+
+
+def _strided32(t):
+    """The same by 32 strided running sums and a tree over them."""
+    a = np.zeros((len(t), 32), t.dtype)
+    for j in range(8):
+        a = a + t[:, 32 * j:32 * j + 32]
+    while a.shape[1] > 1:
+        h = a.shape[1] // 2
+        a = a[:, :h] + a[:, h:]
+    return a[:, 0]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("extra,warps", [(100_000, True), (3_000_000, False)])
+@pytest.mark.parametrize("length", [512, 437, 259])
+def test_spmv_chunk_sums(torch_cuda, length, extra, warps, weighted, dtype):
+    """k = 1, rows of two chunks of up to 256 entries: both kernels (a warp per
+    range up to 64 ranges per SM, else a lane per range) add a chunk in the same
+    order, bit for bit, and whole chunks with no larger error against FP64 than
+    32 strided sums have on the same numbers."""
+    torch = torch_cuda
+    n, rows = 1 << 17, 1500
+    rng = np.random.default_rng(extra)
+    cols = np.stack([np.sort(rng.choice(n, length, replace=False)) for _ in range(rows)])
+    src = np.concatenate([np.repeat(np.arange(rows), length), rng.integers(rows, n, extra)]).astype(np.uint32)
+    dst = np.concatenate([cols.reshape(-1), rng.integers(0, n, extra)]).astype(np.uint32)
+    assert (_whole_runs(src, n) <= 64 * torch.cuda.get_device_properties(0).multi_processor_count) == warps
+    w = rng.uniform(0.5, 1, len(src)).astype(dtype) if weighted else None
+    m = sparse_matrix.create(matrix_image.build(src, dst, w, nrows=n, ncols=n, block_size=(16384, 16384),
+                                                dedup=False, remove_self=False), None)
+    X = rng.standard_normal((n, 1)).astype(dtype)
+    got = _gpu_spmm(torch, m, X)[:rows, 0]
+    t = X[cols, 0]
+    if weighted:
+        t = t * w[:rows * length].reshape(rows, length)
+    c = np.zeros((2, rows, 256), t.dtype)
+    c[0, :, :length // 2], c[1, :, :length - length // 2] = t[:, :length // 2], t[:, length // 2:]
+    assert np.array_equal(got, _blocks256(c[0]) + _blocks256(c[1]))
+    if dtype == "float32" and length == 512:
+        exact = t.astype(np.float64).sum(1)
+        assert np.linalg.norm(got - exact) <= np.linalg.norm(_strided32(c[0]) + _strided32(c[1]) - exact)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("scale,warps", [(15, True), (18, False)])
+def test_spmv_forms_agree(torch_cuda, scale, warps, dtype):
+    """k = 1 on both sides of the line between the warp-per-range kernel and
+    the row kernel, against the row kernel's scaled form with scales of exactly
+    1: equal bits in rows of up to EXACT_ROW_MAX entries, hub rows (whose chunks
+    are added in another order) within RTOL, weighted or not, also for a strided
+    column."""
+    torch = torch_cuda
+    tdt = getattr(torch, dtype)
+    n = 1 << scale
+    src, dst = rmat_edges(scale, seed=4)
+    key = np.unique(src.astype(np.int64) * n + dst)
+    src, dst = (key // n).astype(np.uint32), (key % n).astype(np.uint32)
+    assert (_whole_runs(src, n) <= 64 * torch.cuda.get_device_properties(0).multi_processor_count) == warps
+    ones = torch.ones(n, device="cuda", dtype=tdt)
+    for weighted in (False, True):
+        vals = np.random.default_rng(1).uniform(0.0, 1.0, len(src)).astype(np.float32) if weighted else None
+        m = sparse_matrix.create(matrix_image.build(src, dst, vals, nrows=n, ncols=n, block_size=(16384, 16384),
+                                                    dedup=False, remove_self=False), None)
+        light = torch.from_numpy(np.bincount(src, minlength=n) <= _lib.EXACT_ROW_MAX).cuda()
+        X = torch.randn((n, 1), device="cuda", dtype=tdt)
+        Y1 = m.multiply(X)
+        Ys = torch.empty_like(Y1)
+        assert m.multiply(X, Ys, row_scale_in=ones, row_scale_out=ones)
+        assert torch.equal(Y1[light], Ys[light]) and not bool(light.all())
+        torch.testing.assert_close(Y1, Ys, rtol=RTOL, atol=RTOL * float(Ys.abs().max()))
+        X3 = torch.zeros((n, 3), device="cuda", dtype=tdt)
+        X3[:, :1] = X
+        Y3 = torch.full((n, 3), 7.0, device="cuda", dtype=tdt)
+        assert m.multiply(X3[:, :1], Y3[:, :1])
+        assert torch.equal(Y3[:, :1], Y1) and bool((Y3[:, 1:] == 7).all())
