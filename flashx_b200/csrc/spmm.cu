@@ -1527,8 +1527,9 @@ static int lane_width(const void *X, int64_t ldx, const void *Y, int64_t ldy, in
 // ranges in one round, where its short chain wins (R-MAT scale 16: 18.9
 // against 20.6 us); beyond that a lane per range in the row kernel, which
 // issues a third of the instructions per entry (scale 18 / 20 / 22 / 24: 38 /
-// 111 / 325 / 1400 against 29 / 66 / 251 / 1150 us).  Decided on the whole
-// part, so that a streamed matrix takes the resident one's kernels.
+// 111 / 325 / 1400 against 29 / 66 / 251 / 1150 us).  A streamed part is
+// launched slice by slice, so its largest slice decides (R-MAT scale 18 in
+// slices of 64k entries 700 against 975 us); both kernels give the same bits.
 static bool spmv_by_warps(const gpu_part &p)
 {
 	static std::atomic<unsigned> sms[64];
@@ -1538,7 +1539,9 @@ static bool spmv_by_warps(const gpu_part &p)
 		cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, p.device);
 		sms[p.device & 63].store(n = unsigned(std::max(v, 1)), std::memory_order_relaxed);
 	}
-	return p.n_ranges <= n * 64;
+	uint32_t most = p.streamed ? 0 : p.n_ranges;
+	for (const auto &sl : p.slices) most = std::max(most, sl.nr);
+	return most <= n * 64;
 }
 
 // Run one orientation over all column panels (kPanelBytes of X row each).

@@ -81,3 +81,21 @@ def test_streamed_rejected_by_noalloc(torch_cuda, rmat16):
     rc = _lib.lib.fmx_spmm_noalloc(st.handle, X.data_ptr(), 16, Y.data_ptr(), 16, 16,
                                    torch.cuda.current_stream().cuda_stream)
     assert rc == _lib.FMX_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("slice_entries", [1 << 16, 1 << 19, 1 << 22])
+def test_streamed_spmv_in_small_slices(torch_cuda, weighted, slice_entries):
+    """k = 1 of a matrix beyond 64 ranges per SM: its slices, each below that,
+    take the warp-per-range kernel, the resident matrix the row kernel; equal
+    bits, hub rows included."""
+    torch = torch_cuda
+    n = 1 << 18
+    s, d = rmat_edges(18, seed=3)
+    w = np.random.default_rng(0).uniform(-1, 1, len(s)).astype(np.float32) if weighted else None
+    img = matrix_image.build(s, d, w, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+    res, st = sparse_matrix.create(img, None), sparse_matrix.create_streamed(img, None, slice_entries=slice_entries)
+    assert res.schedule()[2] > 0
+    for dt in (torch.float32, torch.float64):
+        X = torch.randn((n, 1), device="cuda", dtype=dt)
+        assert torch.equal(res.multiply(X), st.multiply(X))
