@@ -242,6 +242,17 @@ struct accum {
 			}
 		}
 	}
+	// s[0] += t
+	__device__ __forceinline__ void add_terms(const A (&t)[VEC])
+	{
+		if constexpr (kPacked) {
+#pragma unroll
+			for (int i = 0; i < VEC / 2; i++) p[i] = add2(p[i], pack2(t[2 * i], t[2 * i + 1]));
+		} else {
+#pragma unroll
+			for (int i = 0; i < VEC; i++) s[0][i] = acc_add(s[0][i], t[i]);
+		}
+	}
 	__device__ __forceinline__ A get(int v, int i) const
 	{
 		if constexpr (kPacked) {
@@ -355,6 +366,23 @@ __device__ __forceinline__ xvec<T, VN> ld_n(const char *p)
 	return r;
 }
 
+// The same for elements `stride` bytes apart, the first `live` of them (zeros
+// behind).
+template <class T, int VN>
+__device__ __forceinline__ xvec<T, VN> ld_apart(const char *p, uint32_t stride, int live)
+{
+	static_assert(sizeof(T) == 2, "2-byte elements");
+	xvec<T, VN> r;
+#pragma unroll
+	for (int i = 0; i < VN; i++) {
+		unsigned short v;
+		asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u16 %0, 0;\n\t@q ld.global.u16 %0, [%1];\n\t}"
+				: "=h"(v) : "l"(p + i * stride), "r"(uint32_t(i < live)));
+		memcpy(&r.v[i], &v, 2);
+	}
+	return r;
+}
+
 // v = *p when `pred` holds (predicated, no branch)
 __device__ __forceinline__ void ld_if(float &v, const float *p, bool pred)
 {
@@ -463,12 +491,14 @@ __device__ __forceinline__ A warp_chunk(const A *t, int lane)
 // K1: k = 1 without row scales (chunks by chunk_sum, in the loop that row runs
 // take: a warp's lanes differ, and a loop of its own took R-MAT scale 18 from
 // 23 to 27 us); else a chunk is one running sum, of whole steps in one-element
-// lanes.
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool K1>
+// lanes.  APART: a lane's columns are colbase + i * G instead of neighbours.
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool K1, bool APART>
 __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, int colbase)
 {
 	constexpr bool kBinary = std::is_void<WT>::value;
 	static_assert(U % kStep == 0, "whole id loads");
+	const int apart = APART ? a.G : 1;
+	const int live = APART ? (a.k - colbase + a.G - 1) / a.G : VN;     // columns below k
 	const char *Xb = static_cast<const char *>(a.X) + size_t(colbase) * sizeof(XT);
 	const char *Hb = static_cast<const char *>(a.xhot) + size_t(colbase) * sizeof(XT);
 	// 32-bit row strides (one wide multiply-add per address); one-element
@@ -502,7 +532,9 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 		for (int u = 0; u < U; u++) {
 			const uint32_t c = raw[u] & kIdxMask;
 			const bool hot = raw[u] & kHot;
-			x[u] = ld_n<XT, VN>((hot ? Hb : Xb) + uint64_t(c) * (hot ? hs : xs));
+			const char *xp = (hot ? Hb : Xb) + uint64_t(c) * (hot ? hs : xs);
+			if constexpr (APART) x[u] = ld_apart<XT, VN>(xp, uint32_t(apart) * uint32_t(sizeof(XT)), live);
+			else x[u] = ld_n<XT, VN>(xp);
 		}
 		// the scales that this step needs, loaded with its rows: s_in of cold
 		// entries (the pack's rows carry theirs) and s_out of the rows that
@@ -562,28 +594,40 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 						if constexpr (SO) v = acc_mul(v, so[u]);
 						out[i] = from_acc<YT, A>(v);
 					}
-					st_y<YT, VN>(yp, out);
+					if constexpr (APART) {
+#pragma unroll
+						for (int i = 0; i < VN; i++)
+							if (i < live) yp[i * apart] = out[i];
+					} else {
+						st_y<YT, VN>(yp, out);
+					}
 					yp += a.ldy;
 					acc.zero();
 				}
 			}
 		};
 		bool done = false;
-		if constexpr (VN == 1) {
+		if constexpr (VN == 1 || APART) {
 			if (rg.slot != kNoSlot) {
-				A t[U];
+				// the step's terms of a column by a tree
+				A r[VN];
 #pragma unroll
-				for (int u = 0; u < U; u++) {
-					t[u] = to_acc<A>(x[u].v[0]);
-					if constexpr (SI) { if (cold) t[u] = acc_mul(t[u], sc[u]); }
-					if constexpr (!kBinary) t[u] = acc_mul(t[u], w[u]);
+				for (int i = 0; i < VN; i++) {
+					A t[U];
+#pragma unroll
+					for (int u = 0; u < U; u++) {
+						t[u] = to_acc<A>(x[u].v[i]);
+						if constexpr (SI) { if (cold) t[u] = acc_mul(t[u], sc[u]); }
+						if constexpr (!kBinary) t[u] = acc_mul(t[u], w[u]);
+					}
+#pragma unroll
+					for (int d = 1; d < U; d *= 2)
+#pragma unroll
+						for (int u = 0; u + d < U; u += 2 * d) t[u] = acc_add(t[u], t[u + d]);
+					r[i] = t[0];
 				}
-#pragma unroll
-				for (int d = 1; d < U; d *= 2)
-#pragma unroll
-					for (int u = 0; u + d < U; u += 2 * d) t[u] = acc_add(t[u], t[u + d]);
-				if constexpr (K1) chunk.add(t[0]);
-				else acc.s[0][0] = acc_add(acc.s[0][0], t[0]);
+				if constexpr (K1) chunk.add(r[0]);
+				else acc.add_terms(r);
 				done = true;
 			}
 		}
@@ -606,7 +650,8 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 			p[0] = chunk.sum(rg.len);
 		} else {
 #pragma unroll
-			for (int i = 0; i < VN; i++) p[i] = acc.get(0, i);
+			for (int i = 0; i < VN; i++)
+				if (!APART || i < live) p[i * apart] = acc.get(0, i);
 		}
 	}
 }
@@ -626,10 +671,11 @@ constexpr int lane_blocks(int bytes, bool scaled, int esize, int step, bool k1)
 constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 && esize >= 4 && plain ? 16 : 8; }
 
 // FORM: kAny, kOne (k = 1 without row scales) or kLoop (the same in a PageRank
-// loop: it returns at once when the loop has ended).
-enum { kAny, kOne, kLoop };
+// loop: it returns at once when the loop has ended) or kApart (VN columns per
+// lane, G apart, in rows that are no whole units: lane_width).
+enum { kAny, kOne, kLoop, kApart };
 template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, int FORM>
-__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U, FORM != kAny))
+__global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U, FORM == kOne || FORM == kLoop))
 spmm_lane_kernel(const spmm_args a)
 {
 	dep_wait();
@@ -637,12 +683,12 @@ spmm_lane_kernel(const spmm_args a)
 	if constexpr (FORM == kLoop) {
 		if (a.state[1]) return;
 	}
-	constexpr bool K1 = FORM != kAny;
+	constexpr bool K1 = FORM == kOne || FORM == kLoop, kSplit = FORM == kApart;
 	const int lane = threadIdx.x & 31;
 	const int G = a.G, R = a.R;
 	const int grp = lane / G;
 	if (grp >= R) return;
-	const int colbase = (lane - grp * G) * VN;
+	const int colbase = (lane - grp * G) * (kSplit ? 1 : VN);
 	constexpr uint32_t wpb = kLaneThreads / 32;
 	const uint32_t wib = threadIdx.x >> 5;
 	const uint32_t ng = gridDim.x * wpb * uint32_t(R);
@@ -653,9 +699,9 @@ spmm_lane_kernel(const spmm_args a)
 	const uint32_t g1 = (wib * gridDim.x + blockIdx.x) * uint32_t(R) + uint32_t(grp);
 	uint32_t base = 0;
 	for (; base + ng <= a.n_ranges; base += ng)
-		run_range<XT, YT, A, WT, VN, U, SI, SO, K1>(a, a.ranges[base + g0], colbase);
+		run_range<XT, YT, A, WT, VN, U, SI, SO, K1, kSplit>(a, a.ranges[base + g0], colbase);
 	if (base + g1 < a.n_ranges)
-		run_range<XT, YT, A, WT, VN, U, SI, SO, K1>(a, a.ranges[base + g1], colbase);
+		run_range<XT, YT, A, WT, VN, U, SI, SO, K1, kSplit>(a, a.ranges[base + g1], colbase);
 }
 
 // k = 1 (SpMV): a warp per range.  The 32 lanes load the range's column ids
@@ -1467,7 +1513,7 @@ static int launch_step(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 	return FMX_OK;
 }
 
-template <class XT, class YT, class A, class WT, int VN, bool SI, bool SO>
+template <class XT, class YT, class A, class WT, int VN, bool SI, bool SO, int FORM>
 static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
 	constexpr int U = lane_step(VN * int(sizeof(XT)), int(sizeof(XT)), std::is_void<WT>::value && !SI && !SO);
@@ -1478,23 +1524,23 @@ static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 	// 20.6, 17.6, 17.2 / 22.6, 20.0, 16.6 / 22.7, 20.6, 17.8 us; at 33 (k = 8 at
 	// scale 17; int64 weighted k = 4) 24.8, 22.7, 24.7 and 30.8, 28.8, 32.4; at 45
 	// (int64, n = 300k) 36.2, 37.1, 41.1 us.
-	if constexpr (VN > 1 && (VN * sizeof(XT) == 16 || VN * sizeof(XT) == 8) && sizeof(XT) >= 4 && !SI && !SO) {
+	if constexpr (FORM == kAny && VN > 1 && (VN * sizeof(XT) == 16 || VN * sizeof(XT) == 8) && sizeof(XT) >= 4 && !SI && !SO) {
 		const uint64_t groups = 148ull * 24 * unsigned(a.R);
 		if (p.nnz <= 24 * groups) return launch_step<XT, YT, A, WT, VN, 32, SI, SO>(p, a, st);
 		if (U < 16 && p.nnz <= 40 * groups) return launch_step<XT, YT, A, WT, VN, 16, SI, SO>(p, a, st);
 	}
-	return launch_step<XT, YT, A, WT, VN, U, SI, SO>(p, a, st);
+	return launch_step<XT, YT, A, WT, VN, U, SI, SO, FORM>(p, a, st);
 }
 
-template <class XT, class YT, class A, class WT, int VN>
+template <class XT, class YT, class A, class WT, int VN, int FORM = kAny>
 static int launch_lanes_scaled(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
 	if constexpr (std::is_floating_point<A>::value && (sizeof(XT) == 4 || VN * sizeof(XT) <= 16)) {
-		if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true>(p, a, st);
-		if (a.s_in) return launch_lanes<XT, YT, A, WT, VN, true, false>(p, a, st);
-		if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true>(p, a, st);
+		if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true, FORM>(p, a, st);
+		if (a.s_in) return launch_lanes<XT, YT, A, WT, VN, true, false, FORM>(p, a, st);
+		if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true, FORM>(p, a, st);
 	}
-	return launch_lanes<XT, YT, A, WT, VN, false, false>(p, a, st);
+	return launch_lanes<XT, YT, A, WT, VN, false, false, FORM>(p, a, st);
 }
 
 static bool aligned_to(const void *p, size_t n) { return (reinterpret_cast<uintptr_t>(p) % n) == 0; }
@@ -1521,6 +1567,26 @@ static int lane_width(const void *X, int64_t ldx, const void *Y, int64_t ldy, in
 	int vn = V16;
 	while (vn > 1 && !fits(vn)) vn /= 2;
 	return vn;
+}
+
+// BF16 rows that are no whole units of two or more elements (odd widths, odd
+// strides or starts): lanes of four elements, G apart, instead of one-element
+// lanes, where those hold at most two rows a warp and an entry's decoding
+// weighs more than its loads (R-MAT scale 21, k = 15 / 31 / 63: unscaled 544 ->
+// 456, 1056 -> 727, 2146 -> 1372 us; D^-1/2 A D^-1/2 1374 -> 861, 2652 -> 1510,
+// 5324 -> 2900 us; before the row kernel 500, 907, 1722 and 985, 1826, 3497 us),
+// and, where cold entries load scales, for 7 to 10 columns of large matrices (7
+// columns at scale 21 722 -> 641 us, unscaled 284 -> 339).  Fewer entries than 300
+// per warp leave the grid to the longest chains, which one-element lanes walk
+// faster (scale 14, k = 15 18.6 against 27 us; scale 16, k = 15 27 against 33 us,
+// k = 17, one row a warp, 45 against 36 us).
+constexpr int kApartUnit = 4;
+template <class XT>
+static bool lanes_apart(const gpu_part &p, int vn, int64_t ldx, int64_t k, bool scales_in)
+{
+	if (sizeof(XT) != 2 || vn != 1 || k < 7 || uint64_t(ldx) * sizeof(XT) >= (1ull << 32)) return false;
+	const uint64_t warps = 148ull * 20 * uint64_t(32 / std::min<int64_t>(k, 32));
+	return k >= 11 ? p.nnz >= 300 * warps : scales_in && p.nnz >= 1500 * warps;
 }
 
 // k = 1: the warp-per-range kernel while its grid (64 warps per SM) takes the
@@ -1596,7 +1662,9 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 	const int vn = lane_width<XT, YT>(X, ldx, Y, ldy, k, sin || sout);
 	constexpr int V32 = int(32 / sizeof(XT));
 	// column panels of at most kPanelBytes of X row, and 32 lanes
-	const int panel = std::min(kPanelBytes / int(sizeof(XT)), 32 * vn);
+	const bool apart = lanes_apart<XT>(p, vn, ldx, k, sin != nullptr);
+	const int unit = apart ? kApartUnit : vn;
+	const int panel = std::min(kPanelBytes / int(sizeof(XT)), 32 * unit);
 	for (int64_t c0 = 0; c0 < k; c0 += panel) {
 		const int kp = int(std::min<int64_t>(panel, k - c0));
 		spmm_args a{};
@@ -1608,7 +1676,7 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 		a.s_in = sin; a.s_out = sout; a.partial = partial;
 		a.ldx = ldx; a.ldy = ldy; a.k = kp;
 		a.n_ranges = p.fine ? p.n_fine : p.n_ranges;
-		a.G = kp / vn;
+		a.G = (kp + unit - 1) / unit;
 		a.R = 32 / a.G;
 		if (!packed)
 			if (int rc = launch_pack<XT, A>(p, static_cast<const XT *>(a.X), ldx, kp, static_cast<XT *>(xhot), kp,
@@ -1619,6 +1687,8 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 					if (k == 1 && !sin && !sout)
 						return launch_step<A, A, A, WT, 1, lane_step(int(sizeof(A)), int(sizeof(A)), std::is_void<WT>::value), false,
 								false, kOne>(p, sa, st);
+				if constexpr (sizeof(XT) == 2)
+					if (apart) return launch_lanes_scaled<XT, YT, A, WT, kApartUnit, kApart>(p, sa, st);
 				switch (vn) {
 				case 1: return launch_lanes_scaled<XT, YT, A, WT, 1>(p, sa, st);
 				case 2: return launch_lanes_scaled<XT, YT, A, WT, 2>(p, sa, st);

@@ -620,3 +620,60 @@ def test_spmv_forms_agree(torch_cuda, scale, warps, dtype):
         Y3 = torch.full((n, 3), 7.0, device="cuda", dtype=tdt)
         assert m.multiply(X3[:, :1], Y3[:, :1])
         assert torch.equal(Y3[:, :1], Y1) and bool((Y3[:, 1:] == 7).all())
+
+
+@pytest.mark.parametrize("ydt", ["float32", "bfloat16"])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("k,pad", [(9, 0), (11, 0), (13, 2), (16, 1), (21, 0), (31, 0), (33, 0), (63, 0), (65, 0), (130, 1)])
+def test_bf16_rows_of_odd_width(torch_cuda, k, pad, weighted, ydt):
+    """BF16 rows that are no whole vectors, on a matrix with enough entries for
+    lanes of four columns G apart: remainders of 1 to 4 columns in the last
+    lanes, several panels, odd strides, with and without scales.  Small integer
+    values, weights and power-of-two scales keep every sum exact (BF16 results:
+    its rounding), in rows of 0 to 256 entries and in two longer ones."""
+    torch = torch_cuda
+    n, mm = 30000, 300 * 148 * 20 * 4
+    src, dst = _graph(n, mm, 60 + k, ((5, 256), (29999, 9000), (77, 300)))
+    rng = np.random.default_rng(k)
+    vals = rng.integers(1, 3, len(src)).astype(np.float32) if weighted else None
+    idx, mat = oracle.build_image(src, dst, vals, block=(16384, 16384), dedup=True)
+    m = sparse_matrix.create(matrix_image.from_bytes(idx, mat), None)
+    assert m.get_nnz() >= 300 * 148 * 20 * (32 // min(k, 32))
+    X = rng.integers(-2, 3, (n, k))
+    s = np.ldexp(1.0, rng.integers(-2, 3, n))
+    sc = torch.from_numpy(s).to("cuda", torch.float32)
+    tdt = getattr(torch, ydt)
+    Xw = torch.full((n, k + pad), 99, dtype=torch.bfloat16, device="cuda")
+    Xw[:, :k] = torch.from_numpy(X).to("cuda", torch.bfloat16)
+    R = oracle.spmm(idx, mat, X.astype(np.float64))
+    Rs = oracle.spmm(idx, mat, X * s[:, None])
+    for si, so, want in ((None, None, R), (sc, None, Rs), (None, sc, R * s[:, None]), (sc, sc, Rs * s[:, None])):
+        Yw = torch.full((n, k + pad), 77, dtype=tdt, device="cuda")
+        assert m.multiply(Xw[:, :k], Yw[:, :k], si, so), _lib.last_error()
+        assert torch.equal(Yw[:, :k].cpu(), torch.from_numpy(want).to(tdt))
+        assert bool((Yw[:, k:] == 77).all())
+
+
+def test_bf16_odd_width_costs_no_more_than_fp32(torch_cuda):
+    """D^-1/2 A D^-1/2 on 31 columns at R-MAT scale 20: BF16 rows, half the
+    bytes, must not take longer than FP32 rows."""
+    torch = torch_cuda
+    n = 1 << 20
+    s, d = rmat_edges(20, seed=1)
+    s, d = (torch.from_numpy(np.concatenate(p).astype(np.int32)).cuda() for p in ((s, d), (d, s)))
+    m = sparse_matrix.from_device_edges(s, d, None, nrows=n, ncols=n, dedup=True)
+    sc = torch.rand(n, device="cuda") + 0.5
+    best = {}
+    for dt in (torch.float32, torch.bfloat16):
+        x = torch.randn((n, 31), device="cuda").to(dt)
+        y = torch.empty_like(x)
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(9)]
+        for _ in range(3):
+            assert m.multiply(x, y, sc, sc)
+        ev[0].record()
+        for e in ev[1:]:
+            assert m.multiply(x, y, sc, sc)
+            e.record()
+        torch.cuda.synchronize()
+        best[dt] = min(a.elapsed_time(b) for a, b in zip(ev, ev[1:]))
+    assert best[torch.bfloat16] <= best[torch.float32]
