@@ -139,6 +139,17 @@ __device__ __forceinline__ void st_y(T *p, const T (&v)[VEC])
 	}
 }
 
+// One whole sector (32-byte aligned).
+template <class T, int VEC>
+__device__ __forceinline__ void st_sector(T *p, const T (&v)[VEC])
+{
+	static_assert(VEC * sizeof(T) == 32, "32 bytes");
+	uint32_t u[8];
+	memcpy(u, v, 32);
+	asm volatile("st.global.cs.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+			:: "l"(p), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]) : "memory");
+}
+
 // Programmatic dependent launch.  A call's kernels are launched with the
 // attribute, so that the next one's blocks come in while the last one's drain;
 // dep_wait() holds them until the kernel before has completed.  Every kernel of
@@ -492,7 +503,9 @@ __device__ __forceinline__ A warp_chunk(const A *t, int lane)
 // take: a warp's lanes differ, and a loop of its own took R-MAT scale 18 from
 // 23 to 27 us); else a chunk is one running sum, of whole steps in one-element
 // lanes.  APART: a lane's columns are colbase + i * G instead of neighbours.
-template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool K1, bool APART>
+// BRANCH: a lane's 32 result bytes go out as one sector or as two halves, by
+// Y's alignment, which makes the row close a branch (branch_close).
+template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, bool K1, bool APART, bool BRANCH>
 __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, int colbase)
 {
 	constexpr bool kBinary = std::is_void<WT>::value;
@@ -598,6 +611,9 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 #pragma unroll
 						for (int i = 0; i < VN; i++)
 							if (i < live) yp[i * apart] = out[i];
+					} else if constexpr (BRANCH) {
+						if ((reinterpret_cast<uintptr_t>(yp) & 31) == 0) st_sector<YT, VN>(yp, out);
+						else st_y<YT, VN>(yp, out);
 					} else {
 						st_y<YT, VN>(yp, out);
 					}
@@ -672,8 +688,9 @@ constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 &&
 
 // FORM: kAny, kOne (k = 1 without row scales) or kLoop (the same in a PageRank
 // loop: it returns at once when the loop has ended) or kApart (VN columns per
-// lane, G apart, in rows that are no whole units: lane_width).
-enum { kAny, kOne, kLoop, kApart };
+// lane, G apart, in rows that are no whole units: lanes_apart) or kBranch
+// (branch_close).
+enum { kAny, kOne, kLoop, kApart, kBranch };
 template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, int FORM>
 __global__ void __launch_bounds__(kLaneThreads, lane_blocks(VN * int(sizeof(XT)), SI || SO, int(sizeof(XT)), U, FORM == kOne || FORM == kLoop))
 spmm_lane_kernel(const spmm_args a)
@@ -683,7 +700,7 @@ spmm_lane_kernel(const spmm_args a)
 	if constexpr (FORM == kLoop) {
 		if (a.state[1]) return;
 	}
-	constexpr bool K1 = FORM == kOne || FORM == kLoop, kSplit = FORM == kApart;
+	constexpr bool K1 = FORM == kOne || FORM == kLoop, kSplit = FORM == kApart, kBr = FORM == kBranch;
 	const int lane = threadIdx.x & 31;
 	const int G = a.G, R = a.R;
 	const int grp = lane / G;
@@ -699,9 +716,9 @@ spmm_lane_kernel(const spmm_args a)
 	const uint32_t g1 = (wib * gridDim.x + blockIdx.x) * uint32_t(R) + uint32_t(grp);
 	uint32_t base = 0;
 	for (; base + ng <= a.n_ranges; base += ng)
-		run_range<XT, YT, A, WT, VN, U, SI, SO, K1, kSplit>(a, a.ranges[base + g0], colbase);
+		run_range<XT, YT, A, WT, VN, U, SI, SO, K1, kSplit, kBr>(a, a.ranges[base + g0], colbase);
 	if (base + g1 < a.n_ranges)
-		run_range<XT, YT, A, WT, VN, U, SI, SO, K1, kSplit>(a, a.ranges[base + g1], colbase);
+		run_range<XT, YT, A, WT, VN, U, SI, SO, K1, kSplit, kBr>(a, a.ranges[base + g1], colbase);
 }
 
 // k = 1 (SpMV): a warp per range.  The 32 lanes load the range's column ids
@@ -1589,6 +1606,18 @@ static bool lanes_apart(const gpu_part &p, int vn, int64_t ldx, int64_t k, bool 
 	return k >= 11 ? p.nnz >= 300 * warps : scales_in && p.nnz >= 1500 * warps;
 }
 
+// BF16 rows into FP32, eight columns a lane.  With one way to store them the
+// compiler predicates the row close, so that every entry pays for its stores
+// and resets; with two it branches around them.  The branch pays from three
+// lanes a row on, where few rows share a warp (R-MAT scale 20 / 22, input scales,
+// k = 32 222 / 784 -> 196 / 714 us, k = 48 341 / 1228 -> 292 / 1088, unscaled k = 64
+// 343 / 1222 -> 298 / 1131; the kernel before this one 218 / 748, 324 / 1160 and
+// 356 / 1265), not below (k = 8 96 us either way), and where the matrix has
+// entries enough (scale 18, k = 48 92 -> 84 us; scale 14, k = 24 25 -> 27).  Stores of
+// whole sectors in a predicated close gained 1 to 5 %; FP32 lanes of 32 bytes
+// measured within 4 % either way, FP64 ones 15 % slower.
+static bool branch_close(const gpu_part &p, int vn, int64_t k) { return vn == 8 && k >= 24 && p.nnz >= (3u << 20); }
+
 // k = 1: the warp-per-range kernel while its grid (64 warps per SM) takes the
 // ranges in one round, where its short chain wins (R-MAT scale 16: 18.9
 // against 20.6 us); beyond that a lane per range in the row kernel, which
@@ -1689,6 +1718,8 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 								false, kOne>(p, sa, st);
 				if constexpr (sizeof(XT) == 2)
 					if (apart) return launch_lanes_scaled<XT, YT, A, WT, kApartUnit, kApart>(p, sa, st);
+				if constexpr (sizeof(XT) == 2 && sizeof(YT) == 4)
+					if (branch_close(p, vn, k)) return launch_lanes_scaled<XT, YT, A, WT, 8, kBranch>(p, sa, st);
 				switch (vn) {
 				case 1: return launch_lanes_scaled<XT, YT, A, WT, 1>(p, sa, st);
 				case 2: return launch_lanes_scaled<XT, YT, A, WT, 2>(p, sa, st);

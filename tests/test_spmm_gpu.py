@@ -677,3 +677,38 @@ def test_bf16_odd_width_costs_no_more_than_fp32(torch_cuda):
         torch.cuda.synchronize()
         best[dt] = min(a.elapsed_time(b) for a, b in zip(ev, ev[1:]))
     assert best[torch.bfloat16] <= best[torch.float32]
+
+
+def _best_ms(torch, call, reps=10):
+    for _ in range(3):
+        assert call()
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(reps + 1)]
+    ev[0].record()
+    for e in ev[1:]:
+        assert call()
+        e.record()
+    torch.cuda.synchronize()
+    return min(a.elapsed_time(b) for a, b in zip(ev, ev[1:]))
+
+
+def _rmat_device(torch, scale):
+    s, d = (torch.from_numpy(x.astype(np.int32)).cuda() for x in rmat_edges(scale, seed=1))
+    return sparse_matrix.from_device_edges(s, d, None, nrows=1 << scale, ncols=1 << scale, dedup=True)
+
+
+def test_wide_bf16_rows_into_fp32(torch_cuda):
+    """BF16 rows of 24 columns or more into FP32 (matrices of 3M entries or more):
+    the same bits whether Y's rows start on sectors or 16 bytes off, and 32
+    columns with input scales cost little more than into BF16 (1.2 times when
+    every entry paid for a row close)."""
+    torch = torch_cuda
+    n, k = 1 << 20, 32
+    m = _rmat_device(torch, 20)
+    x = torch.randn((n, k), device="cuda").to(torch.bfloat16)
+    sc = torch.rand(n, device="cuda") + 0.5
+    y, z = (torch.zeros(n * k + 8, device="cuda")[off:off + n * k].view(n, k) for off in (0, 4))
+    for si, so in ((None, None), (sc, None), (None, sc), (sc, sc)):
+        assert m.multiply(x, y, si, so) and m.multiply(x, z, si, so)
+        assert torch.equal(y, z)
+    b = torch.empty_like(x)
+    assert _best_ms(torch, lambda: m.multiply(x, y, sc, None)) <= 1.12 * _best_ms(torch, lambda: m.multiply(x, b, sc, None))
