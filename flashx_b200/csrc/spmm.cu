@@ -560,8 +560,12 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 		}
 		// steps without a cold entry skip the scales (4-byte types: the second
 		// copy of the sums spills in the others, BF16 695 against 393 us at
-		// scale 21)
-		const bool cold = SI && (sizeof(XT) != 4 || !(all & kHot));
+		// scale 21).  The lanes that are together here decide together: with each
+		// group its own way a warp mostly ran both (input scales, FP32 k = 32, R-MAT
+		// scale 18 / 21 / 23 75 / 440 / 2090 against 70 / 394 / 1700 us); an entry of
+		// the pack takes a scale of 1.  Nothing branches between the mask and the
+		// vote, so every lane of the mask arrives.
+		const bool cold = SI && (sizeof(XT) != 4 || __any_sync(__activemask(), !(all & kHot)));
 		if constexpr (SI)
 			if (cold) {
 #pragma unroll

@@ -712,3 +712,17 @@ def test_wide_bf16_rows_into_fp32(torch_cuda):
         assert torch.equal(y, z)
     b = torch.empty_like(x)
     assert _best_ms(torch, lambda: m.multiply(x, y, sc, None)) <= 1.12 * _best_ms(torch, lambda: m.multiply(x, b, sc, None))
+
+
+def test_input_scales_cost_little(torch_cuda):
+    """Input scales of FP32 rows: a warp runs one copy of a step's sums, the
+    scaled one when any of its groups meets a column outside the pack.  32
+    columns at R-MAT scale 21 stay near the unscaled product (1.2 times when
+    each group went its own way)."""
+    torch = torch_cuda
+    n, k = 1 << 21, 32
+    m = _rmat_device(torch, 21)
+    x = torch.randn((n, k), device="cuda")
+    y = torch.empty_like(x)
+    sc = torch.rand(n, device="cuda") + 0.5
+    assert _best_ms(torch, lambda: m.multiply(x, y, sc, None)) <= 1.14 * _best_ms(torch, lambda: m.multiply(x, y))
