@@ -1556,7 +1556,7 @@ static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 template <class XT, class YT, class A, class WT, int VN, int FORM = kAny>
 static int launch_lanes_scaled(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
-	if constexpr (std::is_floating_point<A>::value && (sizeof(XT) == 4 || VN * sizeof(XT) <= 16)) {
+	if constexpr (std::is_floating_point<A>::value && (sizeof(XT) <= 4 || VN * sizeof(XT) <= 16)) {
 		if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true, FORM>(p, a, st);
 		if (a.s_in) return launch_lanes<XT, YT, A, WT, VN, true, false, FORM>(p, a, st);
 		if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true, FORM>(p, a, st);
@@ -1566,15 +1566,22 @@ static int launch_lanes_scaled(const gpu_part &p, const spmm_args &a, cudaStream
 
 static bool aligned_to(const void *p, size_t n) { return (reinterpret_cast<uintptr_t>(p) % n) == 0; }
 
+// BF16 lanes of 32 bytes exist for unweighted products into BF16.
+template <class XT, class YT, class WT>
+constexpr bool kWideBf16 = sizeof(XT) == 2 && sizeof(YT) == 2 && std::is_void<WT>::value;
+
 // Elements per lane for a call: the widest unit of at most 16 bytes that
 // every X and Y row is made of and starts on (stores go in units of up to 16
 // bytes), or 32 bytes where that measured faster: FP32 with row scales (471
 // against 528 us at R-MAT scale 21, k = 16: the scales cost instructions per
 // entry, which wider lanes halve), and unscaled rows of 96 bytes or more
 // (FP32 k = 32 weighted 786 against 882 us, FP64 k = 16 701 against 784 us at
-// scale 22), but not shorter ones (k = 16 FP32 507 against 412 us).
-template <class XT, class YT>
-static int lane_width(const void *X, int64_t ldx, const void *Y, int64_t ldy, int64_t k, bool scaled)
+// scale 22), but not shorter ones (k = 16 FP32 507 against 412 us).  Of BF16 rows
+// those of 96 bytes or more into BF16, unweighted, on matrices with entries
+// enough (input scales, k = 64, R-MAT scale 21 644 against 557 us, in the lanes
+// before this kernel's 603; scale 16 39 against 43; weighted within 3 %).
+template <class XT, class YT, class WT>
+static int lane_width(const gpu_part &p, const void *X, int64_t ldx, const void *Y, int64_t ldy, int64_t k, bool scaled)
 {
 	if (uint64_t(ldx) * sizeof(XT) >= (1ull << 32)) return 1;
 	auto fits = [&](int vn) {
@@ -1584,7 +1591,8 @@ static int lane_width(const void *X, int64_t ldx, const void *Y, int64_t ldy, in
 	constexpr int V32 = int(32 / sizeof(XT)), V16 = V32 / 2;
 	const bool f32 = std::is_same<XT, float>::value;
 	const int64_t row = std::min<int64_t>(k * int64_t(sizeof(XT)), kPanelBytes);
-	if (sizeof(XT) != 2 && (scaled ? f32 : row >= 96) && fits(V32)) return V32;
+	const bool wide = sizeof(XT) == 2 ? kWideBf16<XT, YT, WT> && row >= 96 && p.nnz >= (8u << 20) : scaled ? f32 : row >= 96;
+	if (wide && fits(V32)) return V32;
 	int vn = V16;
 	while (vn > 1 && !fits(vn)) vn /= 2;
 	return vn;
@@ -1692,7 +1700,7 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 			return run_spmv<A, WT, false>(p, static_cast<const A *>(X), ldx, static_cast<A *>(Y), ldy, st, pr_epi{}, xhot,
 					partial);
 	}
-	const int vn = lane_width<XT, YT>(X, ldx, Y, ldy, k, sin || sout);
+	const int vn = lane_width<XT, YT, WT>(p, X, ldx, Y, ldy, k, sin || sout);
 	constexpr int V32 = int(32 / sizeof(XT));
 	// column panels of at most kPanelBytes of X row, and 32 lanes
 	const bool apart = lanes_apart<XT>(p, vn, ldx, k, sin != nullptr);
@@ -1729,6 +1737,8 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 				case 2: return launch_lanes_scaled<XT, YT, A, WT, 2>(p, sa, st);
 				case 4: return launch_lanes_scaled<XT, YT, A, WT, 4>(p, sa, st);
 				}
+				if constexpr (kWideBf16<XT, YT, WT>)
+					if (vn == 16) return launch_lanes_scaled<XT, YT, A, WT, 16>(p, sa, st);
 				if constexpr (V32 >= 8) return launch_lanes_scaled<XT, YT, A, WT, 8>(p, sa, st);
 				return set_error(FMX_ERR_UNSUPPORTED, "no kernel for lanes of %d elements", vn);
 			}))

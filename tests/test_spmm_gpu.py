@@ -726,3 +726,47 @@ def test_input_scales_cost_little(torch_cuda):
     y = torch.empty_like(x)
     sc = torch.rand(n, device="cuda") + 0.5
     assert _best_ms(torch, lambda: m.multiply(x, y, sc, None)) <= 1.14 * _best_ms(torch, lambda: m.multiply(x, y))
+
+
+@pytest.mark.parametrize("k", [48, 56, 64, 128])
+def test_bf16_wide_rows(torch_cuda, k):
+    """BF16 rows of 96 bytes or more into BF16 in lanes of 16 columns (matrices
+    of 8M entries or more): whole and aligned rows take them, others do not;
+    integer values and power-of-two scales, so that every element is the exact
+    sum rounded once."""
+    torch = torch_cuda
+    n = 30000
+    src, dst = _graph(n, 9_000_000, k, ((5, 256), (29999, 9000), (77, 300)))
+    idx, mat = oracle.build_image(src, dst, None, block=(16384, 16384), dedup=True)
+    m = sparse_matrix.create(matrix_image.from_bytes(idx, mat), None)
+    assert m.get_nnz() >= 8 << 20
+    rng = np.random.default_rng(k)
+    X = rng.integers(-2, 3, (n, k))
+    s = np.ldexp(1.0, rng.integers(-2, 3, n))
+    sc = torch.from_numpy(s).to("cuda", torch.float32)
+    R = oracle.spmm(idx, mat, X.astype(np.float64))
+    Rs = oracle.spmm(idx, mat, X * s[:, None])
+    for pad, off in ((0, 0), (16, 0), (8, 8)):
+        Xw = torch.full((n, k + pad), 99, dtype=torch.bfloat16, device="cuda")
+        Xw[:, off:off + k] = torch.from_numpy(X).to("cuda", torch.bfloat16)
+        for si, so, want in ((None, None, R), (sc, None, Rs), (None, sc, R * s[:, None]), (sc, sc, Rs * s[:, None])):
+            Yw = torch.full((n, k + pad), 77, dtype=torch.bfloat16, device="cuda")
+            assert m.multiply(Xw[:, off:off + k], Yw[:, off:off + k], si, so), _lib.last_error()
+            assert torch.equal(Yw[:, off:off + k].cpu(), torch.from_numpy(want).to(torch.bfloat16))
+            assert bool((Yw[:, :off] == 77).all()) and bool((Yw[:, off + k:] == 77).all())
+
+
+def test_bf16_wide_rows_cost(torch_cuda):
+    """64 BF16 columns with input scales at R-MAT scale 21 against 32: two lanes
+    a 64-byte row, four a 128-byte row (eight of 16 bytes took 1.85 times as
+    long)."""
+    torch = torch_cuda
+    n = 1 << 21
+    m = _rmat_device(torch, 21)
+    sc = torch.rand(n, device="cuda") + 0.5
+    t = {}
+    for k in (32, 64):
+        x = torch.randn((n, k), device="cuda").to(torch.bfloat16)
+        y = torch.empty_like(x)
+        t[k] = _best_ms(torch, lambda: m.multiply(x, y, sc, None))
+    assert t[64] <= 1.72 * t[32]
