@@ -176,3 +176,25 @@ def test_gram_f64_of_few_rows(torch_cuda, n, one_operand):
             t.append(ev[0].elapsed_time(ev[1]))
         best[b] = min(t)
     assert best[32] <= 1.1 * best[33]
+
+
+@pytest.mark.parametrize("b", [2, 16, 33])
+@pytest.mark.parametrize("exponent", [-1030, -1000, 0, 1000])
+def test_chol_inv_at_the_ends_of_the_range(torch_cuda, b, exponent):
+    """G times 2^exponent, down to subnormal pivots, whose reciprocals overflow:
+    T is the unscaled one times 2^(-exponent / 2).  At 2^-1030 the entries keep
+    44 bits; the pivots of G = A^T A + b I are at least b and its entries at most
+    about 4 b, so that their rounding of 2^-44 grows by less than b^2 * 16."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(b)
+    A = torch.randn((2 * b, b), generator=g, device="cuda", dtype=torch.float64)
+    G = A.T @ A + b * torch.eye(b, device="cuda", dtype=torch.float64)
+    T, S = (torch.empty((b, b), dtype=torch.float64, device="cuda") for _ in range(2))
+    info = torch.full((2,), -1, dtype=torch.int32, device="cuda")
+    small = torch.from_numpy(np.ldexp(G.cpu().numpy(), exponent)).cuda()
+    assert _lib.lib.fmx_dense_chol_inv(G.data_ptr(), b, T.data_ptr(), info.data_ptr(), _stream(torch)) == 0
+    assert _lib.lib.fmx_dense_chol_inv(small.data_ptr(), b, S.data_ptr(), info[1:].data_ptr(), _stream(torch)) == 0
+    assert info.tolist() == [0, 0]
+    got = np.ldexp(S.cpu().numpy(), exponent // 2)
+    tol = 16 * b * b * 2.0 ** (-44 if exponent < -1022 else -52)
+    assert np.abs(got - T.cpu().numpy()).max() <= tol * float(T.abs().max())
