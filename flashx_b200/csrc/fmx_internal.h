@@ -21,6 +21,17 @@ namespace fmx {
 // Sets the thread-local message returned by fmx_last_error() and returns code.
 int set_error(int code, const char *fmt, ...);
 
+// While it lives, this thread's memory calls do not end a graph capture that
+// another thread has under way in the default mode.  (They touch no stream that
+// is being captured.)
+struct beside_captures {
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+	beside_captures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+	~beside_captures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+	beside_captures(const beside_captures &) = delete;
+	beside_captures &operator=(const beside_captures &) = delete;
+};
+
 // Pinned host memory of one host thread, allocated by its first use and freed
 // when the thread ends (a page-locked allocation per call can stall for a long
 // time in a process that holds much pinned memory).  Declare it thread_local.
@@ -29,13 +40,19 @@ struct thread_pinned {
 	T *p = nullptr;
 	cudaError_t get(T **out)
 	{
-		const cudaError_t e = p ? cudaSuccess : cudaMallocHost(reinterpret_cast<void **>(&p), sizeof(T));
+		cudaError_t e = cudaSuccess;
+		if (!p) {
+			beside_captures guard;
+			e = cudaMallocHost(reinterpret_cast<void **>(&p), sizeof(T));
+		}
 		*out = p;
 		return e;
 	}
 	~thread_pinned()
 	{
-		if (p) cudaFreeHost(p);
+		if (!p) return;
+		beside_captures guard;
+		cudaFreeHost(p);
 	}
 };
 
