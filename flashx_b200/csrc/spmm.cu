@@ -1560,6 +1560,8 @@ static int launch_lanes_scaled(const gpu_part &p, const spmm_args &a, cudaStream
 		if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true, FORM>(p, a, st);
 		if (a.s_in) return launch_lanes<XT, YT, A, WT, VN, true, false, FORM>(p, a, st);
 		if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true, FORM>(p, a, st);
+	} else if (a.s_in || a.s_out) {
+		return set_error(FMX_ERR_UNSUPPORTED, "no scaled kernel for lanes of %d elements", VN);
 	}
 	return launch_lanes<XT, YT, A, WT, VN, false, false, FORM>(p, a, st);
 }
@@ -1706,6 +1708,8 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 	const bool apart = lanes_apart<XT>(p, vn, ldx, k, sin != nullptr);
 	const int unit = apart ? kApartUnit : vn;
 	const int panel = std::min(kPanelBytes / int(sizeof(XT)), 32 * unit);
+	// the pack that a producer left holds whole rows: one panel
+	if (packed && k > panel) return set_error(FMX_ERR_INVAL, "a packed product of %lld columns takes several panels", (long long)k);
 	for (int64_t c0 = 0; c0 < k; c0 += panel) {
 		const int kp = int(std::min<int64_t>(panel, k - c0));
 		spmm_args a{};

@@ -770,3 +770,23 @@ def test_bf16_wide_rows_cost(torch_cuda):
         y = torch.empty_like(x)
         t[k] = _best_ms(torch, lambda: m.multiply(x, y, sc, None))
     assert t[64] <= 1.72 * t[32]
+
+
+def test_packed_product_takes_one_panel(torch_cuda):
+    """The product whose operand's producer left the hot pack (the library's own
+    entry point, used by the eigensolver's filter) refuses operands of several
+    panels, whose later panels would be multiplied with the first one's pack."""
+    import ctypes as C
+    torch = torch_cuda
+    n = 3000
+    src, dst = _graph(n, 30000, 9)
+    m = sparse_matrix.create(matrix_image.build(src, dst, None, nrows=n, ncols=n, dedup=True), None)
+    call = _lib.lib._ZN3fmx11spmm_packedEPK10fmx_matrixiPKvliPvllS4_S4_P11CUstream_st
+    call.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p,
+                     C.c_void_p, C.c_void_p]
+    st = torch.cuda.current_stream().cuda_stream
+    for k, rc in ((32, _lib.FMX_OK), (16, _lib.FMX_OK), (33, _lib.FMX_ERR_INVAL), (48, _lib.FMX_ERR_INVAL)):
+        x = torch.randn((n, k), device="cuda")
+        y = torch.empty_like(x)
+        assert call(m.handle, _lib.F32, x.data_ptr(), k, _lib.F32, y.data_ptr(), k, k, None, None, st) == rc
+    torch.cuda.synchronize()
