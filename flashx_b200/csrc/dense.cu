@@ -1040,8 +1040,9 @@ gram_dmma_kernel(const float *__restrict__ X, int64_t ldx, int M, const float *_
 	if (r0 - t < n) load(r0, a, b);
 	for (; r0 - t < n; r0 += stride) {
 		float an[U][VM], bn[U][VN];
-		// (a warp's last trip does not wait for loads that nothing reads)
-		if (r0 - t + stride < n) load(r0 + stride, an, bn);
+		// a warp's last trip does not wait for loads that nothing reads (but in the
+		// one-operand form of 16 columns the branch took 2 us of 77)
+		if ((SYM && VM == 2) || r0 - t + stride < n) load(r0 + stride, an, bn);
 #pragma unroll
 		for (int u = 0; u < U; u++) {
 			double da[VM], db[VN];
