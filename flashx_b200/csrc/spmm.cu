@@ -2372,7 +2372,7 @@ int fmx_matrix_layout_digest(const fmx_matrix *m, int transpose, uint64_t *diges
 	mix_host(counts, sizeof(counts));
 	for (int rc : {mix(p.ranges, rg.size() * sizeof(range_t)), mix(p.fine, size_t(p.n_fine) * sizeof(range_t)), mix(p.col, padded * sizeof(uint32_t)),
 			mix(p.val, p.esize ? padded * p.esize : 0), mix(p.heavy, size_t(p.n_heavy) * sizeof(heavy_row)),
-			mix(p.hot_col, size_t(p.n_hot) * sizeof(int32_t))})
+			mix(p.hot_col, size_t(p.n_hot) * sizeof(int32_t)), mix(p.slot, size_t(p.ncols) * sizeof(uint32_t))})
 		if (rc) return rc;
 	*digest = h;
 	return FMX_OK;

@@ -267,11 +267,12 @@ int fmx_matrix_hot(const fmx_matrix *m, uint64_t *n_hot_cols, uint64_t *hot_entr
                    uint64_t *scratch_bytes);
 
 /* A 64-bit FNV-1a digest of one resident orientation (transpose = 0: A,
- * else A^T): the entry stream, values, ranges, heavy-row list, hot columns
- * and the schedule counts.  Two builds of the same matrix (a host image
- * through fmx_matrix_create, device edges through fmx_matrix_build_device)
- * lay it out identically exactly when the digests agree.  Copies the layout
- * to the host: a diagnostic, not for hot paths.  No reference counterpart. */
+ * else A^T): the entry stream, values, ranges, heavy-row list, hot columns, the
+ * columns' hot slots and the schedule counts.  Two builds of the same matrix (a
+ * host image through fmx_matrix_create, device edges through
+ * fmx_matrix_build_device) lay it out identically exactly when the digests
+ * agree.  Copies the layout to the host: a diagnostic, not for hot paths.  No
+ * reference counterpart. */
 int fmx_matrix_layout_digest(const fmx_matrix *m, int transpose, uint64_t *digest);
 
 /* ---- dense kernels of the block eigensolver --------------------------------
