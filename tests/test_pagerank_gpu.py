@@ -243,3 +243,32 @@ def test_pagerank_ends_with_convergence(torch_cuda, n, m, streamed):
 
     best(it)
     assert best(200) <= 1.5 * best(it)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("hub", [300, 4000, 30000])
+def test_pagerank_warp_form_hubs(torch_cuda, hub, weighted):
+    """A warp per range: a row of 2, 16 or 118 chunks (up to 8, up to 64 and more
+    are added by 2, 32 and 256 parts), finished by the warp whose chunk arrives
+    last, has the bits of the product's fixup kernel, weighted or not, and so has
+    the whole loop."""
+    torch = torch_cuda
+    from flashx_b200 import matrix_image, sparse_matrix
+    n = 40000
+    rng = np.random.default_rng(hub)
+    src, dst = _directed(n, 150000, hub)
+    for row, deg in ((7, hub), (39999, hub // 2 + 150)):
+        src = np.concatenate([src, rng.choice(n, deg, replace=False).astype(np.uint32)])
+        dst = np.concatenate([dst, np.full(deg, row, dtype=np.uint32)])
+    # ranges: at most one run per 128 entries and the hubs' chunks
+    assert (len(dst) + n) // 128 + 400 <= 64 * torch.cuda.get_device_properties(0).multi_processor_count
+    w = rng.uniform(0.5, 1, len(src)).astype(np.float32) if weighted else None
+    img = matrix_image.build(src, dst, w, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+    timg = matrix_image.build(dst, src, w, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+    m = sparse_matrix.create(img, timg)
+    ref, ended = _stepwise(torch, m, n, 100)
+    assert ended
+    for cap in (1, 5, 200, 200):
+        got, git = PageRank(m, cap, 0.85)
+        assert git == min(cap, len(ref))
+        assert np.array_equal(got.cpu().numpy(), ref[git - 1])
