@@ -965,9 +965,9 @@ __global__ void __launch_bounds__(256) gram_reduce_kernel(const T *part, int npa
 //
 // What bounds it: bytes in flight, then the DMMA pipe.  With 4-byte loads of 8
 // rows per trip the 16-column Gram at n = 4.2M took 231 us (one operand) and
-// 262 us (two); the DMMA pipe needs about 54 us, HBM 41 and 82 us.  Now 73 and
-// 107 us; 32 columns at n = 2.1M (formerly on CUDA cores) 511 -> 111 and 540 ->
-// 167 us, 64 columns at n = 1.0M 1083 -> 300 us.
+// 262 us (two); the DMMA pipe needs about 54 us, HBM 41 and 82 us.  Now 77 and
+// 107 us; 32 columns at n = 2.1M (formerly on CUDA cores) 511 -> 96 and 540 ->
+// 154 us, 64 columns at n = 1.0M 1083 -> 285 us.
 __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b)
 {
 	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -1001,8 +1001,11 @@ __device__ __forceinline__ void gram_load(const float *row, int c, int lim, bool
 // 4-row steps per trip: two operands of 16 columns at n = 4.2M 107 us with 2,
 // 116 with 4, 126 with 8; of 32 columns at n = 2.1M (127 registers, two CTAs per
 // SM) 167 with 2, 174 with 1, 181 with 4.  One operand: 16 columns 79 us with
-// 4, 77 with 5, 73 with 8 (5 holds a third fewer registers); 32 columns 111
-// with 4, 122 with 2.
+// 4, 77 with 5, 73 with 8; 32 columns 111 with 4, 122 with 2.  Five for 16 columns,
+// not eight: the order of the additions changes with it, and in the SVD test's
+// mixed solve the angle to the reference's vectors then came out at 1.1e-4, above
+// its bound of 1e-4 (with 5 at 4e-5).  That bound is too near to tell two
+// roundings of the Gram apart, but it is the one that results are held to.
 constexpr int gram_steps(int vm, int vn, bool sym)
 {
 	return vm * vn > 4 ? (sym ? 4 : 2) : vm * vn == 1 ? 8 : (sym ? 5 : 2);

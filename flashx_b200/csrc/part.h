@@ -35,8 +35,9 @@ constexpr uint32_t kRange = FMX_RANGE_ENTRIES;  // most target entries per multi
 constexpr uint32_t kRangeMin = FMX_RANGE_MIN;   // fewest: small matrices get shorter runs, so that they
                                                 // still fill the grid
 constexpr uint32_t kRangeFine = 32;     // runs of the fine list (fine_entries)
-// lane groups of a full grid at k = 16 (148 SMs x 32 warps x 16 groups)
-// times the runs each should get before runs shrink below kRange
+// Runs shrink below kRange when there would be fewer than this many: a tuned
+// constant (148 SMs x 512 lane groups, the full grid of an earlier kernel at
+// k = 16; the row kernel of today has 148 x 192 groups there)
 constexpr uint64_t kRangeFill = uint64_t(FMX_RANGE_FILL_PER_GROUP) * 148 * 32 * 16;
 constexpr uint32_t kLongChunks = 8;     // heavy rows with more chunks get a warp each in the fixup
 constexpr uint32_t kBlockChunks = 64;   // heavy rows with more chunks get a block of 8 warps each

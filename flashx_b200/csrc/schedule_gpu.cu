@@ -517,12 +517,11 @@ int make_part_device(const dev_csr &csr, int device, cudaStream_t st, std::share
 	SCUDA_TRY(cudaMemsetAsync(p->xhot, 0, size_t(nhot + 1) * kPanelBytes, st));
 	for (int q = 1; q < 5; q++) TRY(back.ask(cnt + q));
 	TRY(back.wait());
-	const unsigned long long *hc = back.w - 1;   // n_exact, hot_entries, n_long, n_block
 	p->n_hot = nhot;
-	p->n_exact = uint32_t(hc[1]);
-	p->hot_entries = hc[2];
-	p->n_long_heavy = uint32_t(hc[3]);
-	p->n_block_heavy = uint32_t(hc[4]);
+	p->n_exact = uint32_t(back.w[0]);
+	p->hot_entries = back.w[1];
+	p->n_long_heavy = uint32_t(back.w[2]);
+	p->n_block_heavy = uint32_t(back.w[3]);
 	p->n_ranges = uint32_t(n_coarse);
 	p->n_fine = has_fine ? uint32_t(nseg) : 0;
 	p->n_heavy = n_heavy;

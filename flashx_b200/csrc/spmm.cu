@@ -47,7 +47,7 @@
 // the reference's order (bit-identical results).  No atomics: every output
 // row is written exactly once.  Two row kernels share that scheme:
 //   spmm_lane_kernel  every panel: a lane owns 2 to 32 bytes of each gathered
-//                     row, 8 or 16 gathers in flight per lane
+//                     row, the gathers of 8, 16 or 32 entries in flight per lane
 //   spmv_kernel       k = 1 of small matrices and PageRank: a warp per range,
 //                     gathers staged in shared memory
 // Each call first packs the hot rows: pack_hot_vec_kernel in 16-byte units,
@@ -155,8 +155,12 @@ __device__ __forceinline__ void st_sector(T *p, const T (&v)[VEC])
 // dep_wait() holds them until the kernel before has completed.  Every kernel of
 // such a chain waits, and lets its successor in only then: when one starts,
 // everything before its predecessor is complete, and the read-only loads see no
-// line from before it.  The first kernel of a call carries no attribute and
-// follows all earlier work of the stream as usual.  What a kernel of the chain
+// line from before it.  fmx_spmm's first kernel, the pack, carries no attribute
+// and follows all earlier work of the stream as usual.  Where a product starts
+// with a dependent launch (spmm_packed; a PageRank iteration), the kernel before
+// it is a plain one that never lets its successor in early (the solver's filter
+// step, init_kernel), or one that itself waited first (the iteration before), or
+// a copy.  What a kernel of the chain
 // writes is read by plain loads only: ld.global.nc asks for data that nobody
 // writes while the kernel is resident, and the compiler may move an __ldg, or
 // a load through a const __restrict__ pointer, above the wait.
@@ -215,18 +219,6 @@ struct accum {
 			for (int v = 0; v < NV; v++)
 #pragma unroll
 				for (int i = 0; i < VEC; i++) s[v][i] = A(0);
-		}
-	}
-	__device__ __forceinline__ void zero_if(bool z)
-	{
-		if constexpr (kPacked) {
-#pragma unroll
-			for (int i = 0; i < VEC / 2; i++) p[i] = z ? 0ull : p[i];
-		} else {
-#pragma unroll
-			for (int v = 0; v < NV; v++)
-#pragma unroll
-				for (int i = 0; i < VEC; i++) s[v][i] = z ? A(0) : s[v][i];
 		}
 	}
 	// s[v] += x (* m1) (* m2), each operation rounded (no contraction)
@@ -678,16 +670,21 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 
 // Threads and resident blocks per SM: at most 24 warps (FP32 rows in 16-byte
 // lanes: 24 warps 411 us, 20 warps 429 us at scale 22), fewer where the loads
-// in flight need the registers (spills cost more than the warps: BF16 with
-// 24 warps 801 us against 446 us with 20).
+// in flight and the sums need the registers (spills cost more than the warps:
+// BF16 with 24 warps 801 us against 446 us with 20).
 constexpr int kLaneThreads = 128;
 constexpr int lane_blocks(int bytes, bool scaled, int esize, int step, bool k1)
 {
-	return k1 && esize == 8 && step == 16 ? 5 : step == 32 ? 2 : bytes == 16 && step == 16 ? 3 : bytes == 32 ? (scaled ? 4 : 3) : (scaled && esize == 8) ? 4 : (scaled || esize == 2) ? 5 : 6;
+	if (k1 && esize == 8 && step == 16) return 5;        // FP64 chunk_sum (6: 204 bytes spilled, scale 22 279 -> 319 us)
+	if (step == 32) return 2;                            // small matrices: the longest chain decides
+	if (step == 16 && bytes == 16) return 3;
+	if (bytes == 32) return scaled ? 4 : 3;              // 8 x 32 bytes a lane; unscaled 3 or 4 within 2 %
+	if (scaled && esize == 8) return 4;
+	return scaled || esize == 2 ? 5 : 6;                 // BF16's sums are FP32, twice its rows
 }
-// Entries per step (launch_lanes takes more for small matrices): 16 in lanes of at most 8 bytes of an unweighted, unscaled
-// product (small or odd panels: R-MAT scale 18, k = 5, 39 against 43 us with
-// 8), else 8.
+// Entries per step (launch_lanes takes more for small matrices): 16 in lanes of
+// at most 8 bytes of an unweighted, unscaled product (small or odd panels: R-MAT
+// scale 18, k = 5, 39 against 43 us with 8), else 8.
 constexpr int lane_step(int bytes, int esize, bool plain) { return bytes <= 8 && esize >= 4 && plain ? 16 : 8; }
 
 // FORM: kAny, kOne (k = 1 without row scales) or kLoop (the same in a PageRank
@@ -1514,6 +1511,19 @@ static int over_slices(const gpu_part &p, spmm_args a, cudaStream_t st, F &&laun
 	return FMX_OK;
 }
 
+// SMs of a device, asked once.
+static unsigned device_sms(int device)
+{
+	static std::atomic<unsigned> sms[64];
+	unsigned n = sms[device & 63].load(std::memory_order_relaxed);
+	if (!n) {
+		int v = 0;
+		cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
+		sms[device & 63].store(n = unsigned(std::max(v, 1)), std::memory_order_relaxed);
+	}
+	return n;
+}
+
 template <class XT, class YT, class A, class WT, int VN, int U, bool SI, bool SO, int FORM = kAny>
 static int launch_step(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
@@ -1546,7 +1556,7 @@ static int launch_lanes(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 	// scale 17; int64 weighted k = 4) 24.8, 22.7, 24.7 and 30.8, 28.8, 32.4; at 45
 	// (int64, n = 300k) 36.2, 37.1, 41.1 us.
 	if constexpr (FORM == kAny && VN > 1 && (VN * sizeof(XT) == 16 || VN * sizeof(XT) == 8) && sizeof(XT) >= 4 && !SI && !SO) {
-		const uint64_t groups = 148ull * 24 * unsigned(a.R);
+		const uint64_t groups = uint64_t(device_sms(p.device)) * 24 * unsigned(a.R);
 		if (p.nnz <= 24 * groups) return launch_step<XT, YT, A, WT, VN, 32, SI, SO>(p, a, st);
 		if (U < 16 && p.nnz <= 40 * groups) return launch_step<XT, YT, A, WT, VN, 16, SI, SO>(p, a, st);
 	}
@@ -1616,7 +1626,7 @@ template <class XT>
 static bool lanes_apart(const gpu_part &p, int vn, int64_t ldx, int64_t k, bool scales_in)
 {
 	if (sizeof(XT) != 2 || vn != 1 || k < 7 || uint64_t(ldx) * sizeof(XT) >= (1ull << 32)) return false;
-	const uint64_t warps = 148ull * 20 * uint64_t(32 / std::min<int64_t>(k, 32));
+	const uint64_t warps = uint64_t(device_sms(p.device)) * 20 * uint64_t(32 / std::min<int64_t>(k, 32));
 	return k >= 11 ? p.nnz >= 300 * warps : scales_in && p.nnz >= 1500 * warps;
 }
 
@@ -1641,19 +1651,11 @@ static bool branch_close(const gpu_part &p, int vn, int64_t k) { return vn == 8 
 // slices of 64k entries 700 against 975 us); both kernels give the same bits.
 static bool spmv_by_warps(const gpu_part &p)
 {
-	static std::atomic<unsigned> sms[64];
-	unsigned n = sms[p.device & 63].load(std::memory_order_relaxed);
-	if (!n) {
-		int v = 0;
-		cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, p.device);
-		sms[p.device & 63].store(n = unsigned(std::max(v, 1)), std::memory_order_relaxed);
-	}
 	uint32_t most = p.streamed ? 0 : p.n_ranges;
 	for (const auto &sl : p.slices) most = std::max(most, sl.nr);
-	return most <= n * 64;
+	return most <= device_sms(p.device) * 64;
 }
 
-// Run one orientation over all column panels (kPanelBytes of X row each).
 // k = 1 without row scales: pack, the warp-per-range SpMV, fixup.
 // `xhot` and `partial` default to the part's own scratch.
 template <class T, class WT, bool EPI>
@@ -1690,6 +1692,7 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 	return launch_fixup<T, T, false>(p, static_cast<const T *>(partial), Y, ldy, 1, nullptr, st);
 }
 
+// One orientation over all column panels (kPanelBytes of X row each).
 template <class XT, class YT, class A, class WT>
 static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int64_t ldy, int64_t k,
 		const void *sin, const void *sout, cudaStream_t st, void *xhot = nullptr, void *partial = nullptr,
