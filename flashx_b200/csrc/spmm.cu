@@ -416,15 +416,13 @@ __device__ __forceinline__ void ld_wn(const void *val, uint32_t e0, A (&w)[U])
 	}
 }
 
-// A chunk's sum in the kernels of k = 1 without row scales.  A chunk may be
-// added in any fixed order; this one is the same in the lane kernel, whatever
-// its step, and in the warp-per-range kernel, so that the choice between them
-// does not show in the results: binary trees over blocks of 16 places, block b
-// added to running sum b % 4, and a tree over those.  Its error is that of 32
-// strided sums and a tree over them (8000 chunks of 129 to 256 FP32 numbers,
-// RMS against FP64: 7.6e-8 of normal ones against 7.8e-8, 4.0e-8 of uniform
-// ones in both; a single running sum of the blocks has 8.9e-8 and 5.9e-8; a
-// whole binary tree 7.6e-8 and 4.3e-8, for more registers).
+// A chunk's sum in the row kernel at k = 1 without row scales: binary trees over
+// blocks of 16 places, block b added to running sum b % 4, and a tree over
+// those.  Its error is that of the warp-per-range kernel's 32 strided sums and a
+// tree over them (8000 chunks of 129 to 256 FP32 numbers, RMS against FP64:
+// 7.6e-8 of normal ones against 7.8e-8, 4.0e-8 of uniform ones in both; a single
+// running sum of the blocks has 8.9e-8 and 5.9e-8; a whole binary tree 7.6e-8
+// and 4.3e-8, for more registers).  The order does not depend on the step.
 static_assert(kChunk == 256, "chunk_sum and warp_chunk add 256 places");
 template <class A, int U>
 struct chunk_sum {
@@ -462,7 +460,8 @@ struct chunk_sum {
 };
 
 // The same sum by a warp whose lane l holds the terms 32 j + l in t[j], j < 8
-// (zeros beyond the chunk).
+// (zeros beyond the chunk): the warp-per-range kernel's, in a streamed part whose
+// resident form takes the row kernel, so that the products are equal.
 template <class A>
 __device__ __forceinline__ A warp_chunk(const A *t, int lane)
 {
@@ -727,8 +726,9 @@ spmm_lane_kernel(const spmm_args a)
 // then each lane sums whole rows of the range from shared memory in entry
 // order, with one running sum per row and every add rounded, which is the
 // lane-group kernel's arithmetic: rows of up to 256 entries come out
-// identical.  A chunk of a longer row is added up by the whole warp
-// (warp_chunk) into its partial slot.
+// identical.  A chunk of a longer row is added up by the whole warp into its
+// partial slot: each lane its own entries, then a fixed xor tree, or, with
+// BLOCKS, in the row kernel's order (warp_chunk).
 // (spmv_by_warps says which matrices come here.)
 constexpr int kSpmvMax = 512;            // most entries of one range
 static_assert(((kRange - 1 + kExactMax + kStep - 1) / kStep) * kStep <= uint32_t(kSpmvMax) &&
@@ -785,7 +785,7 @@ __device__ __forceinline__ void pr_chunk(const pr_epi &e, float *partial, uint32
 	}
 }
 
-template <class T, class WT, bool EPI>
+template <class T, class WT, bool EPI, bool BLOCKS>
 __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const pr_epi e)
 {
 	constexpr int kWarps = kThreads / 32;
@@ -881,7 +881,15 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			}
 		} else {
 			// a chunk: each lane adds its entries (j order), then a fixed xor tree
-			const T acc = warp_chunk(t, lane);
+			T acc = T(0);
+			if constexpr (BLOCKS) {
+				acc = warp_chunk(t, lane);
+			} else {
+#pragma unroll
+				for (int j = 0; j < J; j++) acc = acc_add(acc, t[j]);
+#pragma unroll
+				for (int o = 16; o > 0; o >>= 1) acc = acc_add(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+			}
 			if constexpr (EPI) pr_chunk(e, static_cast<float *>(a.partial), rg.slot, acc, lane, cnt);
 			else if (lane == 0) static_cast<T *>(a.partial)[int64_t(rg.slot) * kPartialStride] = acc;
 		}
@@ -1648,7 +1656,9 @@ static bool branch_close(const gpu_part &p, int vn, int64_t k) { return vn == 8 
 // issues a third of the instructions per entry (scale 18 / 20 / 22 / 24: 38 /
 // 111 / 325 / 1400 against 29 / 66 / 251 / 1150 us).  A streamed part is
 // launched slice by slice, so its largest slice decides (R-MAT scale 18 in
-// slices of 64k entries 700 against 975 us); both kernels give the same bits.
+// slices of 64k entries 700 against 975 us), while the order of its sums is the
+// resident form's (row_kernel_order).
+static bool row_kernel_order(const gpu_part &p) { return p.n_ranges > device_sms(p.device) * 64; }
 static bool spmv_by_warps(const gpu_part &p)
 {
 	uint32_t most = p.streamed ? 0 : p.n_ranges;
@@ -1678,9 +1688,10 @@ static int run_spmv(const gpu_part &p, const T *X, int64_t ldx, T *Y, int64_t ld
 				nullptr);
 		CUDA_TRY(cudaGetLastError());
 	}
-	auto kern = spmv_kernel<T, WT, EPI>;
-	static std::atomic<unsigned> blocks[64];
-	const unsigned b = cached_blocks(blocks[p.device & 63], kern, p.device, kThreads);
+	const bool in_blocks = row_kernel_order(p);
+	auto kern = in_blocks ? spmv_kernel<T, WT, EPI, true> : spmv_kernel<T, WT, EPI, false>;
+	static std::atomic<unsigned> blocks[2][64];
+	const unsigned b = cached_blocks(blocks[in_blocks][p.device & 63], kern, p.device, kThreads);
 	if (int rc = over_slices(p, a, st, [&](const spmm_args &sa) -> int {
 			if (p.streamed) kern<<<b, kThreads, 0, st>>>(sa, e);
 			else CUDA_TRY(launch_dep(kern, b, kThreads, st, sa, e));

@@ -561,10 +561,10 @@ def _strided32(t):
 @pytest.mark.parametrize("extra,warps", [(100_000, True), (3_000_000, False)])
 @pytest.mark.parametrize("length", [512, 437, 259])
 def test_spmv_chunk_sums(torch_cuda, length, extra, warps, weighted, dtype):
-    """k = 1, rows of two chunks of up to 256 entries: both kernels (a warp per
-    range up to 64 ranges per SM, else a lane per range) add a chunk in the same
-    order, bit for bit, and whole chunks with no larger error against FP64 than
-    32 strided sums have on the same numbers."""
+    """k = 1, rows of two chunks of up to 256 entries, bit for bit: a warp per
+    range (up to 64 ranges per SM) adds a chunk by 32 strided sums and a tree, a
+    lane per range by blocks of 16 into four running sums, and whole chunks with
+    no larger error against FP64 than the former has on the same numbers."""
     torch = torch_cuda
     n, rows = 1 << 17, 1500
     rng = np.random.default_rng(extra)
@@ -582,7 +582,8 @@ def test_spmv_chunk_sums(torch_cuda, length, extra, warps, weighted, dtype):
         t = t * w[:rows * length].reshape(rows, length)
     c = np.zeros((2, rows, 256), t.dtype)
     c[0, :, :length // 2], c[1, :, :length - length // 2] = t[:, :length // 2], t[:, length // 2:]
-    assert np.array_equal(got, _blocks256(c[0]) + _blocks256(c[1]))
+    order = _strided32 if warps else _blocks256
+    assert np.array_equal(got, order(c[0]) + order(c[1]))
     if dtype == "float32" and length == 512:
         exact = t.astype(np.float64).sum(1)
         assert np.linalg.norm(got - exact) <= np.linalg.norm(_strided32(c[0]) + _strided32(c[1]) - exact)
