@@ -830,7 +830,10 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(const spmm_args a, const
 			if (i < rg.len) {
 				const uint32_t c = raw[j] & kIdxMask;
 				const bool hot = raw[j] & kHot;
-				t[j] = ld_n<T, 1>(reinterpret_cast<const char *>((hot ? H : X) + int64_t(c) * (hot ? int64_t(1) : a.ldx))).v[0];
+				// a plain load (the wait's memory clobber keeps it behind): as volatile
+				// asm the 16 guarded FP64 gathers came one after the other, 7.2 us
+				// for a launch of 500 ranges instead of 4.5
+				t[j] = (hot ? H : X)[int64_t(c) * (hot ? int64_t(1) : a.ldx)];
 			}
 		}
 		if constexpr (!kBinary) {
