@@ -99,3 +99,18 @@ def test_streamed_spmv_in_small_slices(torch_cuda, weighted, slice_entries):
     for dt in (torch.float32, torch.float64):
         X = torch.randn((n, 1), device="cuda", dtype=dt)
         assert torch.equal(res.multiply(X), st.multiply(X))
+
+
+def test_streamed_bytes(torch_cuda):
+    """Slices that are copied for longer than their kernels run hold whole runs:
+    the fine runs of small slices, each padded to eight entries, are more to
+    copy.  The products are the same bits."""
+    torch = torch_cuda
+    n = 1 << 18
+    s, d = rmat_edges(18, seed=3)
+    img = matrix_image.build(s, d, None, nrows=n, ncols=n, block_size=(16384, 16384), dedup=True)
+    small, large = (sparse_matrix.create_streamed(img, None, slice_entries=e) for e in (1 << 16, 1 << 19))
+    assert large.stream_info()[1] <= 0.98 * small.stream_info()[1]
+    for k in (1, 16):
+        X = torch.randn((n, k), device="cuda")
+        assert torch.equal(small.multiply(X), large.multiply(X))
