@@ -555,8 +555,11 @@ __device__ __forceinline__ void run_range(const spmm_args &a, const range_t rg, 
 		// group its own way a warp mostly ran both (input scales, FP32 k = 32, R-MAT
 		// scale 18 / 21 / 23 75 / 440 / 2090 against 70 / 394 / 1700 us); an entry of
 		// the pack takes a scale of 1.  Nothing branches between the mask and the
-		// vote, so every lane of the mask arrives.
-		const bool cold = SI && (sizeof(XT) != 4 || __any_sync(__activemask(), !(all & kHot)));
+		// vote, so every lane of the mask arrives.  One-element lanes, whose second
+		// copy costs one add an entry, decide by group (k = 17 at scale 21 2160
+		// against 2219 us with the vote).
+		bool cold = SI && (sizeof(XT) != 4 || !(all & kHot));
+		if constexpr (SI && sizeof(XT) == 4 && VN > 1) cold = __any_sync(__activemask(), cold);
 		if constexpr (SI)
 			if (cold) {
 #pragma unroll
