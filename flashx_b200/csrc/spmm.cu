@@ -1586,9 +1586,11 @@ template <class XT, class YT, class A, class WT, int VN, int FORM = kAny>
 static int launch_lanes_scaled(const gpu_part &p, const spmm_args &a, cudaStream_t st)
 {
 	if constexpr (std::is_floating_point<A>::value && (sizeof(XT) <= 4 || VN * sizeof(XT) <= 16)) {
-		if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true, FORM>(p, a, st);
+		if constexpr (FORM != kBranch) {
+			if (a.s_in && a.s_out) return launch_lanes<XT, YT, A, WT, VN, true, true, FORM>(p, a, st);
+			if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true, FORM>(p, a, st);
+		}
 		if (a.s_in) return launch_lanes<XT, YT, A, WT, VN, true, false, FORM>(p, a, st);
-		if (a.s_out) return launch_lanes<XT, YT, A, WT, VN, false, true, FORM>(p, a, st);
 	} else if (a.s_in || a.s_out) {
 		return set_error(FMX_ERR_UNSUPPORTED, "no scaled kernel for lanes of %d elements", VN);
 	}
@@ -1655,11 +1657,15 @@ static bool lanes_apart(const gpu_part &p, int vn, int64_t ldx, int64_t k, bool 
 // lanes a row on, where few rows share a warp (R-MAT scale 20 / 22, input scales,
 // k = 32 222 / 784 -> 196 / 714 us, k = 48 341 / 1228 -> 292 / 1088, unscaled k = 64
 // 343 / 1222 -> 298 / 1131; the kernel before this one 218 / 748, 324 / 1160 and
-// 356 / 1265), not below (k = 8 96 us either way), and where the matrix has
-// entries enough (scale 18, k = 48 92 -> 84 us; scale 14, k = 24 25 -> 27).  Stores of
+// 356 / 1265), not below (k = 8 96 us either way), where the matrix has entries
+// enough (scale 18, k = 40 66 -> 74 us; scale 14, k = 24 25 -> 27), and without output
+// scales, whose loads the branch holds up (scale 21, k = 48 839 -> 868).  Stores of
 // whole sectors in a predicated close gained 1 to 5 %; FP32 lanes of 32 bytes
 // measured within 4 % either way, FP64 ones 15 % slower.
-static bool branch_close(const gpu_part &p, int vn, int64_t k) { return vn == 8 && k >= 24 && p.nnz >= (3u << 20); }
+static bool branch_close(const gpu_part &p, int vn, int64_t k, bool scales_out)
+{
+	return vn == 8 && k >= 24 && !scales_out && p.nnz >= (8u << 20);
+}
 
 // k = 1: the warp-per-range kernel while its grid (64 warps per SM) takes the
 // ranges in one round, where its short chain wins (R-MAT scale 16: 18.9
@@ -1760,7 +1766,7 @@ static int run_typed(const gpu_part &p, const void *X, int64_t ldx, void *Y, int
 				if constexpr (sizeof(XT) == 2)
 					if (apart) return launch_lanes_scaled<XT, YT, A, WT, kApartUnit, kApart>(p, sa, st);
 				if constexpr (sizeof(XT) == 2 && sizeof(YT) == 4)
-					if (branch_close(p, vn, k)) return launch_lanes_scaled<XT, YT, A, WT, 8, kBranch>(p, sa, st);
+					if (branch_close(p, vn, k, sout != nullptr)) return launch_lanes_scaled<XT, YT, A, WT, 8, kBranch>(p, sa, st);
 				switch (vn) {
 				case 1: return launch_lanes_scaled<XT, YT, A, WT, 1>(p, sa, st);
 				case 2: return launch_lanes_scaled<XT, YT, A, WT, 2>(p, sa, st);

@@ -698,7 +698,7 @@ def _rmat_device(torch, scale):
 
 
 def test_wide_bf16_rows_into_fp32(torch_cuda):
-    """BF16 rows of 24 columns or more into FP32 (matrices of 3M entries or more):
+    """BF16 rows of 24 columns or more into FP32 (matrices of 8M entries or more):
     the same bits whether Y's rows start on sectors or 16 bytes off, and 32
     columns with input scales cost little more than into BF16 (1.2 times when
     every entry paid for a row close)."""
