@@ -1612,7 +1612,12 @@ constexpr bool kWideBf16 = sizeof(XT) == 2 && sizeof(YT) == 2 && std::is_void<WT
 // scale 22), but not shorter ones (k = 16 FP32 507 against 412 us).  Of BF16 rows
 // those of 96 bytes or more into BF16, unweighted, on matrices with entries
 // enough (input scales, k = 64, R-MAT scale 21 644 against 557 us, in the lanes
-// before this kernel's 603; scale 16 39 against 43; weighted within 3 %).
+// before this kernel's 603; scale 16 39 against 43; weighted within 3 %).  FP32
+// rows of less than a line with row scales, in operands of 2 GB or more, stay with
+// 16 bytes: there the gathers miss most of the time, and twice the lanes hide
+// more of it (symmetric scale 25, k = 16 / 24 / 32 14.3 / 19.4 / 19.9 ms against
+// 14.9 / 20.2 / 17.4, the kernel before this one 14.2 / 19.5 / 19.5; scale 24 5.3 /
+// 8.3 / 9.0 against 4.8 / 7.3 / 7.2).
 template <class XT, class YT, class WT>
 static int lane_width(const gpu_part &p, const void *X, int64_t ldx, const void *Y, int64_t ldy, int64_t k, bool scaled)
 {
@@ -1624,7 +1629,8 @@ static int lane_width(const gpu_part &p, const void *X, int64_t ldx, const void 
 	constexpr int V32 = int(32 / sizeof(XT)), V16 = V32 / 2;
 	const bool f32 = std::is_same<XT, float>::value;
 	const int64_t row = std::min<int64_t>(k * int64_t(sizeof(XT)), kPanelBytes);
-	const bool wide = sizeof(XT) == 2 ? kWideBf16<XT, YT, WT> && row >= 96 && p.nnz >= (8u << 20) : scaled ? f32 : row >= 96;
+	const bool huge = p.ncols * uint64_t(ldx) * sizeof(XT) >= (2ull << 30);
+	const bool wide = sizeof(XT) == 2 ? kWideBf16<XT, YT, WT> && row >= 96 && p.nnz >= (8u << 20) : scaled ? f32 && (row >= 128 || !huge) : row >= 96;
 	if (wide && fits(V32)) return V32;
 	int vn = V16;
 	while (vn > 1 && !fits(vn)) vn /= 2;

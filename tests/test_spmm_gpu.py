@@ -791,3 +791,22 @@ def test_packed_product_takes_one_panel(torch_cuda):
         y = torch.empty_like(x)
         assert call(m.handle, _lib.F32, x.data_ptr(), k, _lib.F32, y.data_ptr(), k, k, None, None, st) == rc
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("k", [16, 24, 32])
+def test_scaled_rows_in_huge_operands(torch_cuda, k):
+    """FP32 row scales with an operand that spans 2 GB or more (a few columns of a
+    wide block): rows of less than a line go in 16-byte lanes, with the bits of
+    the 32-byte lanes that take them from a small operand."""
+    torch = torch_cuda
+    n, ld = 1 << 15, 1 << 14
+    src, dst = _graph(n, 400000, k, ((5, 256), (77, 9000)))
+    m = sparse_matrix.create(matrix_image.build(src, dst, None, nrows=n, ncols=n, dedup=True), None)
+    wide = torch.empty((n, ld), device="cuda")
+    x = wide[:, 64:64 + k]
+    x.copy_(torch.randn((n, k), device="cuda"))
+    sc = torch.rand(n, device="cuda") + 0.5
+    for si, so in ((sc, None), (None, sc), (sc, sc)):
+        y, z = torch.empty((n, k), device="cuda"), torch.empty((n, k), device="cuda")
+        assert m.multiply(x, y, si, so) and m.multiply(x.contiguous(), z, si, so)
+        assert torch.equal(y, z)
